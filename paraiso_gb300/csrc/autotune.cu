@@ -97,6 +97,9 @@ extern "C" om_status om_autotune(int kind, int ndim, const int *sizes, const om_
     if (!packed) {
       cands.push_back(b);  // only the integer kernel applies
     } else {
+      om_config a = b;  // no knob set: long runs keep the grid packed between launches
+      a.depth = a.tile_x = a.tile_y = a.life_kernel = 0;
+      cands.push_back(a);
       for (int depth : {24, 32})
         for (int th : {0, 128, 192, 256, 320}) {
           om_config c = b;

@@ -9,13 +9,15 @@
 //             cell' = alive ? 1 : 0
 //             population = reduce Sum cell'      generation = generation + 1
 //
-// Three device paths give bit-identical results:
+// The device paths give bit-identical results:
 //  * life_general_kernel: one int32 cell per thread with the reference's
 //    integer arithmetic; any size, cyclic or open boundary, any cell values.
-//  * life_smallgrid_kernel: whole grid bit-packed in shared memory (one CTA),
-//    all generations of a run in one launch.  Cyclic, width % 32 == 0.
-//  * life_tb_kernel: bit-packed tiles with a 1-word / k-row halo, k
-//    generations per launch (temporal blocking).  Cyclic, width % 32 == 0.
+//  * life_smallreg_kernel, life_smallgrid_kernel: whole grid bit-packed in one
+//    CTA, all generations of a run in one launch.  Cyclic, width % 32 == 0.
+//  * life_reg_kernel, life_ws_kernel, life_tb*_kernel: bit-packed tiles with a
+//    1-word / k-row halo, k generations per launch (temporal blocking).
+//  * long runs and rows that are no whole number of words keep the grid packed
+//    between launches (proceed_packed).  Cyclic, any width above 32.
 // The packed paths require every cell in {0,1}; then num is in [0,8] and
 // the rule equals the bit-sliced adder below, so outputs are identical.
 // After any external write the first generation runs on the general path,
@@ -46,6 +48,7 @@ struct LifeState {
   int pop_cap = 0;
   int last_n = 0;
   int depth = 0, tile_w = 0, tile_h = 0;  // tuned or configured
+  uint32_t *packed[2] = {nullptr, nullptr};  // the packed grid between launches
   // tensor maps of the two cell buffers (cells x words x rows) for the TMA
   // kernels, keyed by buffer address, and their one-word maps (32 cells x 1
   // word x 1 row, no swizzle) for the halo word that wraps around;
@@ -392,7 +395,31 @@ struct TbParams {
   int n0, n1, wd;   // grid in cells, width in words
   int tw, th, kk;   // tile width (words), height (rows), generations
   int nt0, nt1;     // tiles per axis
+  int nb;           // cells in the last word of a row (32 unless n0 % 32 != 0)
 };
+
+// A packed grid: rows of wd = ceil(n0 / 32) words, bit i of word w is cell
+// (32 w + i) mod n0.  Where n0 is no multiple of 32 the last word of a row
+// thus goes on with the row's first cells, so that a tile reads the periodic
+// row as a string of words.
+//
+// Word j of that string for -1 <= j <= wd, as the bits [sh, sh + 32) of words
+// o0 (low) and o1 (high).  Word -1 ends at cell n0 - 1, word wd starts at cell
+// 32 wd; words further out are never needed right (clamped to wd).
+struct ExtWord {
+  int o0, o1, sh;
+};
+__device__ __forceinline__ ExtWord ext_word(int j, int wd, int nb) {
+  if (j < 0) {  // cells n0 - 32 .. n0 - 1
+    if (nb == 32) return ExtWord{wd - 1, wd - 1, 0};
+    return ExtWord{wd - 2, wd - 1, nb};
+  }
+  if (j >= wd) {  // cells 32 wd mod n0 ..
+    if (nb == 32) return ExtWord{0, 0, 0};
+    return ExtWord{0, 1, 32 - nb};
+  }
+  return ExtWord{j, j, 0};
+}
 
 // Temporal blocking: each CTA owns a tw x th tile (words x rows), loads it
 // with a halo of 1 word and kk rows, advances kk generations in shared
@@ -489,34 +516,47 @@ life_tb_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next,
   }
 }
 
-// Row sums used by the sliding-window update: horizontal full-adder of the
-// three cells W, C, E of every bit position (f1 ones, f2 twos) and
-// half-adder of W, E (h1, h2), for one 32-cell word.
+// Row sums used by the sliding-window update: the two-bit sum (f1 ones, f2
+// twos) of the three cells W, C, E of every bit position of one 32-cell word.
 struct RowSums {
-  uint32_t raw, f1, f2, h1, h2;
+  uint32_t raw, f1, f2;
 };
+
+// one three-input bit operation; LUT bit 4x + 2y + z gives its value at (x, y, z)
+template <int LUT>
+__device__ __forceinline__ uint32_t lop3(uint32_t x, uint32_t y, uint32_t z) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(x), "r"(y), "r"(z), "n"(LUT));
+  return d;
+}
+__device__ __forceinline__ uint32_t xor3(uint32_t x, uint32_t y, uint32_t z) {
+  return lop3<0x96>(x, y, z);
+}
+__device__ __forceinline__ uint32_t maj3(uint32_t x, uint32_t y, uint32_t z) {
+  return lop3<0xE8>(x, y, z);
+}
 
 __device__ __forceinline__ RowSums row_sums(uint32_t left, uint32_t w, uint32_t right) {
   const uint32_t W = __funnelshift_l(left, w, 1), E = __funnelshift_r(w, right, 1);
-  RowSums r;
-  r.raw = w;
-  r.f1 = W ^ w ^ E;
-  r.f2 = (W & w) | (E & (W ^ w));
-  r.h1 = W ^ E;
-  r.h2 = W & E;
-  return r;
+  return RowSums{w, xor3(W, w, E), maj3(W, w, E)};
 }
 
-// next state of the middle row b from the sums of rows a (above), b, c:
-// num = s0 + 2*(u + k0) with u = a2 + b2 + c2; alive' = (num==3) | (b & num==2)
-// = (u + k0 == 1) & (s0 | b) = ~u2 & (u1 ^ k0) & (s0 | b).
+// next state of the middle row b from the sums of rows a (above), b, c.  The
+// sum of all nine cells is u0 + 2 (k0 + u1) + 4 u2; a cell lives when it is 3,
+// or 4 with the cell itself alive.  With one = exactly one of (k0, u1, u2):
+//   u0 = 1: sum 3 is one & ~u2;  u0 = 0: sum 4 is u2 ? one : ~one (sum 0 also
+//   gives ~one, but not with the cell alive),
+// and the result is that & (u0 | b).  Nine three-input operations a word with
+// the two of row_sums; the ALU takes 64 lanes a cycle per SM and these, the
+// two shifts and the count are what bounds every packed kernel (the half-adder
+// of the middle row that this form does without made it eleven).
 __device__ __forceinline__ uint32_t life_from_sums(const RowSums &a, const RowSums &b,
                                                    const RowSums &c) {
-  const uint32_t s0 = a.f1 ^ b.h1 ^ c.f1;
-  const uint32_t k0 = (a.f1 & b.h1) | (c.f1 & (a.f1 ^ b.h1));
-  const uint32_t u1 = a.f2 ^ b.h2 ^ c.f2;
-  const uint32_t u2 = (a.f2 & b.h2) | (c.f2 & (a.f2 ^ b.h2));
-  return ~u2 & (u1 ^ k0) & (s0 | b.raw);
+  const uint32_t u0 = xor3(a.f1, b.f1, c.f1), k0 = maj3(a.f1, b.f1, c.f1);
+  const uint32_t u1 = xor3(a.f2, b.f2, c.f2), u2 = maj3(a.f2, b.f2, c.f2);
+  const uint32_t one = lop3<0x16>(k0, u1, u2);
+  const uint32_t hit = lop3<0x29>(u0, u2, one);
+  return lop3<0xE0>(hit, u0, b.raw);
 }
 
 // Whole grid in registers, one packed word per thread: all `gens`
@@ -552,8 +592,9 @@ life_smallreg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next
   const int wup = warp == 0 ? nw - 1 : warp - 1, wdown = warp == nw - 1 ? 0 : warp + 1;
   for (int g = 0; g < gens; ++g) {
     const int b = g & 1;
-    const RowSums me = row_sums(__shfl_sync(0xffffffffu, w, west), w,
-                                __shfl_sync(0xffffffffu, w, east));
+    const uint32_t wl = __shfl_sync(0xffffffffu, w, west), wr = __shfl_sync(0xffffffffu, w, east);
+    const uint32_t W = __funnelshift_l(wl, w, 1), E = __funnelshift_r(w, wr, 1);
+    const RowSums me{w, xor3(W, w, E), maj3(W, w, E)};
     if (first) {
       top[b][warp][0][x] = me.f1;
       top[b][warp][1][x] = me.f2;
@@ -576,7 +617,12 @@ life_smallreg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next
       c.f1 = top[b][wdown][0][x];
       c.f2 = top[b][wdown][1][x];
     }
-    w = life_from_sums(a, me, c);
+    // the neighbours only (h1, h2: W + E): one operation more than
+    // life_from_sums but a shorter chain, which is what bounds this kernel
+    const uint32_t h1 = W ^ E, h2 = W & E;
+    const uint32_t s0 = xor3(a.f1, h1, c.f1), k0 = maj3(a.f1, h1, c.f1);
+    const uint32_t u1 = xor3(a.f2, h2, c.f2), u2 = maj3(a.f2, h2, c.f2);
+    w = ~u2 & (u1 ^ k0) & (s0 | w);
     const uint32_t cnt = __reduce_add_sync(0xffffffffu, __popc(w));
     if (lane == 0 && cnt) atomicAdd(&pop[g], cnt);
   }
@@ -674,6 +720,54 @@ life_tb32_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, Tb
   }
 }
 
+// row sums of a row of one word per lane
+__device__ __forceinline__ RowSums lane_sums(uint32_t w) {
+  return row_sums(__shfl_up_sync(0xffffffffu, w, 1), w, __shfl_down_sync(0xffffffffu, w, 1));
+}
+
+// One generation of a warp's R rows of 32 words in registers; the block's
+// warps are stacked, and each trades the row sums of its first and last row
+// with its neighbours through ex (NW x 2 x 32 pairs, double-buffered by the
+// caller).  The rows between are advanced before the wait: a warp's neighbours
+// have then written theirs, and only the two edge rows follow it.  `arrive`
+// publishes this warp's sums, `wait` waits for the neighbours'.  Returns the
+// lane's count of living cells: of all rows (whole) or of the owned rows and
+// bits only.
+template <int R, int NW, class Arrive, class Wait>
+__device__ __forceinline__ uint32_t life_generation(uint32_t (&rows)[R], uint2 (*ex)[2][32],
+                                                    int warp, int lane, bool whole,
+                                                    uint32_t ownrows, uint32_t colmask, Arrive arrive,
+                                                    Wait wait) {
+  const RowSums s0 = lane_sums(rows[0]), sl = lane_sums(rows[R - 1]);
+  ex[warp][0][lane] = make_uint2(s0.f1, s0.f2);
+  ex[warp][1][lane] = make_uint2(sl.f1, sl.f2);
+  arrive();
+  uint32_t cnt = 0;
+  RowSums ra = s0, rb = lane_sums(rows[1]);
+  const RowSums s1 = rb;
+#pragma unroll
+  for (int i = 1; i < R - 1; ++i) {
+    const RowSums rc = i + 1 < R - 1 ? lane_sums(rows[i + 1]) : sl;
+    rows[i] = life_from_sums(ra, rb, rc);
+    if (whole) cnt += __popc(rows[i]);
+    else if (ownrows & (1u << i)) cnt += __popc(rows[i] & colmask);
+    ra = rb;
+    rb = rc;
+  }
+  wait();
+  const uint2 up = warp > 0 ? ex[warp - 1][1][lane] : make_uint2(0u, 0u);
+  const uint2 down = warp < NW - 1 ? ex[warp + 1][0][lane] : make_uint2(0u, 0u);
+  rows[0] = life_from_sums(RowSums{0u, up.x, up.y}, s0, s1);
+  rows[R - 1] = life_from_sums(ra, sl, RowSums{0u, down.x, down.y});
+  if (whole) {
+    cnt += __popc(rows[0]) + __popc(rows[R - 1]);
+  } else {
+    if (ownrows & 1u) cnt += __popc(rows[0] & colmask);
+    if (ownrows & (1u << (R - 1))) cnt += __popc(rows[R - 1] & colmask);
+  }
+  return cnt;
+}
+
 // Register-resident temporal blocking.  A block is NW warps x R rows of 32
 // packed words (30 owned + halo word each side); warp w keeps rows
 // [wR, wR+R) in registers for all kk generations and trades only its first
@@ -681,17 +775,29 @@ life_tb32_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, Tb
 // generation.  Rows are not shrunk per generation: the stale front from the
 // block's outer rows and columns moves one cell per generation and never
 // reaches the owned rows [kk, kk + th_own) and words 1..tw_own.
-template <int R, int NW, bool VEC>
-__global__ void __launch_bounds__(NW * 32, (NW >= 16 ? 2 : 4))
-life_reg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbParams p,
+//
+// IO: what the tile is read from and written to.  A run of many generations
+// takes the cells in once and out once: its first launch reads int32 cells and
+// writes the packed grid, its last one reads the packed grid and writes cells,
+// and those between stay packed (1/32 of the bytes, rows loaded straight into
+// registers and stored from them).  Any row length is served where both ends
+// are packed.
+enum LifeIo { kCellsToCells = 0, kCellsToPacked = 1, kPackedToPacked = 2, kPackedToCells = 3 };
+
+template <int R, int NW, bool VEC, int IO = kCellsToCells>
+__global__ void __launch_bounds__(NW * 32, (NW >= 32 ? 1 : NW >= 16 ? 2 : 4))
+life_reg_kernel(const void *__restrict__ in, void *__restrict__ out, TbParams p,
                 uint32_t *__restrict__ pop) {
   constexpr int NC = 32, NR = R * NW;
-  extern __shared__ uint32_t A[];  // NR x NC packed words
-  __shared__ uint32_t ex[2][NW][2][NC];
+  constexpr bool PIN = IO == kPackedToPacked || IO == kPackedToCells;
+  constexpr bool POUT = IO == kPackedToPacked || IO == kCellsToPacked;
+  extern __shared__ uint32_t A[];  // NR x NC packed words (not with both ends packed)
+  __shared__ uint2 ex[2][NW][2][NC];
   __shared__ uint32_t spop[32];
   __shared__ int4 nib[16];  // nibble -> its four cells
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 16) nib[tid] = make_int4(tid & 1, (tid >> 1) & 1, (tid >> 2) & 1, (tid >> 3) & 1);
+  if (!POUT && tid < 16)
+    nib[tid] = make_int4(tid & 1, (tid >> 1) & 1, (tid >> 2) & 1, (tid >> 3) & 1);
   const int t = blockIdx.x;
   const int t0 = t % p.nt0, t1 = t / p.nt0;
   // tiles split the grid evenly (sizes differ by at most one word / row)
@@ -701,14 +807,36 @@ life_reg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbP
   const int th_own = (int)((long long)(t1 + 1) * p.n1 / p.nt1) - row0;
   const int kk = p.kk;
   if (tid < 32) spop[tid] = 0;
-  if (VEC)
-    pack_rows32(cur, p.n0, p.n1, p.wd, row0 - kk, col0 - 1, NR, A, warp, NW, lane);
-  else
-    pack_rows(cur, p.n0, p.n1, p.wd, row0 - kk, col0 - 1, NC, NR, A, warp, NW, lane);
-  __syncthreads();
   uint32_t rows[R];
+  if (PIN) {
+    const uint32_t *src = (const uint32_t *)in;
+    const ExtWord e = ext_word(min(col0 - 1 + lane, p.wd), p.wd, p.nb);
+    // the block's rows kk + th_own + kk reach; the rest repeat its last one
+    int gy = (row0 - kk + min(warp * R, th_own + 2 * kk - 1)) % p.n1;
+    if (gy < 0) gy += p.n1;
+    int left = th_own + 2 * kk - 1 - min(warp * R, th_own + 2 * kk - 1);
 #pragma unroll
-  for (int i = 0; i < R; ++i) rows[i] = A[(warp * R + i) * NC + lane];
+    for (int i = 0; i < R; ++i) {
+      const uint32_t *row = src + (size_t)gy * p.wd;
+      rows[i] = p.nb == 32 ? row[e.o0] : __funnelshift_r(row[e.o0], row[e.o1], e.sh);
+      if (left > 0) {
+        --left;
+        if (++gy == p.n1) gy = 0;
+      }
+    }
+    __syncthreads();
+  } else {
+    const int32_t *cur = (const int32_t *)in;
+    if (VEC)
+      pack_rows32(cur, p.n0, p.n1, p.wd, row0 - kk, col0 - 1, min(NR, th_own + 2 * kk), A, warp,
+                  NW, lane);
+    else
+      pack_rows(cur, p.n0, p.n1, p.wd, row0 - kk, col0 - 1, NC, min(NR, th_own + 2 * kk), A, warp,
+                NW, lane);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < R; ++i) rows[i] = A[(warp * R + i) * NC + lane];
+  }
   // owned rows of this warp as a bit mask; owned columns as a lane mask
   uint32_t ownrows = 0;
 #pragma unroll
@@ -716,51 +844,38 @@ life_reg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbP
     const int gr = warp * R + i - kk;
     if (gr >= 0 && gr < th_own) ownrows |= 1u << i;
   }
-  const uint32_t colmask = (lane >= 1 && lane <= tw_own) ? ~0u : 0u;
+  uint32_t colmask = (lane >= 1 && lane <= tw_own) ? ~0u : 0u;
+  // the last word of a row that is no whole number of words counts nb cells
+  const bool ragged = PIN && POUT && p.nb != 32 && col0 + tw_own == p.wd;
+  if (ragged && lane == tw_own) colmask = (1u << p.nb) - 1u;
   // most warps own all their rows or none: those count every row and keep
   // the lane's count only if the lane and the rows are owned (no per-row
   // test); the warps on the block's halo edges test each row
   constexpr uint32_t allrows = R == 32 ? ~0u : ((1u << R) - 1u);
+  const bool whole = ownrows == 0u || (ownrows == allrows && !ragged);
+  auto arrive = [] {};
+  auto wait = [] { __syncthreads(); };
   for (int g = 0; g < kk; ++g) {
-    const int b = g & 1;
-    ex[b][warp][0][lane] = rows[0];
-    ex[b][warp][1][lane] = rows[R - 1];
-    __syncthreads();
-    const uint32_t up = warp > 0 ? ex[b][warp - 1][1][lane] : 0u;
-    const uint32_t down = warp < NW - 1 ? ex[b][warp + 1][0][lane] : 0u;
-    RowSums ra = row_sums(__shfl_up_sync(0xffffffffu, up, 1), up,
-                          __shfl_down_sync(0xffffffffu, up, 1));
-    RowSums rb = row_sums(__shfl_up_sync(0xffffffffu, rows[0], 1), rows[0],
-                          __shfl_down_sync(0xffffffffu, rows[0], 1));
-    uint32_t cnt = 0;
-    if (ownrows == allrows || ownrows == 0u) {
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const uint32_t wn = (i + 1 < R) ? rows[i + 1] : down;
-        const RowSums rc = row_sums(__shfl_up_sync(0xffffffffu, wn, 1), wn,
-                                    __shfl_down_sync(0xffffffffu, wn, 1));
-        const uint32_t out = life_from_sums(ra, rb, rc);
-        rows[i] = out;
-        cnt += __popc(out);
-        ra = rb;
-        rb = rc;
-      }
-      cnt &= ownrows == allrows ? colmask : 0u;
-    } else {
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const uint32_t wn = (i + 1 < R) ? rows[i + 1] : down;
-        const RowSums rc = row_sums(__shfl_up_sync(0xffffffffu, wn, 1), wn,
-                                    __shfl_down_sync(0xffffffffu, wn, 1));
-        const uint32_t out = life_from_sums(ra, rb, rc);
-        rows[i] = out;
-        if (ownrows & (1u << i)) cnt += __popc(out & colmask);
-        ra = rb;
-        rb = rc;
-      }
-    }
+    uint32_t cnt;
+    if (whole)
+      cnt = life_generation<R, NW>(rows, ex[g & 1], warp, lane, true, ownrows, colmask, arrive,
+                                   wait) &
+            (ownrows == allrows ? colmask : 0u);
+    else
+      cnt = life_generation<R, NW>(rows, ex[g & 1], warp, lane, false, ownrows, colmask, arrive,
+                                   wait);
     cnt = __reduce_add_sync(0xffffffffu, cnt);
     if (lane == 0 && cnt) atomicAdd(&spop[g], cnt);
+  }
+  if (POUT) {
+    uint32_t *dst =
+        (uint32_t *)out + (ptrdiff_t)(row0 + warp * R - kk) * p.wd + (col0 + lane - 1);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if ((ownrows & (1u << i)) && lane >= 1 && lane <= tw_own) dst[(size_t)i * p.wd] = rows[i];
+    __syncthreads();
+    if (tid < kk && spop[tid]) atomicAdd(&pop[tid], spop[tid]);
+    return;
   }
   __syncthreads();
 #pragma unroll
@@ -770,7 +885,7 @@ life_reg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbP
   const int sub = lane >> 3, quad = (lane & 7) * 4;
   for (int r = warp; r < th_own; r += NW) {
     const uint32_t *src = A + (r + kk) * NC + 1;
-    int32_t *dst = next + (size_t)(row0 + r) * p.n0 + (size_t)col0 * 32;
+    int32_t *dst = (int32_t *)out + (size_t)(row0 + r) * p.n0 + (size_t)col0 * 32;
     if (VEC) {
       // four cells of a word per lane, as the four cells of a nibble
       for (int c0 = 0; c0 < tw_own; c0 += 16) {
@@ -785,6 +900,58 @@ life_reg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbP
     } else {
       for (int c = 0; c < tw_own; ++c)
         dst[(size_t)c * 32 + lane] = (int32_t)((src[c] >> lane) & 1u);
+    }
+  }
+}
+
+// The packed grid of cells that are all 0 or 1 (rows of any length), one warp
+// per eight words at a time.
+__global__ void __launch_bounds__(256)
+life_pack_kernel(const int32_t *__restrict__ cells, uint32_t *__restrict__ packed, int n0, int n1,
+                 int wd) {
+  const int lane = threadIdx.x & 31;
+  const int groups = (wd + 7) / 8;
+  const long long total = (long long)groups * n1;
+  const long long step = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total;
+       i += step) {
+    const int y = (int)(i / groups), w0 = (int)(i - (long long)y * groups) * 8;
+    const int32_t *row = cells + (size_t)y * n0;
+    int32_t v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      int x = (w0 + j) * 32 + lane;
+      if (x >= n0) x -= n0;  // the row goes on with its first cells (n0 > 32)
+      v[j] = w0 + j < wd ? __ldg(row + x) : 0;
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t w = __ballot_sync(0xffffffffu, v[j] != 0);
+      if (lane == j) mine = w;
+    }
+    if (lane < 8 && w0 + lane < wd) packed[(size_t)y * wd + w0 + lane] = mine;
+  }
+}
+
+// and back: one warp per eight words of a row
+__global__ void __launch_bounds__(256)
+life_unpack_kernel(const uint32_t *__restrict__ packed, int32_t *__restrict__ cells, int n0, int n1,
+                   int wd) {
+  const int lane = threadIdx.x & 31;
+  const int groups = (wd + 7) / 8;
+  const long long total = (long long)groups * n1;
+  const long long step = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total;
+       i += step) {
+    const int y = (int)(i / groups), w0 = (int)(i - (long long)y * groups) * 8;
+    const uint32_t mine = packed[(size_t)y * wd + min(w0 + (lane & 7), wd - 1)];
+    int32_t *row = cells + (size_t)y * n0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t w = __shfl_sync(0xffffffffu, mine, j);
+      const int x = (w0 + j) * 32 + lane;
+      if (x < n0) row[x] = (int32_t)((w >> lane) & 1u);
     }
   }
 }
@@ -820,14 +987,19 @@ __host__ __device__ constexpr bool kStagedPack() {
 // PS: consumer warps synchronise each generation with their two neighbours
 // only (an mbarrier per warp and buffer parity, signalled once the warp's
 // boundary rows are written), instead of a barrier over all consumers
-template <int R, int NWC, int NWP, int NWS, bool TMA = false, int NS = 2, bool PS = false>
+// IO: the first launch of a long run writes the packed grid and the last one
+// reads it (see LifeIo); their store or producer warps then move 1/32 of the
+// bytes with plain word accesses.
+template <int R, int NWC, int NWP, int NWS, bool TMA = false, int NS = 2, bool PS = false,
+          int IO = kCellsToCells>
 __global__ void __launch_bounds__((NWC + NWP + NWS) * 32, 1)
-life_ws_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbParams p,
+life_ws_kernel(const void *__restrict__ in, void *__restrict__ out, TbParams p,
                uint32_t *__restrict__ pop, const __grid_constant__ CUtensorMap tmap,
                const __grid_constant__ CUtensorMap tpatch, uint32_t *err) {
+  const int32_t *cur = (const int32_t *)in;
+  int32_t *next = (int32_t *)out;
   constexpr int NC = 32, NR = R * NWC;
   extern __shared__ __align__(1024) uint32_t buf[];  // 3 x NR x NC packed words
-  __shared__ uint32_t ex[2][NWC][2][NC];
   __shared__ uint32_t spop[32];
   __shared__ int4 nib[16];  // nibble -> its four cells
   __shared__ uint64_t bars[NWP][NS];
@@ -854,6 +1026,12 @@ life_ws_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbPa
     const int col0 = (t % p.nt0) * p.tw, row0 = (t / p.nt0) * p.th;
     const int tw_own = min(p.tw, p.wd - col0), th_own = min(p.th, p.n1 - row0);
     const int sub = lane >> 3, quad = (lane & 7) * 4;
+    if (IO == kCellsToPacked) {
+      for (int r = sw; r < th_own; r += nsw)
+        if (lane < tw_own)
+          ((uint32_t *)out)[(size_t)(row0 + r) * p.wd + col0 + lane] = A[(r + kk) * NC + 1 + lane];
+      return;
+    }
     for (int r = sw; r < th_own; r += nsw) {
       const uint32_t *src = A + (r + kk) * NC + 1;
       int32_t *dst = next + (size_t)(row0 + r) * p.n0 + (size_t)col0 * 32 + quad;
@@ -870,6 +1048,24 @@ life_ws_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbPa
   auto pack_tile = [&](int s, int pw, int npw) {
     const int t = blockIdx.x + s * gridDim.x;
     const int col0 = (t % p.nt0) * p.tw, row0 = (t / p.nt0) * p.th;
+    if (IO == kPackedToCells) {
+      const uint32_t *src =
+          (const uint32_t *)in + ext_word(min(col0 - 1 + lane, p.wd), p.wd, 32).o0;
+      uint32_t *dst = buf + (s % 3) * NR * NC + lane;
+      for (int r0 = pw; r0 < NR; r0 += 4 * npw) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          int gy = (row0 - kk + min(r0 + k * npw, NR - 1)) % p.n1;
+          if (gy < 0) gy += p.n1;
+          w[k] = src[(size_t)gy * p.wd];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (r0 + k * npw < NR) dst[(r0 + k * npw) * NC] = w[k];
+      }
+      return;
+    }
     pack_rows32(cur, p.n0, p.n1, p.wd, row0 - kk, col0 - 1, NR, buf + (s % 3) * NR * NC, pw,
                 npw, lane);
   };
@@ -957,6 +1153,10 @@ life_ws_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbPa
         uint32_t rows[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) rows[i] = A[(warp * R + i) * NC + lane];
+        // while the rows are in registers their buffer holds the exchange
+        static_assert(R >= 8, "the exchange fits in the tile's buffer");
+        uint2(*ex)[NWC][2][NC] = reinterpret_cast<uint2(*)[NWC][2][NC]>(A);
+        asm volatile("bar.sync 1, %0;" ::"r"(NWC * 32) : "memory");
         uint32_t ownrows = 0;
 #pragma unroll
         for (int i = 0; i < R; ++i) {
@@ -964,67 +1164,50 @@ life_ws_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, TbPa
           if (gr >= 0 && gr < th_own) ownrows |= 1u << i;
         }
         const uint32_t colmask = (lane >= 1 && lane <= tw_own) ? ~0u : 0u;
+        constexpr uint32_t allrows = R == 32 ? ~0u : ((1u << R) - 1u);
+        const bool whole = ownrows == allrows || ownrows == 0u;
         for (int g = 0; g < kk; ++g) {
           const int b = PS ? (int)(G & 1u) : (g & 1);
-          ex[b][warp][0][lane] = rows[0];
-          ex[b][warp][1][lane] = rows[R - 1];
-          if (PS) {
+          auto arrive = [&] {
             // A neighbour is at most one use ahead on a buffer: to arrive
             // again it must first see this warp's next generation.  It
             // reads a buffer before it signals the next generation, so
             // this warp's rewrite two generations on cannot overtake it.
-            __syncwarp();
-            if (lane == 0) tma::mbar_arrive(&cbar[warp][b]);
-            const uint32_t par = (G >> 1) & 1u;
-            if (warp > 0) tma::mbar_wait(&cbar[warp - 1][b], par, err);
-            if (warp < NWC - 1) tma::mbar_wait(&cbar[warp + 1][b], par, err);
-            ++G;
-          } else {
-            asm volatile("bar.sync 1, %0;" ::"r"(NWC * 32) : "memory");
-          }
-          const uint32_t up = warp > 0 ? ex[b][warp - 1][1][lane] : 0u;
-          const uint32_t down = warp < NWC - 1 ? ex[b][warp + 1][0][lane] : 0u;
-          RowSums ra = row_sums(__shfl_up_sync(0xffffffffu, up, 1), up,
-                                __shfl_down_sync(0xffffffffu, up, 1));
-          RowSums rb = row_sums(__shfl_up_sync(0xffffffffu, rows[0], 1), rows[0],
-                                __shfl_down_sync(0xffffffffu, rows[0], 1));
-          uint32_t cnt = 0;
-          constexpr uint32_t allrows = R == 32 ? ~0u : ((1u << R) - 1u);
-          if (ownrows == allrows || ownrows == 0u) {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-              const uint32_t wn = (i + 1 < R) ? rows[i + 1] : down;
-              const RowSums rc = row_sums(__shfl_up_sync(0xffffffffu, wn, 1), wn,
-                                          __shfl_down_sync(0xffffffffu, wn, 1));
-              const uint32_t out = life_from_sums(ra, rb, rc);
-              rows[i] = out;
-              cnt += __popc(out);
-              ra = rb;
-              rb = rc;
+            if (PS) {
+              __syncwarp();
+              if (lane == 0) tma::mbar_arrive(&cbar[warp][b]);
             }
-            cnt &= ownrows == allrows ? colmask : 0u;
-          } else {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-              const uint32_t wn = (i + 1 < R) ? rows[i + 1] : down;
-              const RowSums rc = row_sums(__shfl_up_sync(0xffffffffu, wn, 1), wn,
-                                          __shfl_down_sync(0xffffffffu, wn, 1));
-              const uint32_t out = life_from_sums(ra, rb, rc);
-              rows[i] = out;
-              if (ownrows & (1u << i)) cnt += __popc(out & colmask);
-              ra = rb;
-              rb = rc;
+          };
+          auto wait = [&] {
+            if (PS) {
+              const uint32_t par = (G >> 1) & 1u;
+              if (warp > 0) tma::mbar_wait(&cbar[warp - 1][b], par, err);
+              if (warp < NWC - 1) tma::mbar_wait(&cbar[warp + 1][b], par, err);
+              ++G;
+            } else {
+              asm volatile("bar.sync 1, %0;" ::"r"(NWC * 32) : "memory");
             }
-          }
+          };
+          uint32_t cnt;
+          if (whole)
+            cnt = life_generation<R, NWC>(rows, ex[b], warp, lane, true, ownrows, colmask, arrive,
+                                          wait) &
+                  (ownrows == allrows ? colmask : 0u);
+          else
+            cnt = life_generation<R, NWC>(rows, ex[b], warp, lane, false, ownrows, colmask,
+                                          arrive, wait);
           cnt = __reduce_add_sync(0xffffffffu, cnt);
           if (lane == 0 && cnt) atomicAdd(&spop[g], cnt);
         }
+        asm volatile("bar.sync 1, %0;" ::"r"(NWC * 32) : "memory");
 #pragma unroll
         for (int i = 0; i < R; ++i) A[(warp * R + i) * NC + lane] = rows[i];
       }
     } else if (warp < NWC + NWP) {
       if (s < m)
-        if (TMA) {
+        if (IO == kPackedToCells) {
+          pack_tile(s, warp - NWC, NWP);
+        } else if (TMA) {
           // rows pw, pw + NWP, ... of tile s, NS - 1 boxes ahead (the first
           // rows of tile s + 1 follow the last of tile s); a slot is issued
           // into only after the row it held was packed
@@ -1096,9 +1279,40 @@ __global__ void life_finalize_kernel(LifeScalars *s, const uint32_t *pop, int n)
 // ones spread over every SM with the temporally blocked tiles.
 static const int kSmallMaxWords = 4096;
 
+// whether packed kernels serve the grid: every cell 0 or 1, cyclic, rows of
+// whole words or of at least one word and a cell
+static bool life_packed_ok(const Handle *h) {
+  return h->cyclic && h->cfg.variant == 0 && (h->size[0] % 32 == 0 || h->size[0] > 32);
+}
+
+// Whether a run of n generations goes through the packed grid: rows that are
+// no whole number of words from two generations on (a single one is cheaper
+// one cell per thread than packed, advanced and unpacked), others with no
+// launch knob set, beyond the one-CTA grids, when one launch of at most 32
+// generations cannot do.
+static bool life_run_packed(const Handle *h, int n) {
+  if (!life_packed_ok(h)) return false;
+  if (h->size[0] % 32 != 0) return n >= 2;
+  const om_config &c = h->cfg;
+  return n > 32 && (long long)(h->size[0] / 32) * h->size[1] > kSmallMaxWords && c.depth == 0 &&
+         c.tile_x == 0 && c.tile_y == 0 && c.life_kernel == 0 && c.life_io == 0 &&
+         c.grid_limit == 0;
+}
+
 static om_status life_reserve(Handle *h, int kernel_id, int n) {
-  (void)kernel_id;
   LifeState *st = life_state(h);
+  if (h->kernels[kernel_id].name == "proceed" && !st->packed[0] && life_run_packed(h, n)) {
+    const size_t words = (size_t)((h->size[0] + 31) / 32) * h->size[1];
+    for (int i = 0; i < 2; ++i)
+      if (injected_alloc_failure() ||
+          cudaMalloc(&st->packed[i], words * sizeof(uint32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(st->packed[0]);
+        st->packed[0] = st->packed[1] = nullptr;
+        set_error("Life: cannot allocate the packed grid");
+        return OM_ERR_NOMEM;
+      }
+  }
   if (n <= st->pop_cap) return OM_OK;
   int cap = std::max(n, 1024);
   uint32_t *p = nullptr;
@@ -1136,7 +1350,7 @@ static cudaError_t launch_reg(int v, const int32_t *cur, int32_t *next, const Tb
                               uint32_t *pop, cudaStream_t s) {
   const RegVariant rv = kRegVariants[v];
   const size_t smem = sizeof(uint32_t) * 32 * rv.R * rv.NW;
-  void (*k)(const int32_t *, int32_t *, TbParams, uint32_t *) = nullptr;
+  void (*k)(const void *, void *, TbParams, uint32_t *) = nullptr;
   switch (v) {
     case 0: k = life_reg_kernel<16, 8, VEC>; break;
     case 1: k = life_reg_kernel<24, 8, VEC>; break;
@@ -1176,7 +1390,9 @@ static const int kAutoWsVariant = 3;
 
 // `tmap`, `tpatch`: the tensor maps of `cur` for the TMA variants (ignored
 // by the others); at most `ctas` persistent CTAs
-static cudaError_t launch_ws(int v, const int32_t *cur, int32_t *next, const TbParams &p,
+// io: kCellsToCells, or the first or last launch of a packed run (automatic
+// variants only)
+static cudaError_t launch_ws(int v, int io, const void *cur, void *next, const TbParams &p,
                              uint32_t *pop, int ctas, const CUtensorMap &tmap,
                              const CUtensorMap &tpatch, uint32_t *err, cudaStream_t s) {
   const WsVariant wv = kWsVariants[v];
@@ -1189,9 +1405,15 @@ static cudaError_t launch_ws(int v, const int32_t *cur, int32_t *next, const TbP
     // three tile buffers, then two staged rows (2 x 4 KB) per producer warp
     smem += sizeof(int4) * 512 * wv.NWP;
   }
-  void (*k)(const int32_t *, int32_t *, TbParams, uint32_t *, const CUtensorMap,
-            const CUtensorMap, uint32_t *) = nullptr;
-  switch (v) {
+  void (*k)(const void *, void *, TbParams, uint32_t *, const CUtensorMap, const CUtensorMap,
+            uint32_t *) = nullptr;
+  if (io == kCellsToPacked)
+    k = v == kAutoWsVariantTma ? life_ws_kernel<22, 16, 8, 8, true, 2, false, kCellsToPacked>
+                               : life_ws_kernel<20, 16, 8, 8, false, 2, false, kCellsToPacked>;
+  else if (io == kPackedToCells)
+    k = v == kAutoWsVariantTma ? life_ws_kernel<22, 16, 8, 8, true, 2, false, kPackedToCells>
+                               : life_ws_kernel<20, 16, 8, 8, false, 2, false, kPackedToCells>;
+  else switch (v) {
     case 0: k = life_ws_kernel<24, 16, 8, 8>; break;
     case 1: k = life_ws_kernel<16, 16, 8, 8>; break;
     case 2: k = life_ws_kernel<24, 16, 12, 4>; break;
@@ -1227,7 +1449,7 @@ static int reg_occupancy(int device, int v, bool vec) {
   if (known) return known;
   const RegVariant rv = kRegVariants[v];
   const size_t smem = sizeof(uint32_t) * 32 * rv.R * rv.NW;
-  void (*k)(const int32_t *, int32_t *, TbParams, uint32_t *) = nullptr;
+  void (*k)(const void *, void *, TbParams, uint32_t *) = nullptr;
   switch (v) {
     case 0: k = vec ? life_reg_kernel<16, 8, true> : life_reg_kernel<16, 8, false>; break;
     case 1: k = vec ? life_reg_kernel<24, 8, true> : life_reg_kernel<24, 8, false>; break;
@@ -1285,6 +1507,132 @@ static int reg_plan(int device, bool vec, int wd, int n1, int kk, int *nt0_out, 
   return best_v;
 }
 
+// Variants of the register kernel with a packed end or two (R rows x NW
+// warps): short blocks let a grid of a few million cells spread over every SM
+// (2048^2 x 100: 126-128 us with 64- to 128-row blocks, 168 with 192 rows, 230
+// with 320), tall ones waste less on halo rows where tiles are many (16384^2:
+// 1936 us with 64 rows, 1290 with 192, 1176 with 384).
+static const RegVariant kPackedVariants[] = {{4, 16}, {6, 16}, {8, 16}, {12, 16},
+                                             {16, 16}, {20, 16}, {24, 16}, {8, 8}};
+static const int kNumPackedVariants = 8;
+
+typedef void (*RegKernel)(const void *, void *, TbParams, uint32_t *);
+template <int IO> static RegKernel packed_kernel(int v) {
+  switch (v) {
+    case 0: return life_reg_kernel<4, 16, true, IO>;
+    case 1: return life_reg_kernel<6, 16, true, IO>;
+    case 2: return life_reg_kernel<8, 16, true, IO>;
+    case 3: return life_reg_kernel<12, 16, true, IO>;
+    case 4: return life_reg_kernel<16, 16, true, IO>;
+    case 5: return life_reg_kernel<20, 16, true, IO>;
+    case 6: return life_reg_kernel<24, 16, true, IO>;
+    default: return life_reg_kernel<8, 8, true, IO>;
+  }
+}
+static RegKernel packed_kernel(int v, int io) {
+  return io == kCellsToPacked   ? packed_kernel<kCellsToPacked>(v)
+         : io == kPackedToCells ? packed_kernel<kPackedToCells>(v)
+                                : packed_kernel<kPackedToPacked>(v);
+}
+static size_t packed_smem(int v, int io) {
+  return io == kPackedToPacked
+             ? 0
+             : sizeof(uint32_t) * 32 * kPackedVariants[v].R * kPackedVariants[v].NW;
+}
+
+// resident blocks per SM of a packed variant (queried once per device)
+static int packed_occupancy(int device, int v, int io) {
+  static std::atomic<int> cache[64][kNumPackedVariants][4];
+  if (device < 0 || device >= 64) return 1;
+  std::atomic<int> &c = cache[device][v][io];
+  const int known = c.load(std::memory_order_relaxed);
+  if (known) return known;
+  const RegKernel k = packed_kernel(v, io);
+  const size_t smem = packed_smem(v, io);
+  int n = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kPackedVariants[v].NW * 32, smem) !=
+          cudaSuccess ||
+      n < 1) {
+    cudaGetLastError();
+    n = 1;
+  }
+  c.store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// A launch of the packed register kernel: variant, generations, tile grid.
+struct PackedPlan {
+  int v, kk, nt0, nt1;
+  double cycles;  // of the model below
+  double rate() const { return cycles / kk; }
+};
+
+// The plan of least modelled time over depths kmin .. kmax: per generation
+// (rate 0), or, for a run's first and last launch, beyond what its generations
+// would take at `rate` cycles each between them.
+// Per generation a block keeps a sub-partition's ALU busy for 22 cycles per
+// row of each of its warps (nine bit operations and two shifts at 16 lanes a
+// cycle), about two rows' worth for the exchanged rows and 40 for the count; a
+// block alone on its SM also waits about 250 for the exchange.  A launch costs
+// about 4000 cycles before and after, the packed rows' load and store 1500 a
+// round, and cells that are read or written 4 KB a row at about 48 bytes a
+// cycle.
+static PackedPlan packed_plan(int device, int wd, int n1, int io, int kmin, int kmax,
+                              double rate = 0) {
+  const int sms = sm_count(device);
+  PackedPlan best{-1, 1, 1, 1, 0};
+  double best_cost = 1e300;
+  for (int v = 0; v < kNumPackedVariants; ++v) {
+    const RegVariant rv = kPackedVariants[v];
+    const int NR = rv.R * rv.NW;
+    const int occ = packed_occupancy(device, v, io);
+    const double alu = rv.NW * ((rv.R + 2) * 22.0 + 40.0) / 4.0;
+    for (int kk = kmin; kk <= kmax; ++kk) {
+      const int thm = NR - 2 * kk;
+      if (thm < 4) break;
+      const int nt0min = (wd + 29) / 30, nt1min = (n1 + thm - 1) / thm;
+      for (int nt0 = nt0min; nt0 <= nt0min + 1 && nt0 <= wd; ++nt0) {
+        const long long tiles = (long long)nt0 * nt1min;
+        const long long per = (tiles + sms - 1) / sms;
+        const long long rounds = (per + occ - 1) / occ;
+        const double c = (double)std::min<long long>(per, occ);
+        double gen = std::max(c * alu, alu + 250.0) * (double)(per / occ);
+        if (per % occ) gen += std::max((double)(per % occ) * alu, alu + 250.0);
+        double cyc = 4000.0 + kk * gen + 1500.0 * (double)rounds;
+        if (io != kPackedToPacked) {
+          const int rows = (n1 + nt1min - 1) / nt1min + (io == kCellsToPacked ? 2 * kk : 0);
+          cyc += (double)per * rows * 4096.0 / 48.0;
+        }
+        const double cost = rate > 0 ? cyc - kk * rate : cyc / kk;
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = PackedPlan{v, kk, nt0, nt1min, cyc};
+        }
+      }
+    }
+  }
+  return best;
+}
+
+static om_status launch_packed(Handle *h, const PackedPlan &pl, int io, const void *in, void *out,
+                               TbParams p, uint32_t *pop) {
+  p.kk = pl.kk;
+  p.nt0 = pl.nt0;
+  p.nt1 = pl.nt1;
+  const RegKernel k = packed_kernel(pl.v, io);
+  const size_t smem = packed_smem(pl.v, io);
+  OM_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaEvent_t ev = prof_begin(h);
+  k<<<pl.nt0 * pl.nt1, kPackedVariants[pl.v].NW * 32, smem, h->stream>>>(in, out, p, pop);
+  OM_CUDA_CHECK(cudaGetLastError());
+  prof_end(h, ev, io == kPackedToPacked ? "life_packed_kernel" : "life_reg_kernel",
+           (double)p.n0 * p.n1 * pl.kk);
+  h->launches++;
+  return OM_OK;
+}
+
 // register variant for kk generations: the smallest block whose owned rows
 // (block rows - 2kk) reach the requested tile height (default 320, the
 // 24-row x 16-warp block at depth 32: fastest in the GB300 tile sweep)
@@ -1339,6 +1687,129 @@ static om_status launch_general(Handle *h, uint32_t *pop) {
   return OM_OK;
 }
 
+// the warp-specialised variant the automatic choice takes for tiles of depth
+// kk: on grids of at least 1.5 of its tiles per SM; -1 on smaller ones
+static int auto_ws_variant(Handle *h, int wd, int n1, int kk, bool tma_ok) {
+  const int av = tma_ok ? kAutoWsVariantTma : kAutoWsVariant;
+  const WsVariant wv = kWsVariants[av];
+  const int th = std::min(wv.R * wv.NWC - 2 * kk, n1);
+  const long long tiles = (long long)((wd + 29) / 30) * ((n1 + th - 1) / th);
+  return th > 0 && 2 * tiles >= 3LL * sm_count(h->device) ? av : -1;
+}
+
+static om_status launch_ws_tiles(Handle *h, int v, int io, const void *in, void *out, TbParams q,
+                                 int mi, uint32_t *pop) {
+  LifeState *st = life_state(h);
+  const WsVariant wv = kWsVariants[v];
+  q.tw = std::min(30, q.wd);
+  q.th = std::min(wv.R * wv.NWC - 2 * q.kk, q.n1);
+  q.nt0 = (q.wd + q.tw - 1) / q.tw;
+  q.nt1 = (q.n1 + q.th - 1) / q.th;
+  cudaEvent_t ev = prof_begin(h);
+  const int ctas = h->cfg.grid_limit > 0 ? std::min(h->cfg.grid_limit, sm_count(h->device))
+                                         : sm_count(h->device);
+  cudaError_t e = launch_ws(v, io, in, out, q, pop, ctas, st->tmap[mi < 0 ? 0 : mi],
+                            st->tpatch[mi < 0 ? 0 : mi],
+                            &((LifeScalars *)h->d_scalars)->wait_error, h->stream);
+  if (e != cudaSuccess) {
+    set_error(std::string("life_ws_kernel: ") + cudaGetErrorString(e));
+    return OM_ERR_CUDA;
+  }
+  prof_end(h, ev, wv.tma ? "life_ws_tma_kernel" : "life_ws_kernel",
+           (double)q.n0 * q.n1 * q.kk);
+  h->launches++;
+  return OM_OK;
+}
+
+// Generations per launch at the two ends of a packed run on the
+// warp-specialised kernel: fewer leave it waiting for the cells' 4 bytes each
+// (16384^2 x 100 generations: 1280 us at 8, 1230 at 12, 1176 at 22), more only
+// add halo rows (1189 at 26, 1207 at 30).
+static const int kWsEdgeDepth = 22;
+
+// Generations g .. n - 1 of a run through the packed grid.  With every launch
+// reading and writing int32 cells a 16384^2 run of 100 generations moved 9 GB
+// in four launches (1955 us); with the cells read once and written once it
+// takes 1176 us, bound by the ALU's bit operations (76 % of its cycles) between
+// the ends.  2048^2 x 100: 205 -> 128 us.  Rows of 1000 cells (1000 x 700 x
+// 100) no longer take a launch of the one-cell kernel per generation: 496 ->
+// 95 us.
+static om_status proceed_packed(Handle *h, int n, int g) {
+  LifeState *st = life_state(h);
+  if (!st->packed[0]) {
+    set_error("Life: packed grid not reserved");
+    return OM_ERR_STATE;
+  }
+  Array &a = h->arrays[0];
+  TbParams p{};
+  p.n0 = h->size[0];
+  p.n1 = h->size[1];
+  p.wd = (p.n0 + 31) / 32;
+  p.nb = p.n0 - 32 * (p.wd - 1);
+  const bool ragged = p.nb != 32;
+  uint32_t **pk = st->packed;
+  int cur = 0;
+  const long long rows8 = (long long)((p.wd + 7) / 8) * p.n1;
+  const unsigned io_grid =
+      (unsigned)std::max<long long>(1, std::min<long long>((rows8 + 7) / 8, 8LL * sm_count(h->device)));
+  int ws = -1, mi = -1, edge = 0;
+  PackedPlan first{}, last{};
+  if (ragged) {
+    cudaEvent_t ev = prof_begin(h);
+    life_pack_kernel<<<io_grid, 256, 0, h->stream>>>((const int32_t *)a.d(), pk[0], p.n0, p.n1,
+                                                     p.wd);
+    OM_CUDA_CHECK(cudaGetLastError());
+    prof_end(h, ev, "life_pack_kernel", 0.0);
+    h->launches++;
+  } else {
+    mi = p.wd >= 32 ? life_tmap(st, a.d(), p.n0, p.n1) : -1;
+    ws = auto_ws_variant(h, p.wd, p.n1, 32, mi >= 0);
+    if (ws >= 0) {
+      edge = std::min(kWsEdgeDepth, (n - g) / 2);
+      p.kk = edge;
+      OM_TRY(launch_ws_tiles(h, ws, kCellsToPacked, a.d(), pk[0], p, mi, st->d_pop + g));
+    } else {
+      const double rate = packed_plan(h->device, p.wd, p.n1, kPackedToPacked, 4, 32).rate();
+      const int most = std::min(24, (n - g) / 2);
+      first = packed_plan(h->device, p.wd, p.n1, kCellsToPacked, 1, most, rate);
+      last = packed_plan(h->device, p.wd, p.n1, kPackedToCells, 1, most, rate);
+      OM_TRY(launch_packed(h, first, kCellsToPacked, a.d(), pk[0], p, st->d_pop + g));
+      edge = last.kk;
+      g += first.kk - edge;
+    }
+    g += edge;
+  }
+  const int rem = n - g - edge;
+  if (rem > 0) {
+    // launches of near-equal depth, at most the best one
+    const int kbest =
+        packed_plan(h->device, p.wd, p.n1, kPackedToPacked, std::min(4, rem), std::min(32, rem)).kk;
+    const int nl = (rem + kbest - 1) / kbest;
+    for (int l = 0; l < nl; ++l) {
+      const int kk = rem / nl + (l < rem % nl ? 1 : 0);
+      const PackedPlan pl = packed_plan(h->device, p.wd, p.n1, kPackedToPacked, kk, kk);
+      OM_TRY(launch_packed(h, pl, kPackedToPacked, pk[cur], pk[1 - cur], p, st->d_pop + g));
+      cur = 1 - cur;
+      g += kk;
+    }
+  }
+  if (ragged) {
+    cudaEvent_t ev = prof_begin(h);
+    life_unpack_kernel<<<io_grid, 256, 0, h->stream>>>(pk[cur], (int32_t *)a.d_next(), p.n0, p.n1,
+                                                       p.wd);
+    OM_CUDA_CHECK(cudaGetLastError());
+    prof_end(h, ev, "life_unpack_kernel", 0.0);
+    h->launches++;
+  } else if (ws >= 0) {
+    p.kk = edge;
+    OM_TRY(launch_ws_tiles(h, ws, kPackedToCells, pk[cur], a.d_next(), p, -1, st->d_pop + g));
+  } else {
+    OM_TRY(launch_packed(h, last, kPackedToCells, pk[cur], a.d_next(), p, st->d_pop + g));
+  }
+  a.swap();
+  return OM_OK;
+}
+
 static om_status life_proceed(Handle *h, int n) {
   LifeState *st = life_state(h);
   if (n > st->pop_cap) {
@@ -1348,14 +1819,17 @@ static om_status life_proceed(Handle *h, int n) {
   Array &a = h->arrays[0];
   OM_CUDA_CHECK(cudaMemsetAsync(st->d_pop, 0, (size_t)n * sizeof(uint32_t), h->stream));
   const int n0 = h->size[0], n1 = h->size[1];
-  const bool packed_ok = h->cyclic && (n0 % 32 == 0) && h->cfg.variant == 0;
+  const bool ragged = n0 % 32 != 0;
+  const bool packed_ok = life_packed_ok(h) && (!ragged || n >= 2);
   int g = 0;
   if (!packed_ok || !st->binary) {
     const int first = packed_ok ? 1 : n;
     for (; g < first; ++g) OM_TRY(launch_general(h, st->d_pop + g));
     st->binary = true;
   }
-  if (g < n) {
+  if (g < n && (ragged || life_run_packed(h, n - g))) {
+    OM_TRY(proceed_packed(h, n, g));
+  } else if (g < n) {
     const int wd = n0 / 32;
     if (32 % wd == 0 && (n1 * wd) % 32 == 0 && n1 * wd <= 1024 && n1 * wd >= 32) {
       // one packed word per thread of one CTA, in registers
@@ -1380,7 +1854,7 @@ static om_status life_proceed(Handle *h, int n) {
       a.swap();
     } else {
       TbParams p;
-      p.n0 = n0; p.n1 = n1; p.wd = wd;
+      p.n0 = n0; p.n1 = n1; p.wd = wd; p.nb = 32;
       const bool l32 = life_pick_tiles(h, p);
       const bool reg = st->tile_w == 0;
       const int kmax = p.kk;
@@ -1407,13 +1881,7 @@ static om_status life_proceed(Handle *h, int n) {
       // the driver describes
       const bool tma_ok = wd >= 32 && life_tmap(st, a.d(), n0, n1) >= 0 &&
                           life_tmap(st, a.d_next(), n0, n1) >= 0;
-      if (reg && ws == 0 && st->tile_h == 0) {
-        const int av = tma_ok ? kAutoWsVariantTma : kAutoWsVariant;
-        const WsVariant wv = kWsVariants[av];
-        const int th = std::min(wv.R * wv.NWC - 2 * kmax, n1);
-        const long long tiles = (long long)((wd + 29) / 30) * ((n1 + th - 1) / th);
-        if (th > 0 && 2 * tiles >= 3LL * sm_count(h->device)) ws = av + 1;
-      }
+      if (reg && ws == 0 && st->tile_h == 0) ws = auto_ws_variant(h, wd, n1, kmax, tma_ok) + 1;
       if (ws >= 1 && kWsVariants[std::min(ws - 1, kNumWsVariants - 1)].tma && !tma_ok) {
         set_error("Life: the TMA kernel variants need rows of at least 1024 cells and a "
                   "tensor map of the grid");
@@ -1425,28 +1893,9 @@ static om_status life_proceed(Handle *h, int n) {
         if (reg && ws >= 1) {
           // warp-specialised persistent kernel, variant ws - 1
           const int v = std::min(ws - 1, kNumWsVariants - 1);
-          const WsVariant wv = kWsVariants[v];
-          TbParams q = p;
-          q.tw = std::min(30, wd);
-          q.th = std::min(wv.R * wv.NWC - 2 * kk, n1);
-          q.nt0 = (wd + q.tw - 1) / q.tw;
-          q.nt1 = (n1 + q.th - 1) / q.th;
-          cudaEvent_t ev = prof_begin(h);
-          const int mi = wv.tma ? life_tmap(st, a.d(), n0, n1) : -1;
-          const int ctas = h->cfg.grid_limit > 0
-                               ? std::min(h->cfg.grid_limit, sm_count(h->device))
-                               : sm_count(h->device);
-          cudaError_t e = launch_ws(v, (const int32_t *)a.d(), (int32_t *)a.d_next(), q,
-                                    st->d_pop + g, ctas, st->tmap[mi < 0 ? 0 : mi],
-                                    st->tpatch[mi < 0 ? 0 : mi],
-                                    &((LifeScalars *)h->d_scalars)->wait_error, h->stream);
-          if (e != cudaSuccess) {
-            set_error(std::string("life_ws_kernel: ") + cudaGetErrorString(e));
-            return OM_ERR_CUDA;
-          }
-          prof_end(h, ev, wv.tma ? "life_ws_tma_kernel" : "life_ws_kernel",
-                   (double)n0 * n1 * kk);
-          h->launches++;
+          OM_TRY(launch_ws_tiles(h, v, kCellsToCells, a.d(), a.d_next(), p,
+                                 kWsVariants[v].tma ? life_tmap(st, a.d(), n0, n1) : -1,
+                                 st->d_pop + g));
           a.swap();
           g += kk;
           continue;
@@ -1518,8 +1967,7 @@ static void life_restore_key(Handle *h, uint64_t key) { life_state(h)->binary = 
 static void life_array_written(Handle *h, Array *a) {
   LifeState *st = life_state(h);
   st->binary = false;
-  const bool packed_ok = h->cyclic && (h->size[0] % 32 == 0) && h->cfg.variant == 0;
-  if (!packed_ok || !st->d_flag || h->capturing) return;
+  if (!life_packed_ok(h) || !st->d_flag || h->capturing) return;
   uint32_t bad = 1;
   if (cudaMemsetAsync(st->d_flag, 0, sizeof(uint32_t), h->stream) != cudaSuccess ||
       life_check_cells_into((const int32_t *)a->d(), a->count, st->d_flag, h->stream) !=
@@ -1536,6 +1984,8 @@ static void life_free(Handle *h) {
   if (st) {
     if (st->d_pop) cudaFree(st->d_pop);
     if (st->d_flag) cudaFree(st->d_flag);
+    cudaFree(st->packed[0]);
+    cudaFree(st->packed[1]);
     delete st;
   }
   h->impl = nullptr;
@@ -1584,7 +2034,7 @@ cudaError_t life_check_cells_into(const int32_t *cells, size_t n, uint32_t *flag
 cudaError_t life_tb_launch_into(const int32_t *cur, int32_t *next, int n0, int n1, int gens,
                                 uint32_t *pop, cudaStream_t s) {
   TbParams p;
-  p.n0 = n0; p.n1 = n1; p.wd = n0 / 32;
+  p.n0 = n0; p.n1 = n1; p.wd = n0 / 32; p.nb = 32;
   p.kk = gens;
   p.tw = std::min(32, p.wd);
   p.th = std::min(64, n1);

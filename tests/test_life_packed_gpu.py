@@ -1,0 +1,53 @@
+"""Life runs through the packed grid (rows of any length from 33 cells, and
+long runs of any grid beyond one CTA) against the oracle: rows that end 1, 31
+or 8 cells into a word, tiles that wrap in both axes, grids narrower or lower
+than a tile, and run lengths around the launches they are split into."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def check(pg, oracle, size, gens, seed=3, parts=1):
+    init = oracle.life_bernoulli(size[0], size[1], seed, 0.35)
+    life = pg.Life(size)
+    life.write("cell", init)
+    rc, rp = oracle.life_run(init, gens * parts, cyclic=True)
+    for k in range(parts):
+        life.proceed(gens)
+        assert np.array_equal(life.population_history(gens), rp[k * gens:(k + 1) * gens])
+    assert np.array_equal(life.read("cell"), rc)
+    assert life.population == rp[-1] and life.generation == gens * parts
+    life.close()
+
+
+@pytest.mark.parametrize("gens", [2, 33, 70])
+@pytest.mark.parametrize("size", [(33, 64), (63, 5), (65, 9), (95, 300), (1000, 70), (1023, 77),
+                                  (961, 1), (1921, 513), (4001, 37), (40, 3000)])
+def test_ragged_rows(om_lib, oracle, size, gens):
+    check(om_lib, oracle, size, gens)
+
+
+@pytest.mark.parametrize("size,gens", [((1024, 160), 33), ((2048, 2048), 100), ((992, 3001), 65),
+                                       ((32, 5000), 131), ((8192, 17), 40), ((3040, 4096), 57),
+                                       ((10240, 3000), 34), ((12032, 4000), 90)])
+def test_long_runs(om_lib, oracle, size, gens):
+    # packed register blocks, and the warp-specialised ends on the large grids
+    check(om_lib, oracle, size, gens)
+
+
+def test_graph_replay_and_parity(om_lib, oracle):
+    check(om_lib, oracle, (200, 130), 35, parts=3)
+    check(om_lib, oracle, (1536, 200), 35, parts=3)
+
+
+def test_ragged_nonbinary_first_step(om_lib, oracle):
+    init = oracle.life_bernoulli(250, 96, 2, 0.3)
+    init[10, 10], init[20, 249], init[50, 0] = 3, -1, 7
+    life = om_lib.Life((250, 96))
+    life.write("cell", init)
+    life.proceed(30)
+    rc, rp = oracle.life_run(init, 30, cyclic=True)
+    assert np.array_equal(life.read("cell"), rc)
+    assert np.array_equal(life.population_history(30), rp)
+    life.close()

@@ -12,8 +12,8 @@
 // The device paths give bit-identical results:
 //  * life_general_kernel: one int32 cell per thread with the reference's
 //    integer arithmetic; any size, cyclic or open boundary, any cell values.
-//  * life_smallreg_kernel, life_smallgrid_kernel: whole grid bit-packed in one
-//    CTA, all generations of a run in one launch.  Cyclic, width % 32 == 0.
+//  * life_smallreg_kernel: a small grid bit-packed in the registers of one CTA,
+//    all generations of a run in one launch.  Cyclic, any width up to 1024.
 //  * life_reg_kernel, life_ws_kernel, life_tb*_kernel: bit-packed tiles with a
 //    1-word / k-row halo, k generations per launch (temporal blocking).
 //  * long runs and rows that are no whole number of words keep the grid packed
@@ -347,50 +347,6 @@ __device__ __forceinline__ void pack_rows32_async(const int32_t *__restrict__ cu
   }
 }
 
-// Whole grid in shared memory: all `gens` generations in one launch.
-__global__ void __launch_bounds__(512)
-life_smallgrid_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next,
-                      int n0, int n1, int gens, uint32_t *__restrict__ pop) {
-  extern __shared__ uint32_t sm[];
-  __shared__ uint32_t spop[3];
-  const int wd = n0 >> 5;
-  const int nw = wd * n1;
-  uint32_t *A = sm, *B = sm + nw;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nthreads = blockDim.x, nwarps = nthreads >> 5;
-  pack_rows(cur, n0, n1, wd, 0, 0, wd, n1, A, warp, nwarps, lane);
-  if (tid < 3) spop[tid] = 0;
-  __syncthreads();
-  for (int g = 0; g < gens; ++g) {
-    uint32_t cnt = 0;
-    for (int i = tid; i < nw; i += nthreads) {
-      const int y = i / wd, x = i - y * wd;
-      const int ym = (y == 0 ? n1 - 1 : y - 1) * wd, y0 = y * wd,
-                yp = (y == n1 - 1 ? 0 : y + 1) * wd;
-      const int xm = x == 0 ? wd - 1 : x - 1, xp = x == wd - 1 ? 0 : x + 1;
-      const uint32_t r = life_word(A[ym + xm], A[ym + x], A[ym + xp],
-                                   A[y0 + xm], A[y0 + x], A[y0 + xp],
-                                   A[yp + xm], A[yp + x], A[yp + xp]);
-      B[i] = r;
-      cnt += __popc(r);
-    }
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    if (lane == 0 && cnt) atomicAdd(&spop[g % 3], cnt);
-    __syncthreads();
-    if (tid == 0) {
-      pop[g] = spop[g % 3];
-      spop[(g + 2) % 3] = 0;
-    }
-    uint32_t *t = A; A = B; B = t;
-  }
-  // unpack: lane i of the warp writes bit i of the word
-  for (int i = warp; i < nw; i += nwarps) {
-    const int y = i / wd, x = i - y * wd;
-    const uint32_t w = A[i];
-    next[(size_t)y * n0 + (size_t)x * 32 + lane] = (int32_t)((w >> lane) & 1u);
-  }
-}
-
 struct TbParams {
   int n0, n1, wd;   // grid in cells, width in words
   int tw, th, kk;   // tile width (words), height (rows), generations
@@ -559,79 +515,162 @@ __device__ __forceinline__ uint32_t life_from_sums(const RowSums &a, const RowSu
   return lop3<0xE0>(hit, u0, b.raw);
 }
 
-// Whole grid in registers, one packed word per thread: all `gens`
-// generations in one launch of one CTA.  The grid is wd = n0 / 32 words
-// wide with wd dividing 32, so a warp holds 32 / wd whole rows: lane L has
-// word L % wd of row L / wd of its warp.  West and east words come from
-// the lanes beside (wrapping within the row), the row sums of the rows
-// above and below from lanes L -+ wd; the warp's top and bottom rows take
-// them from the neighbouring warps through shared memory (double-buffered
-// by generation parity, so one barrier per generation).  Each warp adds its
-// population into pop[g] (zeroed by the caller).
-__global__ void __launch_bounds__(1024)
-life_smallreg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, int n0, int n1,
-                     int gens, uint32_t *__restrict__ pop) {
-  __shared__ uint32_t top[2][32][2][32];  // [parity][warp][f1, f2][word]: first row's sums
-  __shared__ uint32_t bot[2][32][2][32];  // last row's sums
-  const int wd = n0 >> 5, rw = 32 / wd;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int x = lane % wd, r = lane / wd, y = warp * rw + r;
-  // pack this thread's word: cells 32x .. 32x + 31 of row y
-  const int32_t *src = cur + (size_t)y * n0 + 32 * x;
-  uint32_t w = 0;
+// A small grid in the registers of one CTA: all generations of a run in one
+// launch, any row length (wd = ceil(n0 / 32) <= 32 words, the last of nb
+// cells).
+struct SmallParams {
+  int n0, n1, wd, nb;
+  int gens;  // 1 .. kSmallMaxGens
+  int nw;    // warps that advance rows; the block's others only move cells
+  int h;     // halo rows each side, and generations between exchanges
+};
+static const int kSmallThreads = 512;
+static const int kSmallMaxGens = 4096;  // populations kept in shared memory
+
+// A warp has rg = 32 / wd groups of lanes, each lane one word of R rows: R rg
+// rows of the whole width, of which the middle ones are the warp's own share of
+// the grid and h above and below are copies.  A generation needs no other warp:
+// west and east words and the row sums above and below a lane's rows come from
+// the lanes beside.  Every h generations, when the copies are stale up to the
+// own rows, the warps trade own rows for copies through shared memory.
+// RAG: nb < 32.  The last word's bits above nb stay 0; the word west of the
+// first is the last one with cell n0 - 1 in its top bit, and the last word's
+// east neighbour is cell 0 at bit nb - 1.
+template <int R, bool RAG>
+__global__ void __launch_bounds__(kSmallThreads)
+life_smallreg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, SmallParams p,
+                     uint32_t *__restrict__ pop) {
+  extern __shared__ uint32_t S[];  // 2 x words, then the populations
+  const int wd = p.wd, n1 = p.n1, nwords = wd * n1;
+  uint32_t *spop = S + 2 * nwords;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NWB = kSmallThreads / 32;
+  for (int i = tid; i < p.gens; i += kSmallThreads) spop[i] = 0;
+  // pack the cells, eight words of the grid in flight per warp
+  for (int i0 = warp * 8; i0 < nwords; i0 += NWB * 8) {
+    int32_t v[8];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int4 v = __ldg(reinterpret_cast<const int4 *>(src) + q);
-    w |= ((uint32_t)v.x | ((uint32_t)v.y << 1) | ((uint32_t)v.z << 2) | ((uint32_t)v.w << 3))
-         << (4 * q);
-  }
-  const int west = x == 0 ? lane + wd - 1 : lane - 1;
-  const int east = x == wd - 1 ? lane - wd + 1 : lane + 1;
-  const int up = (lane - wd) & 31, down = (lane + wd) & 31;
-  const bool first = r == 0, last = r == rw - 1;
-  const int wup = warp == 0 ? nw - 1 : warp - 1, wdown = warp == nw - 1 ? 0 : warp + 1;
-  for (int g = 0; g < gens; ++g) {
-    const int b = g & 1;
-    const uint32_t wl = __shfl_sync(0xffffffffu, w, west), wr = __shfl_sync(0xffffffffu, w, east);
-    const uint32_t W = __funnelshift_l(wl, w, 1), E = __funnelshift_r(w, wr, 1);
-    const RowSums me{w, xor3(W, w, E), maj3(W, w, E)};
-    if (first) {
-      top[b][warp][0][x] = me.f1;
-      top[b][warp][1][x] = me.f2;
+    for (int j = 0; j < 8; ++j) {
+      const int i = min(i0 + j, nwords - 1), y = i / wd, x = (i - y * wd) * 32 + lane;
+      v[j] = x < p.n0 ? __ldg(cur + (size_t)y * p.n0 + x) : 0;
     }
-    if (last) {
-      bot[b][warp][0][x] = me.f1;
-      bot[b][warp][1][x] = me.f2;
-    }
-    RowSums a, c;
-    a.f1 = __shfl_sync(0xffffffffu, me.f1, up);
-    a.f2 = __shfl_sync(0xffffffffu, me.f2, up);
-    c.f1 = __shfl_sync(0xffffffffu, me.f1, down);
-    c.f2 = __shfl_sync(0xffffffffu, me.f2, down);
-    __syncthreads();
-    if (first) {
-      a.f1 = bot[b][wup][0][x];
-      a.f2 = bot[b][wup][1][x];
-    }
-    if (last) {
-      c.f1 = top[b][wdown][0][x];
-      c.f2 = top[b][wdown][1][x];
-    }
-    // the neighbours only (h1, h2: W + E): one operation more than
-    // life_from_sums but a shorter chain, which is what bounds this kernel
-    const uint32_t h1 = W ^ E, h2 = W & E;
-    const uint32_t s0 = xor3(a.f1, h1, c.f1), k0 = maj3(a.f1, h1, c.f1);
-    const uint32_t u1 = xor3(a.f2, h2, c.f2), u2 = maj3(a.f2, h2, c.f2);
-    w = ~u2 & (u1 ^ k0) & (s0 | w);
-    const uint32_t cnt = __reduce_add_sync(0xffffffffu, __popc(w));
-    if (lane == 0 && cnt) atomicAdd(&pop[g], cnt);
-  }
-  int32_t *dst = next + (size_t)y * n0 + 32 * x;
+    uint32_t mine = 0;
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
-    reinterpret_cast<int4 *>(dst)[q] =
-        make_int4((int)((w >> (4 * q)) & 1u), (int)((w >> (4 * q + 1)) & 1u),
-                  (int)((w >> (4 * q + 2)) & 1u), (int)((w >> (4 * q + 3)) & 1u));
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t w = __ballot_sync(0xffffffffu, v[j] != 0);
+      if (lane == j) mine = w;
+    }
+    if (lane < 8 && i0 + lane < nwords) S[i0 + lane] = mine;
+  }
+  __syncthreads();
+  if (warp < p.nw) {
+    const int rg = 32 / wd, x = lane % wd, r = lane / wd, h = p.h;
+    // this warp's own rows: local rows h .. h + own, row j of the block of
+    // copies is row (start - h + j) mod n1 of the grid
+    const int start = (int)((long long)warp * n1 / p.nw);
+    const int own = (int)((long long)(warp + 1) * n1 / p.nw) - start;
+    const int j0 = r * R;
+    const int g0 = ((start - h + j0) % n1 + n1) % n1;
+    const bool used = r < rg;
+    uint32_t rows[R], ownrow = 0;  // own rows of this lane
+    {
+      int gy = g0;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        rows[i] = S[gy * wd + x];
+        if (used && j0 + i >= h && j0 + i < h + own) ownrow |= 1u << i;
+        gy = gy + 1 == n1 ? 0 : gy + 1;
+      }
+    }
+    const int west = used && x == 0 ? lane + wd - 1 : (lane == 0 ? 0 : lane - 1);
+    const int east = used && x == wd - 1 ? lane - wd + 1 : (lane == 31 ? 31 : lane + 1);
+    const int up = (lane - wd) & 31, down = (lane + wd) & 31;
+    const bool lastw = x == wd - 1;
+    const int lsh = RAG && x == 0 ? 32 - p.nb : 0;       // of the west word
+    const int esh = RAG && lastw ? p.nb - 1 : 31;        // of the east word
+    const uint32_t keep = RAG && lastw ? (1u << p.nb) - 1u : ~0u;
+    auto sums = [&](uint32_t w, uint32_t &f1, uint32_t &f2) {
+      const uint32_t wl = __shfl_sync(0xffffffffu, w, west);
+      const uint32_t wr = __shfl_sync(0xffffffffu, w, east);
+      const uint32_t W = __funnelshift_l(RAG ? wl << lsh : wl, w, 1);
+      const uint32_t E = RAG ? (w >> 1) | (wr << esh) : __funnelshift_r(w, wr, 1);
+      f1 = xor3(W, w, E);
+      f2 = maj3(W, w, E);
+    };
+    uint32_t *buf = S + nwords;  // the buffer of the next exchange
+    // counts of an even generation and the next, and those of the pair before,
+    // summed over the warp while the next generation is under way
+    uint32_t pair = 0, done = 0;
+    int left = h;                // generations until the copies are stale
+    for (int g = 0; g < p.gens; ++g) {
+      const uint32_t sum = g & 1 ? 0u : __reduce_add_sync(0xffffffffu, done);
+      // sums of rows -1 (the lane above's last) .. R (the lane below's first)
+      uint32_t f1[R + 2], f2[R + 2];
+#pragma unroll
+      for (int i = 0; i < R; ++i) sums(rows[i], f1[i + 1], f2[i + 1]);
+      f1[0] = __shfl_sync(0xffffffffu, f1[R], up);
+      f2[0] = __shfl_sync(0xffffffffu, f2[R], up);
+      f1[R + 1] = __shfl_sync(0xffffffffu, f1[1], down);
+      f2[R + 1] = __shfl_sync(0xffffffffu, f2[1], down);
+      uint32_t cnt = 0;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        uint32_t w = life_from_sums(RowSums{0u, f1[i], f2[i]},
+                                    RowSums{rows[i], f1[i + 1], f2[i + 1]},
+                                    RowSums{0u, f1[i + 2], f2[i + 2]});
+        if (RAG) w &= keep;
+        rows[i] = w;
+        cnt += ownrow & (1u << i) ? __popc(w) : 0;
+      }
+      // a warp's count is at most 32 x 32 R < 2^16: two generations a sum
+      if (g & 1) {
+        done = pair | cnt << 16;
+      } else {
+        pair = cnt;
+        if (g > 0 && lane < 2) atomicAdd(&spop[g - 2 + lane], (sum >> (16 * lane)) & 0xffffu);
+      }
+      if (--left == 0 && g != p.gens - 1) {
+        left = h;
+        int gy = g0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          if (ownrow & (1u << i)) buf[gy * wd + x] = rows[i];
+          gy = gy + 1 == n1 ? 0 : gy + 1;
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(p.nw * 32) : "memory");
+        gy = g0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          if (!(ownrow & (1u << i))) rows[i] = buf[gy * wd + x];
+          gy = gy + 1 == n1 ? 0 : gy + 1;
+        }
+        // the other buffer may be written at the next exchange: its last
+        // readers passed this one's barrier
+        buf = buf == S ? S + nwords : S;
+      }
+    }
+    {  // the last one or two generations
+      const bool odd = p.gens & 1;
+      const uint32_t sum = __reduce_add_sync(0xffffffffu, odd ? pair : done);
+      if (lane < (odd ? 1 : 2))
+        atomicAdd(&spop[p.gens - (odd ? 1 : 2) + lane], (sum >> (16 * lane)) & 0xffffu);
+    }
+    // into the buffer that no warp still reads
+    int gy = g0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (ownrow & (1u << i)) buf[gy * wd + x] = rows[i];
+      gy = gy + 1 == n1 ? 0 : gy + 1;
+    }
+    if (tid == 0) spop[p.gens] = (uint32_t)(buf - S);
+  }
+  __syncthreads();
+  const uint32_t *out = S + spop[p.gens];
+  for (int i = tid; i < p.gens; i += kSmallThreads) pop[i] += spop[i];
+  for (int i = warp; i < nwords; i += NWB) {
+    const int y = i / wd, x = (i - y * wd) * 32 + lane;
+    if (x < p.n0) next[(size_t)y * p.n0 + x] = (int32_t)((out[i] >> lane) & 1u);
+  }
 }
 
 // Temporal blocking with one lane per packed word: a tile is 32 words wide
@@ -1275,28 +1314,80 @@ __global__ void life_finalize_kernel(LifeScalars *s, const uint32_t *pop, int n)
 // host side
 // ---------------------------------------------------------------------------
 
-// Grids up to this many packed words run all generations in one CTA; larger
-// ones spread over every SM with the temporally blocked tiles.
-static const int kSmallMaxWords = 4096;
+// The small kernel's variants (rows per lane).
+static const int kSmallRows[] = {2, 3, 4, 5, 6, 8};
+static const int kNumSmallRows = 6;
+
+typedef void (*SmallKernel)(const int32_t *, int32_t *, SmallParams, uint32_t *);
+template <bool RAG> static SmallKernel small_kernel(int v) {
+  switch (v) {
+    case 0: return life_smallreg_kernel<2, RAG>;
+    case 1: return life_smallreg_kernel<3, RAG>;
+    case 2: return life_smallreg_kernel<4, RAG>;
+    case 3: return life_smallreg_kernel<5, RAG>;
+    case 4: return life_smallreg_kernel<6, RAG>;
+    default: return life_smallreg_kernel<8, RAG>;
+  }
+}
+
+// The small kernel's plan for a grid: variant, warps and halo of least modelled
+// cycles per generation (nw 0: no plan fits).  The model follows 128^2 on
+// GB300, where 2 rows x 12 warps take 362 cycles a generation, 2 x 16 390,
+// 3 x 8 402, 5 x 4 405, 4 x 8 490, 8 x 4 580 and 3 x 16 560 (one word a thread
+// in 16 warps with an exchange every generation: 440).
+struct SmallPlan {
+  int v, nw, h;
+  double cycles;
+};
+static SmallPlan small_plan(int n0, int n1) {
+  SmallPlan best{0, 0, 0, 0};
+  const int wd = (n0 + 31) / 32;
+  if (wd > 32 || n1 > 2048) return best;
+  for (int v = 0; v < kNumSmallRows; ++v) {
+    const int R = kSmallRows[v], rows = (32 / wd) * R;
+    for (int nw = 1; nw <= kSmallThreads / 32 && nw <= n1; ++nw) {
+      const int own = (n1 + nw - 1) / nw, h = (rows - own) / 2;
+      if (h < 1) continue;
+      const double c = (40.0 + 38.0 * R * ((nw + 3) / 4) + 30.0 * R + 60.0 / h) *
+                       (n0 % 32 ? 1.2 : 1.0);
+      if (best.nw == 0 || c < best.cycles) best = SmallPlan{v, nw, h, c};
+    }
+  }
+  return best;
+}
+// Whether a grid runs in one CTA: the small kernel's cycles per generation
+// against the packed tiles' (about 1000 at least, with launches, packing and
+// unpacking around them).
+static bool life_small(const Handle *h) {
+  const SmallPlan pl = small_plan(h->size[0], h->size[1]);
+  return pl.nw > 0 && pl.cycles < 1000.0;
+}
 
 // whether packed kernels serve the grid: every cell 0 or 1, cyclic, rows of
 // whole words or of at least one word and a cell
 static bool life_packed_ok(const Handle *h) {
-  return h->cyclic && h->cfg.variant == 0 && (h->size[0] % 32 == 0 || h->size[0] > 32);
+  return h->cyclic && h->cfg.variant == 0 &&
+         (h->size[0] % 32 == 0 || h->size[0] > 32 || life_small(h));
+}
+
+// Launch knobs (om_config depth, tile_x, tile_y, life_kernel) apply to grids of
+// more than this many packed words; smaller ones run on whatever fits them.
+static const long long kKnobWords = 4096;
+static bool life_knobs(const Handle *h) {
+  const om_config &c = h->cfg;
+  return (long long)((h->size[0] + 31) / 32) * h->size[1] > kKnobWords &&
+         (c.depth != 0 || c.tile_x != 0 || c.tile_y != 0 || c.life_kernel != 0 || c.life_io != 0 ||
+          c.grid_limit != 0);
 }
 
 // Whether a run of n generations goes through the packed grid: rows that are
 // no whole number of words from two generations on (a single one is cheaper
 // one cell per thread than packed, advanced and unpacked), others with no
-// launch knob set, beyond the one-CTA grids, when one launch of at most 32
-// generations cannot do.
+// launch knob set, when one launch of at most 32 generations cannot do.
 static bool life_run_packed(const Handle *h, int n) {
-  if (!life_packed_ok(h)) return false;
+  if (!life_packed_ok(h) || life_small(h)) return false;
   if (h->size[0] % 32 != 0) return n >= 2;
-  const om_config &c = h->cfg;
-  return n > 32 && (long long)(h->size[0] / 32) * h->size[1] > kSmallMaxWords && c.depth == 0 &&
-         c.tile_x == 0 && c.tile_y == 0 && c.life_kernel == 0 && c.life_io == 0 &&
-         c.grid_limit == 0;
+  return n > 32 && !life_knobs(h);
 }
 
 static om_status life_reserve(Handle *h, int kernel_id, int n) {
@@ -1650,10 +1741,10 @@ static int reg_variant(int kk, int want_th) {
 // Tile choice: tile_w 0 (default) selects the register-resident kernel,
 // 30 the one-lane-per-word shared-memory kernel, other widths the general
 // tile kernel.  Depth defaults to 32 generations per launch.
-static bool life_pick_tiles(Handle *h, TbParams &p) {
+static bool life_pick_tiles(Handle *h, TbParams &p, bool knobs) {
   LifeState *st = life_state(h);
-  const bool lane_per_word = st->tile_w == 0 || st->tile_w == 30;
-  p.kk = st->depth > 0 ? std::min(st->depth, 32) : 32;
+  const bool lane_per_word = !knobs || st->tile_w == 0 || st->tile_w == 30;
+  p.kk = knobs && st->depth > 0 ? std::min(st->depth, 32) : 32;
   p.tw = lane_per_word ? 30 : st->tile_w;
   p.th = st->tile_h > 0 ? st->tile_h : 128;
   p.tw = std::min(p.tw, p.wd);
@@ -1820,43 +1911,44 @@ static om_status life_proceed(Handle *h, int n) {
   OM_CUDA_CHECK(cudaMemsetAsync(st->d_pop, 0, (size_t)n * sizeof(uint32_t), h->stream));
   const int n0 = h->size[0], n1 = h->size[1];
   const bool ragged = n0 % 32 != 0;
-  const bool packed_ok = life_packed_ok(h) && (!ragged || n >= 2);
+  const bool small = life_small(h);
+  // on rows that are no whole number of words, a few generations are cheaper
+  // one cell per thread than packed, advanced and unpacked
+  const bool packed_ok = life_packed_ok(h) && (!ragged || n >= (small ? 4 : 2));
   int g = 0;
   if (!packed_ok || !st->binary) {
     const int first = packed_ok ? 1 : n;
     for (; g < first; ++g) OM_TRY(launch_general(h, st->d_pop + g));
     st->binary = true;
   }
-  if (g < n && (ragged || life_run_packed(h, n - g))) {
+  if (g < n && packed_ok && small) {
+    const SmallPlan pl = small_plan(n0, n1);
+    SmallParams sp{n0, n1, (n0 + 31) / 32, 0, 0, pl.nw, pl.h};
+    sp.nb = n0 - 32 * (sp.wd - 1);
+    const SmallKernel k = ragged ? small_kernel<true>(pl.v) : small_kernel<false>(pl.v);
+    for (; g < n; g += sp.gens) {
+      sp.gens = std::min(n - g, kSmallMaxGens);
+      const size_t smem = sizeof(uint32_t) * (2 * (size_t)sp.wd * n1 + sp.gens + 1);
+      OM_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      cudaEvent_t ev = prof_begin(h);
+      k<<<1, kSmallThreads, smem, h->stream>>>((const int32_t *)a.d(), (int32_t *)a.d_next(), sp,
+                                               st->d_pop + g);
+      OM_CUDA_CHECK(cudaGetLastError());
+      prof_end(h, ev, "life_smallreg_kernel", (double)n0 * n1 * sp.gens);
+      h->launches++;
+      a.swap();
+    }
+  } else if (g < n && (ragged || life_run_packed(h, n - g))) {
     OM_TRY(proceed_packed(h, n, g));
   } else if (g < n) {
     const int wd = n0 / 32;
-    if (32 % wd == 0 && (n1 * wd) % 32 == 0 && n1 * wd <= 1024 && n1 * wd >= 32) {
-      // one packed word per thread of one CTA, in registers
-      cudaEvent_t ev = prof_begin(h);
-      life_smallreg_kernel<<<1, n1 * wd, 0, h->stream>>>(
-          (const int32_t *)a.d(), (int32_t *)a.d_next(), n0, n1, n - g, st->d_pop + g);
-      OM_CUDA_CHECK(cudaGetLastError());
-      prof_end(h, ev, "life_smallreg_kernel", (double)n0 * n1 * (n - g));
-      h->launches++;
-      a.swap();
-    } else if ((size_t)wd * n1 <= (size_t)kSmallMaxWords) {
-      const size_t smem = 2 * sizeof(uint32_t) * (size_t)wd * n1;
-      OM_CUDA_CHECK(cudaFuncSetAttribute(life_smallgrid_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-      cudaEvent_t ev = prof_begin(h);
-      life_smallgrid_kernel<<<1, 512, smem, h->stream>>>(
-          (const int32_t *)a.d(), (int32_t *)a.d_next(), n0, n1, n - g, st->d_pop + g);
-      OM_CUDA_CHECK(cudaGetLastError());
-      prof_end(h, ev, "life_smallgrid_kernel", (double)n0 * n1 * (n - g));
-      h->launches++;
-      a.swap();
-    } else {
+    {
       TbParams p;
       p.n0 = n0; p.n1 = n1; p.wd = wd; p.nb = 32;
-      const bool l32 = life_pick_tiles(h, p);
-      const bool reg = st->tile_w == 0;
+      const bool knobs = life_knobs(h);
+      const bool l32 = life_pick_tiles(h, p, knobs);
+      const bool reg = !knobs || st->tile_w == 0;
+      const int tile_h = knobs ? st->tile_h : 0;
       const int kmax = p.kk;
       p.nt0 = (p.wd + p.tw - 1) / p.tw;
       p.nt1 = (p.n1 + p.th - 1) / p.th;
@@ -1876,12 +1968,12 @@ static om_status life_proceed(Handle *h, int n) {
       // given takes it too on grids of at least 1.5 of its tiles per SM,
       // where it overlaps one tile's loads and stores with another's
       // generations, and the register-resident blocks on smaller grids
-      int ws = h->cfg.life_kernel;
+      int ws = knobs ? h->cfg.life_kernel : 0;
       // TMA rows need a grid at least one box (32 words) wide whose buffers
       // the driver describes
       const bool tma_ok = wd >= 32 && life_tmap(st, a.d(), n0, n1) >= 0 &&
                           life_tmap(st, a.d_next(), n0, n1) >= 0;
-      if (reg && ws == 0 && st->tile_h == 0) ws = auto_ws_variant(h, wd, n1, kmax, tma_ok) + 1;
+      if (reg && ws == 0 && tile_h == 0) ws = auto_ws_variant(h, wd, n1, kmax, tma_ok) + 1;
       if (ws >= 1 && kWsVariants[std::min(ws - 1, kNumWsVariants - 1)].tma && !tma_ok) {
         set_error("Life: the TMA kernel variants need rows of at least 1024 cells and a "
                   "tensor map of the grid");
@@ -1902,9 +1994,9 @@ static om_status life_proceed(Handle *h, int n) {
         }
         if (reg) {
           TbParams q = p;
-          const int v = st->tile_h > 0 ? reg_variant(kk, st->tile_h)
+          const int v = tile_h > 0 ? reg_variant(kk, tile_h)
                                        : reg_plan(h->device, vec, wd, n1, kk, &q.nt0, &q.nt1);
-          if (st->tile_h > 0) {
+          if (tile_h > 0) {
             const int thm = std::min(kRegVariants[v].R * kRegVariants[v].NW - 2 * kk, n1);
             q.nt0 = (wd + 29) / 30;
             q.nt1 = (n1 + thm - 1) / thm;

@@ -36,6 +36,34 @@ def test_long_runs(om_lib, oracle, size, gens):
     check(om_lib, oracle, size, gens)
 
 
+@pytest.mark.parametrize("gens", [1, 2, 7, 64, 301])
+@pytest.mark.parametrize("size", [(1, 1), (1, 9), (3, 3), (31, 2), (32, 1), (33, 40), (80, 48),
+                                  (96, 33), (128, 128), (127, 129), (160, 100), (512, 60),
+                                  (1000, 8), (1024, 17), (992, 1)])
+def test_one_cta_grids(om_lib, oracle, size, gens):
+    # rows of 1 to 32 words, lane groups that do not fill the warp, fewer rows
+    # than the halo
+    check(om_lib, oracle, size, gens)
+
+
+def test_one_cta_long_run(om_lib, oracle):
+    check(om_lib, oracle, (70, 20), 4097)   # more generations than one launch counts
+
+
+@pytest.mark.parametrize("cfg", [{"life_kernel": 5}, {"depth": 3, "tile_x": 4, "tile_y": 8},
+                                 {"life_io": 1}])
+def test_knobs_do_not_apply_to_small_grids(om_lib, oracle, cfg):
+    init = oracle.life_bernoulli(512, 256, 7, 0.3)
+    for gens in (20, 50):
+        life = om_lib.Life((512, 256), **cfg)
+        life.write("cell", init)
+        life.proceed(gens)
+        rc, rp = oracle.life_run(init, gens, cyclic=True)
+        assert np.array_equal(life.read("cell"), rc)
+        assert np.array_equal(life.population_history(gens), rp)
+        life.close()
+
+
 def test_graph_replay_and_parity(om_lib, oracle):
     check(om_lib, oracle, (200, 130), 35, parts=3)
     check(om_lib, oracle, (1536, 200), 35, parts=3)

@@ -198,7 +198,7 @@ __device__ __forceinline__ hs::Flux<R> wall_flux(R g, const hf::Consts<R> &k,
                                                  const hs::Prim<R> &L, R cl,
                                                  const hs::Prim<R> &Rt, R cr) {
   if constexpr (FA) return hf::hllc<AX>(k, L, cl, Rt, cr);
-  else return hs::hllc<AX>(g, L, cl, Rt, cr);
+  else return hs::hllc<AX>(k, L, cl, Rt, cr);
 }
 
 // MUSCL face values in the exact or the production algebra
@@ -222,7 +222,7 @@ __device__ __forceinline__ hs::Prim<R> cell_update(R g, const hf::Consts<R> &k,
                                                    const hs::Flux<R> &l1, const hs::Flux<R> &r1,
                                                    R *cons = nullptr) {
   if constexpr (FA) return hf::update(k, b, dtdx0, dtdx1, l0, r0, l1, r1, cons);
-  else return hs::update(g, b, dtdx0, dtdx1, l0, r0, l1, r1, cons);
+  else return hs::update(k, b, dtdx0, dtdx1, l0, r0, l1, r1, cons);
 }
 
 }  // namespace hk
@@ -614,28 +614,30 @@ template <class R> struct PlainView {
 
 // stage-1 state at (x, y): order-1 walls recomputed from the primitives
 template <class R>
-__device__ __forceinline__ hs::Prim<R> plain_stage1(const PlainView<R> &V, R g, R dtdx0, R dtdx1,
-                                                    int x, int y) {
+__device__ __forceinline__ hs::Prim<R> plain_stage1(const PlainView<R> &V, const hs::Gas<R> &k,
+                                                    R dtdx0, R dtdx1, int x, int y) {
   const hs::Prim<R> c = V.at(x, y), xm = V.at(x - 1, y), xp = V.at(x + 1, y),
                     ym = V.at(x, y - 1), yp = V.at(x, y + 1);
+  const R g = k.g;
   const R cc = hs::sound(g, c.rho, c.p);
-  const hs::Flux<R> l0 = hs::hllc<0>(g, xm, hs::sound(g, xm.rho, xm.p), c, cc);
-  const hs::Flux<R> r0 = hs::hllc<0>(g, c, cc, xp, hs::sound(g, xp.rho, xp.p));
-  const hs::Flux<R> l1 = hs::hllc<1>(g, ym, hs::sound(g, ym.rho, ym.p), c, cc);
-  const hs::Flux<R> r1 = hs::hllc<1>(g, c, cc, yp, hs::sound(g, yp.rho, yp.p));
-  return hs::update(g, c, dtdx0, dtdx1, l0, r0, l1, r1);
+  const hs::Flux<R> l0 = hs::hllc<0>(k, xm, hs::sound(g, xm.rho, xm.p), c, cc);
+  const hs::Flux<R> r0 = hs::hllc<0>(k, c, cc, xp, hs::sound(g, xp.rho, xp.p));
+  const hs::Flux<R> l1 = hs::hllc<1>(k, ym, hs::sound(g, ym.rho, ym.p), c, cc);
+  const hs::Flux<R> r1 = hs::hllc<1>(k, c, cc, yp, hs::sound(g, yp.rho, yp.p));
+  return hs::update(k, c, dtdx0, dtdx1, l0, r0, l1, r1);
 }
 
 template <int AX, class R>
 __device__ __forceinline__ hs::Flux<R> plain_wall2(const hs::Prim<R> &a0, const hs::Prim<R> &a1,
                                                    const hs::Prim<R> &a2, const hs::Prim<R> &a3,
-                                                   R g) {
+                                                   const hs::Gas<R> &k) {
+  const R g = k.g;
   hs::Prim<R> L, Rt;
   hs::muscl(a0.rho, a1.rho, a2.rho, a3.rho, L.rho, Rt.rho);
   hs::muscl(a0.v0, a1.v0, a2.v0, a3.v0, L.v0, Rt.v0);
   hs::muscl(a0.v1, a1.v1, a2.v1, a3.v1, L.v1, Rt.v1);
   hs::muscl(a0.p, a1.p, a2.p, a3.p, L.p, Rt.p);
-  return hs::hllc<AX>(g, L, hs::sound(g, L.rho, L.p), Rt, hs::sound(g, Rt.rho, Rt.p));
+  return hs::hllc<AX>(k, L, hs::sound(g, L.rho, L.p), Rt, hs::sound(g, Rt.rho, Rt.p));
 }
 
 template <class R>
@@ -643,7 +645,7 @@ __global__ void __launch_bounds__(128)
 hydro_plain_step_kernel(PlainView<R> V, R *__restrict__ orho, R *__restrict__ ov0,
                         R *__restrict__ ov1, R *__restrict__ op, double gamma, R dtG, R dR0,
                         R dR1) {
-  const R g = (R)gamma;
+  const hs::Gas<R> g = hs::gas<R>((R)gamma);
   const R dtHalf = dtG / R(2);
   const R h0 = dtHalf / dR0, h1 = dtHalf / dR1;
   const R f0 = dtG / dR0, f1 = dtG / dR1;

@@ -11,11 +11,61 @@
 
 #include <cuda_runtime.h>
 
+#include "exact_f64.cuh"
+
 namespace om {
 namespace hs {
 
-template <class R> __device__ __forceinline__ R omax(R a, R b) { return (a < b) ? b : a; }
-template <class R> __device__ __forceinline__ R omin(R a, R b) { return (b < a) ? b : a; }
+// The operations of the scheme that are not plain additions and
+// multiplications.  In double they run on the integer pipes with the same
+// results (exact_f64.cuh): GB300's double pipe is what bounds an FP64 step.
+template <class R> __device__ __forceinline__ bool less(R a, R b) { return a < b; }
+template <> __device__ __forceinline__ bool less(double a, double b) { return xf::less(a, b); }
+template <class R> __device__ __forceinline__ bool lesseq(R a, R b) { return a <= b; }
+template <> __device__ __forceinline__ bool lesseq(double a, double b) {
+  return xf::lesseq(a, b);
+}
+template <class R> __device__ __forceinline__ R omax(R a, R b) { return less(a, b) ? b : a; }
+template <class R> __device__ __forceinline__ R omin(R a, R b) { return less(b, a) ? b : a; }
+template <class R> __device__ __forceinline__ bool positive(R x) { return R(0) < x; }
+template <> __device__ __forceinline__ bool positive(double x) { return xf::positive(x); }
+template <class R> __device__ __forceinline__ R div(R a, R b) { return a / b; }
+template <> __device__ __forceinline__ double div(double a, double b) { return xf::div(a, b); }
+template <class R> __device__ __forceinline__ R root(R x) { return sqrt(x); }
+template <> __device__ __forceinline__ double root(double x) { return xf::sqrt_rn(x); }
+template <class R> __device__ __forceinline__ R half(R x) { return x / R(2); }
+template <> __device__ __forceinline__ double half(double x) { return xf::half(x); }
+// 0 + x, and x + 0 p
+template <class R> __device__ __forceinline__ R plus_zero(R x) { return R(0) + x; }
+template <> __device__ __forceinline__ double plus_zero(double x) { return xf::plus_zero(x); }
+template <class R> __device__ __forceinline__ R plus_none(R x, R p) { return x + p * R(0); }
+template <> __device__ __forceinline__ double plus_none(double x, double p) {
+  return xf::plus_none(x, p);
+}
+// a divisor used more than once
+template <class R> struct Divisor {
+  R b;
+  __device__ __forceinline__ explicit Divisor(R x) : b(x) {}
+  __device__ __forceinline__ R under(R a) const { return a / b; }
+};
+template <> struct Divisor<double> {
+  xf::Divisor d;
+  __device__ __forceinline__ explicit Divisor(double x) : d(xf::divisor(x)) {}
+  __device__ __forceinline__ double under(double a) const { return xf::div(a, d); }
+};
+
+// gamma and what the scheme forms of it
+template <class R> struct Gas {
+  R g, gm1, gm1inv, qc;  // gamma, gamma-1, 1/(gamma-1), (gamma+1)/(2 gamma)
+};
+template <class R> __device__ __forceinline__ Gas<R> gas(R g) {
+  Gas<R> k;
+  k.g = g;
+  k.gm1 = g - R(1);
+  k.gm1inv = R(1) / k.gm1;
+  k.qc = (g + R(1)) / (R(2) * g);
+  return k;
+}
 
 template <class R> struct Prim { R rho, v0, v1, p; };
 // 16-byte aligned: a record in shared memory moves as one 128-bit access
@@ -24,101 +74,112 @@ template <class R> struct alignas(16) Flux { R fd, fm0, fm1, fe; };
 
 // kineticEnergy x = 0.5 * contract (\i -> velocity x !i * momentum x !i)
 template <class R> __device__ __forceinline__ R kinetic(R v0, R v1, R m0, R m1) {
-  return R(0.5) * ((R(0) + v0 * m0) + v1 * m1);
+  return half(plus_zero(v0 * m0) + v1 * m1);
 }
 
 // energy of a primitive record: Ek + 1/(gamma-1) * p
-template <class R> __device__ __forceinline__ R energy_prim(R g, R rho, R v0, R v1, R p) {
+template <class R>
+__device__ __forceinline__ R energy_prim(const Gas<R> &k, R rho, R v0, R v1, R p) {
   const R m0 = rho * v0, m1 = rho * v1;
-  return kinetic(v0, v1, m0, m1) + (R(1) / (g - R(1))) * p;
+  return kinetic(v0, v1, m0, m1) + k.gm1inv * p;
+}
+
+// m va + p [the axis is AX]
+template <bool ON, class R> __device__ __forceinline__ R mome_flux(R m, R va, R p) {
+  return ON ? m * va + p : plus_none(m * va, p);
 }
 
 // fluxes along axis AX of a primitive record
 template <int AX, class R>
-__device__ __forceinline__ Flux<R> flux_prim(R g, R rho, R v0, R v1, R p) {
+__device__ __forceinline__ Flux<R> flux_prim(const Gas<R> &k, R rho, R v0, R v1, R p) {
   const R m0 = rho * v0, m1 = rho * v1;
-  const R e = kinetic(v0, v1, m0, m1) + (R(1) / (g - R(1))) * p;
+  const R e = kinetic(v0, v1, m0, m1) + k.gm1inv * p;
   const R h = e + p;
   const R va = AX == 0 ? v0 : v1;
   Flux<R> f;
   f.fd = AX == 0 ? m0 : m1;
-  f.fm0 = m0 * va + p * (AX == 0 ? R(1) : R(0));
-  f.fm1 = m1 * va + p * (AX == 1 ? R(1) : R(0));
+  f.fm0 = mome_flux<AX == 0>(m0, va, p);
+  f.fm1 = mome_flux<AX == 1>(m1, va, p);
   f.fe = h * va;
   return f;
 }
 
 // fluxes along AX of a conserved record (velocity m/rho, p = (g-1)(E-Ek))
 template <int AX, class R>
-__device__ __forceinline__ Flux<R> flux_cons(R g, R rho, R m0, R m1, R e) {
-  const R v0 = m0 / rho, v1 = m1 / rho;
-  const R p = (g - R(1)) * (e - kinetic(v0, v1, m0, m1));
+__device__ __forceinline__ Flux<R> flux_cons(const Gas<R> &k, R rho, R m0, R m1, R e) {
+  const Divisor<R> d(rho);
+  const R v0 = d.under(m0), v1 = d.under(m1);
+  const R p = k.gm1 * (e - kinetic(v0, v1, m0, m1));
   const R h = e + p;
   const R va = AX == 0 ? v0 : v1;
   Flux<R> f;
   f.fd = AX == 0 ? m0 : m1;
-  f.fm0 = m0 * va + p * (AX == 0 ? R(1) : R(0));
-  f.fm1 = m1 * va + p * (AX == 1 ? R(1) : R(0));
+  f.fm0 = mome_flux<AX == 0>(m0, va, p);
+  f.fm1 = mome_flux<AX == 1>(m1, va, p);
   f.fe = h * va;
   return f;
 }
 
 // soundSpeed' dens pres = sqrt (kGamma * pres / dens)
 template <class R> __device__ __forceinline__ R sound(R g, R rho, R p) {
-  return sqrt((g * p) / rho);
+  return root(div(g * p, rho));
 }
 
 // hllcQ sp p, condition as written in HydroMain.hs
-template <class R> __device__ __forceinline__ R hllc_q(R g, R sp, R p) {
-  const R t = sqrt(R(1) + (g + R(1)) / (R(2) * g) * (sp / p - R(1)));
-  return (p <= sp) ? R(1) : t;
+template <class R> __device__ __forceinline__ R hllc_q(const Gas<R> &k, R sp, R p) {
+  if (lesseq(p, sp)) return R(1);
+  return root(R(1) + k.qc * (div(sp, p) - R(1)));
 }
 
 template <int AX, class R>
-__device__ __forceinline__ Flux<R> star_flux(R g, R sstar, R shock, R rho, R v0, R v1,
+__device__ __forceinline__ Flux<R> star_flux(const Gas<R> &k, R sstar, R shock, R rho, R v0, R v1,
                                              R p) {
   const R speed = AX == 0 ? v0 : v1;
-  const R dens = rho * (shock - speed) / (shock - sstar);
+  const R ds = shock - speed;
+  const Divisor<R> d(rho);
+  const R dens = div(rho * ds, shock - sstar);
   const R mome0 = dens * (AX == 0 ? sstar : v0);
   const R mome1 = dens * (AX == 1 ? sstar : v1);
-  const R e = energy_prim(g, rho, v0, v1, p);
-  const R enrg = dens * (e / rho + (sstar - speed) * (sstar + p / rho / (shock - speed)));
-  return flux_cons<AX>(g, dens, mome0, mome1, enrg);
+  const R e = energy_prim(k, rho, v0, v1, p);
+  const R enrg = dens * (d.under(e) + (sstar - speed) * (sstar + div(d.under(p), ds)));
+  return flux_cons<AX>(k, dens, mome0, mome1, enrg);
 }
 
 // The wall record's fluxes of hllc i left right (HydroMain.hs:237-268).
 // cl, cr: sound speeds of the two states.
 template <int AX, class R>
-__device__ __forceinline__ Flux<R> hllc(R g, const Prim<R> &L, R cl, const Prim<R> &Rt,
-                                        R cr) {
-  const R densMid = (L.rho + Rt.rho) / R(2);
-  const R soundMid = (cl + cr) / R(2);
+__device__ __forceinline__ Flux<R> hllc(const Gas<R> &k, const Prim<R> &L, R cl,
+                                        const Prim<R> &Rt, R cr) {
+  const R densMid = half(L.rho + Rt.rho);
+  const R soundMid = half(cl + cr);
   const R uL = AX == 0 ? L.v0 : L.v1;
   const R uR = AX == 0 ? Rt.v0 : Rt.v1;
-  const R psraw = (L.p + Rt.p) / R(2) - densMid * soundMid * (uR - uL);
-  const R presStar = omax(R(0), psraw);
-  const R qL = hllc_q(g, presStar, L.p), qR = hllc_q(g, presStar, Rt.p);
+  const R psraw = half(L.p + Rt.p) - densMid * soundMid * (uR - uL);
+  const R presStar = positive(psraw) ? psraw : R(0);
+  const R qL = hllc_q(k, presStar, L.p), qR = hllc_q(k, presStar, Rt.p);
   const R shockLeft = uL - cl * qL;
   const R shockRight = uR + cr * qR;
-  const R shockStar = (Rt.p - L.p + L.rho * uL * (shockLeft - uL) -
-                       Rt.rho * uR * (shockRight - uR)) /
-                      (L.rho * (shockLeft - uL) - Rt.rho * (shockRight - uR));
+  const R dL = shockLeft - uL, dR = shockRight - uR;
+  const R shockStar = div(Rt.p - L.p + L.rho * uL * dL - Rt.rho * uR * dR,
+                          L.rho * dL - Rt.rho * dR);
   // select (0 < SL) L (select (0 < S*) L* (select (0 < SR) R* R)): pick the
   // side first, then evaluate one physical or star flux on it, so a warp
   // whose faces take different cases does not run both star states
-  const bool posL = R(0) < shockLeft, posS = R(0) < shockStar, posR = R(0) < shockRight;
+  const bool posL = positive(shockLeft), posS = positive(shockStar), posR = positive(shockRight);
   const bool useL = posL || posS;
   const bool star = useL ? !posL : posR;
   const R xr = useL ? L.rho : Rt.rho, x0 = useL ? L.v0 : Rt.v0, x1 = useL ? L.v1 : Rt.v1,
           xp = useL ? L.p : Rt.p;
   const R shock = useL ? shockLeft : shockRight;
-  const Flux<R> fs = star_flux<AX>(g, shockStar, shock, xr, x0, x1, xp);
-  const Flux<R> fp = flux_prim<AX>(g, xr, x0, x1, xp);
-  return star ? fs : fp;
+  if (star) return star_flux<AX>(k, shockStar, shock, xr, x0, x1, xp);
+  return flux_prim<AX>(k, xr, x0, x1, xp);
 }
 
 template <class R> __device__ __forceinline__ R absmaller(R a, R b) {
   return (a * b <= R(0)) ? R(0) : ((fabs(a) < fabs(b)) ? a : b);
+}
+template <> __device__ __forceinline__ double absmaller(double a, double b) {
+  return xf::absmaller(a, b);
 }
 
 // interpolateSingle 2 (minmod MUSCL): face value left (l) and right (r)
@@ -127,8 +188,8 @@ __device__ __forceinline__ void muscl(R x0, R x1, R x2, R x3, R &l, R &r) {
   const R d01 = x1 - x0, d12 = x2 - x1, d23 = x3 - x2;
   const R d1 = absmaller(d01, d12);
   const R d2 = absmaller(d12, d23);
-  l = x1 + d1 / R(2);
-  r = x2 - d2 / R(2);
+  l = x1 + half(d1);
+  r = x2 - half(d2);
 }
 
 // Conservative update of base state b by the axis-1 walls, then the axis-0
@@ -136,12 +197,12 @@ __device__ __forceinline__ void muscl(R x0, R x1, R x2, R x3, R &l, R &r) {
 // bindPrimitive (max 1e-2 rho) v (max 1e-2 p).  cons (optional): the new
 // conserved state (rho, m0, m1, E) before the primitive recovery.
 template <class R>
-__device__ __forceinline__ Prim<R> update(R g, const Prim<R> &b, R dtdx0, R dtdx1,
+__device__ __forceinline__ Prim<R> update(const Gas<R> &k, const Prim<R> &b, R dtdx0, R dtdx1,
                                           const Flux<R> &l0, const Flux<R> &r0,
                                           const Flux<R> &l1, const Flux<R> &r1,
                                           R *cons = nullptr) {
   const R m0 = b.rho * b.v0, m1 = b.rho * b.v1;
-  const R e = kinetic(b.v0, b.v1, m0, m1) + (R(1) / (g - R(1))) * b.p;
+  const R e = kinetic(b.v0, b.v1, m0, m1) + k.gm1inv * b.p;
   const R d1 = b.rho + dtdx1 * (l1.fd - r1.fd);
   const R a0 = m0 + dtdx1 * (l1.fm0 - r1.fm0);
   const R a1 = m1 + dtdx1 * (l1.fm1 - r1.fm1);
@@ -156,8 +217,9 @@ __device__ __forceinline__ Prim<R> update(R g, const Prim<R> &b, R dtdx0, R dtdx
     cons[2] = b1;
     cons[3] = e2;
   }
-  const R v0 = b0 / d2, v1 = b1 / d2;
-  const R pn = (g - R(1)) * (e2 - kinetic(v0, v1, b0, b1));
+  const Divisor<R> d(d2);
+  const R v0 = d.under(b0), v1 = d.under(b1);
+  const R pn = k.gm1 * (e2 - kinetic(v0, v1, b0, b1));
   Prim<R> q;
   q.rho = omax(R(1e-2), d2);
   q.v0 = v0;
@@ -170,8 +232,8 @@ __device__ __forceinline__ Prim<R> update(R g, const Prim<R> &b, R dtdx0, R dtdx
 template <class R>
 __device__ __forceinline__ R timescale(R g, R dR0, R dR1, R rho, R v0, R v1, R p) {
   const R c = sound(g, rho, p);
-  const R t0 = dR0 / (c + fabs(v0));
-  const R t1 = dR1 / (c + fabs(v1));
+  const R t0 = div(dR0, c + fabs(v0));
+  const R t1 = div(dR1, c + fabs(v1));
   return omin(t0, t1);
 }
 
@@ -329,18 +391,8 @@ template <class T> __device__ __forceinline__ T splat(float c);
 template <> __device__ __forceinline__ float splat<float>(float c) { return c; }
 template <> __device__ __forceinline__ f2 splat<f2>(float c) { return pack(c, c); }
 
-template <class R> struct Consts {
-  R g, gm1, gm1inv, qc;  // gamma, gamma-1, 1/(gamma-1), (gamma+1)/(2 gamma)
-};
-
-template <class R> __device__ __forceinline__ Consts<R> consts(R g) {
-  Consts<R> k;
-  k.g = g;
-  k.gm1 = g - R(1);
-  k.gm1inv = R(1) / k.gm1;
-  k.qc = (g + R(1)) / (R(2) * g);
-  return k;
-}
+template <class R> using Consts = hs::Gas<R>;
+template <class R> __device__ __forceinline__ Consts<R> consts(R g) { return hs::gas(g); }
 
 // the constants of the algebra in the number type T
 template <class T> struct K {

@@ -41,10 +41,18 @@ struct LifeScalars {  // device/host scalar block
   uint32_t wait_error;  // raised by a kernel whose bounded wait ran out
 };
 
+// Populations kept in pinned host memory beside the scalars.  A run's results
+// are a few words that its last kernel writes there: copies around the run
+// (scalars in, scalars out, history out) cost more than small runs compute.
+static const int kHistory = 4096;
+
 struct LifeState {
   bool binary = true;           // every cell is known to be 0 or 1
-  uint32_t *d_pop = nullptr;    // populations of the last run, per generation
-  uint32_t *d_flag = nullptr;   // raised by the cell-value check
+  // populations of a run, per generation; all 0 between runs of at most
+  // kHistory generations, whose results go to the host block (pop_clear)
+  uint32_t *d_pop = nullptr;
+  bool pop_clear = false;
+  uint32_t *d_flag = nullptr;   // raised by the cell-value check; [1]: a wait ran out
   int pop_cap = 0;
   int last_n = 0;
   int depth = 0, tile_w = 0, tile_h = 0;  // tuned or configured
@@ -80,6 +88,9 @@ static int life_tmap(LifeState *st, const void *cells, int n0, int n1) {
 }
 
 static LifeState *life_state(Handle *h) { return (LifeState *)h->impl; }
+static uint32_t *life_history(Handle *h) {
+  return (uint32_t *)((char *)h->h_scalars + h->result_offset());
+}
 
 cudaError_t life_check_cells_into(const int32_t *cells, size_t n, uint32_t *flag,
                                   cudaStream_t s);
@@ -523,6 +534,7 @@ struct SmallParams {
   int gens;  // 1 .. kSmallMaxGens
   int nw;    // warps that advance rows; the block's others only move cells
   int h;     // halo rows each side, and generations between exchanges
+  int before;  // generations of the run before these (populations in pop)
 };
 static const int kSmallThreads = 512;
 static const int kSmallMaxGens = 4096;  // populations kept in shared memory
@@ -539,7 +551,7 @@ static const int kSmallMaxGens = 4096;  // populations kept in shared memory
 template <int R, bool RAG>
 __global__ void __launch_bounds__(kSmallThreads)
 life_smallreg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next, SmallParams p,
-                     uint32_t *__restrict__ pop) {
+                     uint32_t *__restrict__ pop, LifeScalars *scalars, uint32_t *hist) {
   extern __shared__ uint32_t S[];  // 2 x words, then the populations
   const int wd = p.wd, n1 = p.n1, nwords = wd * n1;
   uint32_t *spop = S + 2 * nwords;
@@ -666,7 +678,19 @@ life_smallreg_kernel(const int32_t *__restrict__ cur, int32_t *__restrict__ next
   }
   __syncthreads();
   const uint32_t *out = S + spop[p.gens];
-  for (int i = tid; i < p.gens; i += kSmallThreads) pop[i] += spop[i];
+  for (int i = tid; i < p.gens; i += kSmallThreads) {
+    if (hist) hist[p.before + i] = spop[i];
+    else pop[i] += spop[i];
+  }
+  if (hist && tid == 0) {
+    for (int i = 0; i < p.before; ++i) {
+      hist[i] = pop[i];
+      pop[i] = 0;
+    }
+    scalars->population = (int32_t)spop[p.gens - 1];
+    scalars->generation =
+        (int32_t)((uint32_t)scalars->generation + (uint32_t)(p.before + p.gens));
+  }
   for (int i = warp; i < nwords; i += NWB) {
     const int y = i / wd, x = (i - y * wd) * 32 + lane;
     if (x < p.n0) next[(size_t)y * p.n0 + x] = (int32_t)((out[i] >> lane) & 1u);
@@ -1305,9 +1329,28 @@ __global__ void life_fill_kernel(int32_t *cell, int n0, int n1, int ms0, int lm,
   cell[(y + lm) * ms0 + (x + lm)] = ((h >> 11) < thr) ? 1 : 0;
 }
 
-__global__ void life_finalize_kernel(LifeScalars *s, const uint32_t *pop, int n) {
-  s->population = (int32_t)pop[n - 1];
-  s->generation = (int32_t)((uint32_t)s->generation + (uint32_t)n);
+__global__ void life_reset_kernel(LifeScalars *s) { *s = LifeScalars{}; }
+
+// The run's results into the host block; hist (n <= kHistory): the populations,
+// which are cleared for the next run.
+__global__ void __launch_bounds__(256)
+life_finalize_kernel(LifeScalars *s, uint32_t *hist, uint32_t *pop, uint32_t *wait, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    if (!hist && i != n - 1) continue;
+    const uint32_t c = pop[i];
+    if (i == n - 1) {
+      s->population = (int32_t)c;
+      s->generation = (int32_t)((uint32_t)s->generation + (uint32_t)n);
+      if (*wait) {
+        s->wait_error = 1;
+        *wait = 0;
+      }
+    }
+    if (hist) {
+      hist[i] = c;
+      pop[i] = 0;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1318,7 +1361,8 @@ __global__ void life_finalize_kernel(LifeScalars *s, const uint32_t *pop, int n)
 static const int kSmallRows[] = {2, 3, 4, 5, 6, 8};
 static const int kNumSmallRows = 6;
 
-typedef void (*SmallKernel)(const int32_t *, int32_t *, SmallParams, uint32_t *);
+typedef void (*SmallKernel)(const int32_t *, int32_t *, SmallParams, uint32_t *, LifeScalars *,
+                            uint32_t *);
 template <bool RAG> static SmallKernel small_kernel(int v) {
   switch (v) {
     case 0: return life_smallreg_kernel<2, RAG>;
@@ -1405,7 +1449,7 @@ static om_status life_reserve(Handle *h, int kernel_id, int n) {
       }
   }
   if (n <= st->pop_cap) return OM_OK;
-  int cap = std::max(n, 1024);
+  int cap = std::max(n, kHistory);
   uint32_t *p = nullptr;
   if (cudaMalloc(&p, (size_t)cap * sizeof(uint32_t)) != cudaSuccess) {
     cudaGetLastError();
@@ -1416,6 +1460,7 @@ static om_status life_reserve(Handle *h, int kernel_id, int n) {
   if (st->d_pop) cudaFree(st->d_pop);
   st->d_pop = p;
   st->pop_cap = cap;
+  st->pop_clear = false;
   return OM_OK;
 }
 
@@ -1423,7 +1468,8 @@ static om_status life_init(Handle *h, int n) {
   (void)n;
   Array &a = h->arrays[0];
   OM_CUDA_CHECK(cudaMemsetAsync(a.d(), 0, a.count * sizeof(int32_t), h->stream));
-  OM_CUDA_CHECK(cudaMemsetAsync(h->d_scalars, 0, sizeof(LifeScalars), h->stream));
+  life_reset_kernel<<<1, 1, 0, h->stream>>>((LifeScalars *)h->d_scalars);
+  OM_CUDA_CHECK(cudaGetLastError());
   life_state(h)->binary = true;
   life_state(h)->last_n = 0;
   return OM_OK;
@@ -1801,7 +1847,7 @@ static om_status launch_ws_tiles(Handle *h, int v, int io, const void *in, void 
                                          : sm_count(h->device);
   cudaError_t e = launch_ws(v, io, in, out, q, pop, ctas, st->tmap[mi < 0 ? 0 : mi],
                             st->tpatch[mi < 0 ? 0 : mi],
-                            &((LifeScalars *)h->d_scalars)->wait_error, h->stream);
+                            st->d_flag + 1, h->stream);
   if (e != cudaSuccess) {
     set_error(std::string("life_ws_kernel: ") + cudaGetErrorString(e));
     return OM_ERR_CUDA;
@@ -1901,6 +1947,35 @@ static om_status proceed_packed(Handle *h, int n, int g) {
   return OM_OK;
 }
 
+// whether a run is one launch of the small kernel, which writes its results too
+static bool life_one_launch(const Handle *h, int n) {
+  return life_packed_ok(h) && life_small(h) && ((const LifeState *)h->impl)->binary &&
+         n <= kHistory;
+}
+
+// gens generations of a small grid; populations added to pop, or with hist
+// written there with the run's other results (and those of the `before`
+// generations in pop)
+static om_status launch_small(Handle *h, int gens, uint32_t *pop, uint32_t *hist, int before) {
+  Array &a = h->arrays[0];
+  const int n0 = h->size[0], n1 = h->size[1];
+  const SmallPlan pl = small_plan(n0, n1);
+  SmallParams sp{n0, n1, (n0 + 31) / 32, 0, gens, pl.nw, pl.h, before};
+  sp.nb = n0 - 32 * (sp.wd - 1);
+  const SmallKernel k = n0 % 32 ? small_kernel<true>(pl.v) : small_kernel<false>(pl.v);
+  const size_t smem = sizeof(uint32_t) * (2 * (size_t)sp.wd * n1 + gens + 1);
+  if (smem > 48 * 1024)
+    OM_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaEvent_t ev = prof_begin(h);
+  k<<<1, kSmallThreads, smem, h->stream>>>((const int32_t *)a.d(), (int32_t *)a.d_next(), sp, pop,
+                                           (LifeScalars *)h->d_scalars, hist);
+  OM_CUDA_CHECK(cudaGetLastError());
+  prof_end(h, ev, "life_smallreg_kernel", (double)n0 * n1 * gens);
+  h->launches++;
+  a.swap();
+  return OM_OK;
+}
+
 static om_status life_proceed(Handle *h, int n) {
   LifeState *st = life_state(h);
   if (n > st->pop_cap) {
@@ -1908,13 +1983,22 @@ static om_status life_proceed(Handle *h, int n) {
     return OM_ERR_STATE;
   }
   Array &a = h->arrays[0];
-  OM_CUDA_CHECK(cudaMemsetAsync(st->d_pop, 0, (size_t)n * sizeof(uint32_t), h->stream));
+  uint32_t *hist = n <= kHistory ? life_history(h) : nullptr;
   const int n0 = h->size[0], n1 = h->size[1];
   const bool ragged = n0 % 32 != 0;
   const bool small = life_small(h);
-  // on rows that are no whole number of words, a few generations are cheaper
+  // on rows that are no whole number of words, a single generation is cheaper
   // one cell per thread than packed, advanced and unpacked
-  const bool packed_ok = life_packed_ok(h) && (!ragged || n >= (small ? 4 : 2));
+  const bool packed_ok = life_packed_ok(h) && (!ragged || small || n >= 2);
+  if (life_one_launch(h, n)) {
+    OM_TRY(launch_small(h, n, nullptr, hist, 0));
+    st->last_n = n;
+    return OM_OK;
+  }
+  if (!st->pop_clear)
+    OM_CUDA_CHECK(cudaMemsetAsync(st->d_pop, 0, sizeof(uint32_t) * (size_t)std::max(n, kHistory),
+                                  h->stream));
+  st->pop_clear = false;
   int g = 0;
   if (!packed_ok || !st->binary) {
     const int first = packed_ok ? 1 : n;
@@ -1922,21 +2006,15 @@ static om_status life_proceed(Handle *h, int n) {
     st->binary = true;
   }
   if (g < n && packed_ok && small) {
-    const SmallPlan pl = small_plan(n0, n1);
-    SmallParams sp{n0, n1, (n0 + 31) / 32, 0, 0, pl.nw, pl.h};
-    sp.nb = n0 - 32 * (sp.wd - 1);
-    const SmallKernel k = ragged ? small_kernel<true>(pl.v) : small_kernel<false>(pl.v);
-    for (; g < n; g += sp.gens) {
-      sp.gens = std::min(n - g, kSmallMaxGens);
-      const size_t smem = sizeof(uint32_t) * (2 * (size_t)sp.wd * n1 + sp.gens + 1);
-      OM_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      cudaEvent_t ev = prof_begin(h);
-      k<<<1, kSmallThreads, smem, h->stream>>>((const int32_t *)a.d(), (int32_t *)a.d_next(), sp,
-                                               st->d_pop + g);
-      OM_CUDA_CHECK(cudaGetLastError());
-      prof_end(h, ev, "life_smallreg_kernel", (double)n0 * n1 * sp.gens);
-      h->launches++;
-      a.swap();
+    if (hist) {
+      OM_TRY(launch_small(h, n - g, st->d_pop, hist, g));
+      st->pop_clear = true;
+      st->last_n = n;
+      return OM_OK;
+    }
+    for (int gens; g < n; g += gens) {
+      gens = std::min(n - g, kSmallMaxGens);
+      OM_TRY(launch_small(h, gens, st->d_pop + g, nullptr, 0));
     }
   } else if (g < n && (ragged || life_run_packed(h, n - g))) {
     OM_TRY(proceed_packed(h, n, g));
@@ -2030,18 +2108,24 @@ static om_status life_proceed(Handle *h, int n) {
       }
     }
   }
-  life_finalize_kernel<<<1, 1, 0, h->stream>>>((LifeScalars *)h->d_scalars, st->d_pop, n);
+  life_finalize_kernel<<<1, 256, 0, h->stream>>>((LifeScalars *)h->d_scalars, hist, st->d_pop,
+                                                 st->d_flag + 1, n);
   OM_CUDA_CHECK(cudaGetLastError());
+  st->pop_clear = hist != nullptr;
   h->launches++;
   st->last_n = n;
   return OM_OK;
 }
 
-static uint64_t life_state_key(Handle *h) { return life_state(h)->binary ? 1 : 0; }
+static uint64_t life_state_key(Handle *h) {
+  const LifeState *st = life_state(h);
+  return (st->binary ? 1 : 0) | (st->pop_clear ? 2 : 0);
+}
 
 static void life_after_replay(Handle *h, int kernel_id, int n) {
   LifeState *st = life_state(h);
   if (h->kernels[kernel_id].name == "proceed") {
+    if (!life_one_launch(h, n)) st->pop_clear = n <= kHistory;
     st->binary = true;
     st->last_n = n;
   } else {
@@ -2050,7 +2134,11 @@ static void life_after_replay(Handle *h, int kernel_id, int n) {
   }
 }
 
-static void life_restore_key(Handle *h, uint64_t key) { life_state(h)->binary = key != 0; }
+static void life_restore_key(Handle *h, uint64_t key) {
+  LifeState *st = life_state(h);
+  st->binary = (key & 1) != 0;
+  st->pop_clear = (key & 2) != 0;
+}
 
 // New cell contents came from the host.  The packed kernels need every cell
 // in {0, 1}; one read-only pass (HBM speed, a fraction of one generation)
@@ -2160,19 +2248,22 @@ om_status life_setup(Handle *h) {
   h->ops.after_run = [](Handle *hh) -> om_status {
     LifeScalars *sc = (LifeScalars *)hh->h_scalars;
     if (!sc->wait_error) return OM_OK;
-    sc->wait_error = 0;  // cleared on the device by the next upload
+    sc->wait_error = 0;
     set_error("Life: a kernel's bounded wait for its tensor copies ran out; the cells of "
               "this run are unspecified");
     return OM_ERR_CUDA;
   };
   OM_TRY(alloc_array(h, "cell", sizeof(int32_t)));
-  if (cudaMalloc(&st->d_flag, sizeof(uint32_t)) != cudaSuccess) {
+  if (cudaMalloc(&st->d_flag, 2 * sizeof(uint32_t)) != cudaSuccess) {
     set_error("Life: cannot allocate the cell-value flag");
     return OM_ERR_NOMEM;
   }
+  OM_CUDA_CHECK(cudaMemsetAsync(st->d_flag, 0, 2 * sizeof(uint32_t), h->stream));
   h->scalars.push_back({"population", kInt, offsetof(LifeScalars, population)});
   h->scalars.push_back({"generation", kInt, offsetof(LifeScalars, generation)});
   h->scalar_bytes = sizeof(LifeScalars);
+  h->result_bytes = kHistory * sizeof(uint32_t);
+  h->scalars_on_host = true;
   h->kernels.push_back({"init", life_init});
   h->kernels.push_back({"proceed", life_proceed});
   return OM_OK;
@@ -2210,7 +2301,9 @@ extern "C" om_status om_life_population_history(om_handle H, int32_t *out, int n
   if (h->kind != OM_KIND_LIFE) { set_error("not a Life handle"); return OM_ERR_ARG; }
   LifeState *st = life_state(h);
   const int m = std::min(n, st->last_n);
-  if (m > 0) {
+  if (m > 0 && st->last_n <= kHistory) {
+    std::memcpy(out, life_history(h), (size_t)m * sizeof(int32_t));
+  } else if (m > 0) {
     OM_CUDA_CHECK(cudaSetDevice(h->device));
     OM_CUDA_CHECK(cudaMemcpyAsync(out, st->d_pop, (size_t)m * sizeof(int32_t),
                                   cudaMemcpyDeviceToHost, h->stream));

@@ -12,6 +12,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -130,13 +131,14 @@ om_status bring_host(Handle *h, Array &a) {
 om_status upload_scalars(Handle *h) {
   if (!h->scalar_bytes) return OM_OK;
   if (h->ops.before_upload) h->ops.before_upload(h);
+  if (h->scalars_on_host) return OM_OK;
   OM_CUDA_CHECK(cudaMemcpyAsync(h->d_scalars, h->h_scalars, h->scalar_bytes,
                                 cudaMemcpyHostToDevice, h->stream));
   return OM_OK;
 }
 
 om_status download_scalars(Handle *h) {
-  if (!h->scalar_bytes) return OM_OK;
+  if (!h->scalar_bytes || h->scalars_on_host) return OM_OK;
   OM_CUDA_CHECK(cudaMemcpyAsync(h->h_scalars, h->d_scalars, h->scalar_bytes,
                                 cudaMemcpyDeviceToHost, h->stream));
   return OM_OK;
@@ -188,6 +190,8 @@ struct om_handle_s {
     int launches = 0;
   };
   std::map<std::tuple<int, int, uint64_t>, GraphEntry> graphs;
+  // keys run once, by plain launches: a run is captured when it comes again
+  std::set<std::tuple<int, int, uint64_t>> once;
   int last_launches = 0;
 };
 
@@ -234,13 +238,15 @@ om_status create_handle(int kind, const int sizes[2], const om_config &cfg,
   h->own_stream = true;
   om_status s = setup(h, ctx);
   if (s == OM_OK && h->scalar_bytes) {
-    if (cudaMallocHost(&h->h_scalars, h->scalar_bytes) != cudaSuccess ||
-        cudaMalloc(&h->d_scalars, h->scalar_bytes) != cudaSuccess) {
+    const size_t bytes = h->result_offset() + h->result_bytes;
+    if (cudaMallocHost(&h->h_scalars, bytes) != cudaSuccess ||
+        (!h->scalars_on_host && cudaMalloc(&h->d_scalars, h->scalar_bytes) != cudaSuccess)) {
       cudaGetLastError();
       set_error("om_create: scalar block allocation failed");
       s = OM_ERR_NOMEM;
     } else {
-      std::memset(h->h_scalars, 0, h->scalar_bytes);
+      std::memset(h->h_scalars, 0, bytes);
+      if (h->scalars_on_host) h->d_scalars = h->h_scalars;
     }
   }
   if (s == OM_OK && cudaStreamSynchronize(h->stream) != cudaSuccess) {
@@ -314,8 +320,8 @@ om_status om_destroy(om_handle H) {
     cudaFree(a.dev[1]);
     if (a.host) cudaFreeHost(a.host);
   }
+  if (h->d_scalars && h->d_scalars != h->h_scalars) cudaFree(h->d_scalars);
   if (h->h_scalars) cudaFreeHost(h->h_scalars);
-  if (h->d_scalars) cudaFree(h->d_scalars);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   cudaGetLastError();
   delete H;
@@ -413,6 +419,10 @@ om_status om_run_n(om_handle H, int kernel_id, int n) {
   const uint64_t key2 = mask ^ (skey << 32);
   auto key = std::make_tuple(kernel_id, n, key2);
   auto it = H->graphs.find(key);
+  if (it == H->graphs.end() && H->once.insert(key).second) {
+    OM_TRY(run_plain(H, kernel_id, n));
+    return finish(h);
+  }
   if (it == H->graphs.end()) {
     om_handle_s::GraphEntry e;
     cudaGraph_t g = nullptr;

@@ -124,8 +124,14 @@ struct Handle {
   std::vector<Scalar> scalars;
   std::vector<Kernel> kernels;
   size_t scalar_bytes = 0;
+  // pinned host memory after the scalar block, for a kind's other results
+  size_t result_bytes = 0;
+  // kernels read and write the host block itself (few accesses per run):
+  // nothing is copied before and after a run, d_scalars is h_scalars
+  bool scalars_on_host = false;
   void *h_scalars = nullptr;  // pinned
   void *d_scalars = nullptr;
+  size_t result_offset() const { return (scalar_bytes + 255) / 256 * 256; }
   bool scalars_dirty = true;  // host scalar block changed since last upload
   void *impl = nullptr;       // kind-specific state
   void (*impl_free)(Handle *) = nullptr;

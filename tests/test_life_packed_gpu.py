@@ -79,3 +79,27 @@ def test_ragged_nonbinary_first_step(om_lib, oracle):
     assert np.array_equal(life.read("cell"), rc)
     assert np.array_equal(life.population_history(30), rp)
     life.close()
+
+
+def test_results_in_host_memory(om_lib, oracle):
+    # populations and scalars across runs that keep their history on the host
+    # (up to 4096 generations) and on the device, in any order, and host writes
+    # to the scalars between runs
+    for size in ((96, 40), (1500, 30), (2048, 160)):
+        init = oracle.life_bernoulli(size[0], size[1], 4, 0.35)
+        life = om_lib.Life(size)
+        life.write("cell", init)
+        total = 0
+        rc, rp = oracle.life_run(init, 4700, cyclic=True)
+        for k, gens in enumerate((3, 4100, 2, 2, 500, 7, 7, 7)):
+            if k == 4:
+                life.generation = 1000
+            life.proceed(gens)
+            assert np.array_equal(life.population_history(gens), rp[total:total + gens])
+            total += gens
+            assert life.population == rp[total - 1]
+            assert life.generation == (total if k < 4 else total - 4107 + 1000)
+        life.init()
+        assert life.population == 0 and life.generation == 0
+        assert life.population_history(5).size == 0
+        life.close()

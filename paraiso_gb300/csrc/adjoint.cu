@@ -867,7 +867,9 @@ static om_status launch_tape(Handle *h, AdjointScratch *s, void *const *in, void
   a.gamma = h->cfg.gamma;
   a.gamma_f = (float)h->cfg.gamma;
   a.sc = s->sc;
-  a.read_slot = read_slot;
+  a.ts_read = ts_word(read_slot);
+  a.ts_write = ts_word(1 - read_slot);
+  a.ts_clear = 0;
   a.dt_hist = s->dt_scratch;
   a.lm = 0;
   a.ms0 = h->size[0];

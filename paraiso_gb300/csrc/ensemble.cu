@@ -88,7 +88,9 @@ static om_status ens_upload_args(om_ensemble E) {
       x.gamma = E->gamma;
       x.gamma_f = (float)E->gamma;
       x.sc = E->d_sc + k;
-      x.read_slot = p;
+      x.ts_read = ts_word(p);
+      x.ts_write = ts_word(1 - p);
+      x.ts_clear = 0;
       x.dt_hist = &E->d_sc[k].dt_last;
       x.lm = 0;
       x.ms0 = E->n0[k];

@@ -123,15 +123,31 @@ static om_status ensure_tsmin(Handle *h) {
   return OM_OK;
 }
 
+// The three CFL minima that the steps of a run rotate through: the scalar
+// block's two and one beside it.  A step reads one, writes the next and sets
+// the third to all ones for the step after, so a run clears one instead of one
+// per step (a memset between two steps costs a small grid about 2 us of 12).
+static int ts_slot(Handle *h, int i) {
+  return i < 2 ? ts_word(i) : (int)(h->result_offset() / sizeof(unsigned long long));
+}
+// The slot that a run of n steps from slot r ends in, one of the scalar
+// block's: the rotation starts with 1 - r or, where that would end beside the
+// block, with the third.
+static int ts_final(int r, int n) { return n % 3 == 0 ? r : 1 - r; }
+
 static om_status proceed_fused(Handle *h, int n) {
   HydroState *st = hst(h);
   OM_TRY(ensure_tsmin(h));
   const double cells = (double)h->size[0] * h->size[1];
+  const int stile = !st->fp64 && st->variant != 2
+                        ? hydro_step_tile(st->tile, h->size[0], h->size[1], st->lm > 0, h->device,
+                                          h->cfg.grid_limit)
+                        : st->tile;
   const bool persist = !st->fp64 && st->variant != 2 && st->lm == 0 &&
-                       hydro_tile_is_persistent(st->tile) &&
+                       hydro_tile_is_persistent(stile) &&
                        hydro_persist_fits(h->size[0], h->size[1]);
   // the persistent kernel's form that runs (the profile name follows it)
-  const int form = persist ? hydro_persist_form_for(hydro_persist_form(st->tile),
+  const int form = persist ? hydro_persist_form_for(hydro_persist_form(stile),
                                                     (long long)(h->size[0] / 32) * (h->size[1] / 32),
                                                     h->device, h->cfg.grid_limit)
                            : -1;
@@ -141,9 +157,11 @@ static om_status proceed_fused(Handle *h, int n) {
                                             : form == 1 ? "hydro_pair_kernel"
                                                         : "hydro_persist_kernel")
                                          : "hydro_fused_kernel_f32";
+  int rd = st->slot, wr = n % 3 == 2 ? 2 : 1 - rd;
+  OM_CUDA_CHECK(cudaMemsetAsync((unsigned long long *)h->d_scalars + ts_slot(h, wr), 0xFF,
+                                sizeof(unsigned long long), h->stream));
   for (int k = 0; k < n; ++k) {
-    OM_CUDA_CHECK(cudaMemsetAsync(&hsc_dev(h)->tsmin[1 - st->slot], 0xFF,
-                                  sizeof(unsigned long long), h->stream));
+    const int third = 3 - rd - wr;
     HydroStepArgs a;
     a.rho = h->arrays[0].d(); a.v0 = h->arrays[1].d();
     a.v1 = h->arrays[2].d(); a.p = h->arrays[3].d();
@@ -154,7 +172,9 @@ static om_status proceed_fused(Handle *h, int n) {
     a.gamma = h->cfg.gamma;
     a.gamma_f = (float)h->cfg.gamma;
     a.sc = hsc_dev(h);
-    a.read_slot = st->slot;
+    a.ts_read = ts_slot(h, rd);
+    a.ts_write = ts_slot(h, wr);
+    a.ts_clear = k + 1 < n ? ts_slot(h, third) : 0;
     a.dt_hist = st->d_dt + k;
     a.lm = st->lm;
     a.ms0 = (int)h->memory_size(0);
@@ -162,7 +182,7 @@ static om_status proceed_fused(Handle *h, int n) {
     a.grid_limit = h->cfg.grid_limit;
     cudaEvent_t ev = prof_begin(h);
     cudaError_t e = st->fp64 ? hydro_fused_f64(a, st->tile, h->stream, nullptr)
-                             : hydro_fused_f32(a, st->tile, st->variant == 2, h->stream, nullptr);
+                             : hydro_fused_f32(a, stile, st->variant == 2, h->stream, nullptr);
     if (e != cudaSuccess) {
       set_error(std::string("Hydro fused step: ") + cudaGetErrorString(e));
       return OM_ERR_CUDA;
@@ -170,8 +190,10 @@ static om_status proceed_fused(Handle *h, int n) {
     prof_end(h, ev, kname, cells);
     h->launches++;
     for (int i = 0; i < 4; ++i) h->arrays[i].swap();
-    st->slot = 1 - st->slot;
+    rd = wr;
+    wr = third;
   }
+  st->slot = rd;
   st->last_n = n;
   return OM_OK;
 }
@@ -260,7 +282,7 @@ static void hydro_after_replay(Handle *h, int kernel_id, int n) {
   HydroState *st = hst(h);
   if (h->kernels[kernel_id].name == "proceed") {
     ts_mark_current(h);
-    st->slot ^= (n & 1);
+    st->slot = ts_final(st->slot, n);
     st->last_n = n;
   } else {
     st->ts_valid = false;
@@ -446,6 +468,7 @@ om_status hydro_setup(Handle *h) {
   h->scalars.push_back({"extent0", kDouble, offsetof(HydroScalars, extent0)});
   h->scalars.push_back({"extent1", kDouble, offsetof(HydroScalars, extent1)});
   h->scalar_bytes = sizeof(HydroScalars);
+  h->result_bytes = sizeof(unsigned long long);  // the third CFL minimum (ts_slot)
   h->kernels.push_back({"init", hydro_init});
   h->kernels.push_back({"proceed", hydro_proceed});
   const size_t cells = h->memory_size_total();

@@ -35,9 +35,8 @@ static cudaError_t launch_fused(const HydroStepArgs &a0, cudaStream_t s, int *gr
   cudaError_t e = cudaFuncSetAttribute(hydro_fused_kernel<R, TX, TY, NT, OPEN>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  hydro_fused_kernel<R, TX, TY, NT, OPEN><<<a.nt0 * nt1, NT, smem, s>>>(a);
   if (grid_out) *grid_out = a.nt0 * nt1;
-  return cudaGetLastError();
+  return launch_step(hydro_fused_kernel<R, TX, TY, NT, OPEN, false>, a.nt0 * nt1, NT, smem, s, a);
 }
 
 template <class R>

@@ -22,9 +22,9 @@ static cudaError_t launch_fast(const HydroStepArgs &a0, cudaStream_t s, int *gri
   cudaError_t e = cudaFuncSetAttribute(hydro_fused_kernel<float, TX, TY, NT, OPEN, true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  hydro_fused_kernel<float, TX, TY, NT, OPEN, true><<<a.nt0 * nt1, NT, smem, s>>>(a);
   if (grid_out) *grid_out = a.nt0 * nt1;
-  return cudaGetLastError();
+  return launch_step(hydro_fused_kernel<float, TX, TY, NT, OPEN, true>, a.nt0 * nt1, NT, smem, s,
+                     a);
 }
 
 // The production sweep over a periodic grid: strips of TX columns, segments
@@ -159,12 +159,41 @@ cudaError_t hydro_fused_tape(int fp64, bool exact, const HydroStepArgs &a0, cons
   }
 }
 
+// A grid with at most a tile or two per SM is bound by the chain of a tile's
+// five phases, not by throughput: more threads per cell shorten it.  Measured
+// per step in a captured run of 50 (us; 32 x 32 or persistent tiles first):
+//   64^2   8.5, 16 x 8 by 256 threads 4.3      100^2 8.3, 4.8
+//   128^2  8.3, 16 x 8 5.65, 32 x 16 by 1024 5.56
+//   256^2  11.4, 32 x 16 by 1024 5.56, by 512 11.6, 32 x 8 by 512 7.5
+//   384 x 256 (192 tiles of 32 x 16 on 152 SMs)  12.0, by 512 8.2, by 1024 9.3
+//   500 x 300 (304)  12.2, by 512 8.5, by 1024 9.8
+//   512^2 (512)  persistent 12.3, 32 x 16 by 512 13.3
+//   500 x 700 (704, not persistent)  17.6, 32 x 16 by 512 15.9
+//   1000 x 700 (1408)  27.4, 32 x 16 by 512 28.4
+int hydro_step_tile(int tile, int n0, int n1, bool open, int device, int grid_limit) {
+  if (grid_limit > 0 || !(open || tile == kPairGroups32x32)) return tile;
+  const long long sms = sm_count(device);
+  auto tiles = [&](int tx, int ty) { return (long long)((n0 + tx - 1) / tx) * ((n1 + ty - 1) / ty); };
+  if (!open && tiles(16, 8) <= sms) return kThin16x8;
+  if (tiles(32, 16) <= sms) return kThin32x16;
+  if (tiles(32, 16) <= 2 * sms) return kThin32x16h;
+  if (!open && !hydro_persist_fits(n0, n1) && tiles(32, 16) <= 6 * sms) return kThin32x16h;
+  return tile;
+}
+
 cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaStream_t s,
                             int *grid_out) {
   if (exact) return hydro_fused_f32_exact(a, s, grid_out);
-  // an open grid (margins, jet boundary condition) runs the 32x16 tile
-  if (a.lm > 0) return launch_fast<32, 16, 256, true>(a, s, grid_out);
+  // an open grid (margins, jet boundary condition) runs 32x16 tiles
+  if (a.lm > 0) switch (tile) {
+    case kThin32x16: return launch_fast<32, 16, 1024, true>(a, s, grid_out);
+    case kThin32x16h: return launch_fast<32, 16, 512, true>(a, s, grid_out);
+    default: return launch_fast<32, 16, 256, true>(a, s, grid_out);
+  }
   switch (tile) {
+    case kThin16x8: return launch_fast<16, 8, 256>(a, s, grid_out);
+    case kThin32x16: return launch_fast<32, 16, 1024>(a, s, grid_out);
+    case kThin32x16h: return launch_fast<32, 16, 512>(a, s, grid_out);
     case kPersist32x32:
     case kPair32x32:
     case kPairGroups32x32:

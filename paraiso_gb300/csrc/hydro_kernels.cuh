@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "hydro_scheme.cuh"
@@ -45,16 +46,27 @@ struct HydroStepArgs {
   double gamma;
   float gamma_f;                   // (float)gamma
   HydroScalars *sc;
-  int read_slot;                   // tsmin slot holding min of the current state
+  // words of the scalar block's allocation that hold the CFL minimum of the
+  // current state, that of the new one (all ones before the step), and one
+  // that the step sets to all ones for the step after (0: none)
+  int ts_read, ts_write, ts_clear;
+  // persistent kernels: at most this many CTAs (0 = as many as stay
+  // resident); read by the host launcher only
+  int grid_limit;
   double *dt_hist;                 // dt of this step is written to dt_hist[0]
   // open boundary only (the OPEN kernels): margin width, memory row pitch
   // (n0 + 2 lm) and the CFL timescale minimum of the margin cells
   int lm, ms0;
   const unsigned long long *margin_min;
-  // persistent kernels: at most this many CTAs (0 = as many as stay
-  // resident); read by the host launcher only
-  int grid_limit;
 };
+
+// word of the scalar block that is tsmin[slot]
+constexpr int ts_word(int slot) {
+  return (int)(offsetof(HydroScalars, tsmin) / sizeof(unsigned long long)) + slot;
+}
+__device__ __forceinline__ unsigned long long *ts_at(const HydroStepArgs &a, int word) {
+  return reinterpret_cast<unsigned long long *>(a.sc) + word;
+}
 
 // What a taped step keeps for the reverse sweep (periodic grids; arrays of
 // n0 x n1 values of the OM's Real type): the stage-1 state q; per stage the
@@ -170,9 +182,17 @@ template <> struct Reals<double> {
   static __device__ __forceinline__ double gamma(const HydroStepArgs &a) { return a.gamma; }
 };
 
+// Programmatic dependent launch: the next step's blocks may be scheduled while
+// this one drains (launch_dependents), and wait for its completion before they
+// read or write anything (wait).  Both do nothing in an ordinary launch.
+__device__ __forceinline__ void step_begin() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 // dt of this step in the OM's Real type: dtG = cfl * reduce Min dts
 template <class R> __device__ __forceinline__ R step_dt(const HydroStepArgs &a) {
-  const R tsmin = ts_from_bits<R>(a.sc->tsmin[a.read_slot]);
+  const R tsmin = ts_from_bits<R>(*ts_at(a, a.ts_read));
   return Reals<R>::cfl(a.sc) * tsmin;
 }
 
@@ -461,9 +481,10 @@ __device__ __forceinline__ void fused_tile(const HydroStepArgs &a, int tile,
       }
     }
   }
-  hk::block_min_to(m, &a.sc->tsmin[1 - a.read_slot], red);
-  if (OPEN && tile == 0 && tid == 0) atomicMin(&a.sc->tsmin[1 - a.read_slot], *a.margin_min);
+  hk::block_min_to(m, ts_at(a, a.ts_write), red);
+  if (OPEN && tile == 0 && tid == 0) atomicMin(ts_at(a, a.ts_write), *a.margin_min);
   if (tile == 0 && tid == 0) {
+    if (a.ts_clear) *ts_at(a, a.ts_clear) = ~0ull;
     a.dt_hist[0] = (double)dtG;
     a.sc->dt_last = (double)dtG;
     a.sc->time = a.sc->time + (double)dtG;
@@ -475,6 +496,7 @@ __global__ void __launch_bounds__(NT)
 hydro_fused_kernel(HydroStepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned long long red[32];
+  hk::step_begin();
   fused_tile<R, TX, TY, NT, OPEN, false, FA>(
       a, blockIdx.x, *reinterpret_cast<FusedSmem<R, TX, TY> *>(smem_raw), red);
 }

@@ -11,6 +11,24 @@
 
 namespace om {
 
+// A step's launch that may be scheduled while the step before it drains (the
+// kernel starts with hk::step_begin).
+template <class... P, class... A>
+cudaError_t launch_step(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s,
+                        A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Tile shapes of the fused kernel available to the tuner (FP32 production
 // build; FP64 and the exact FP32 variant run 32x16).
 // The sweep shapes (kSweep*) walk strips of TX columns down the grid in
@@ -23,8 +41,16 @@ namespace om {
 enum HydroTile {
   kTile32x8 = 0, kTile32x16 = 1, kTile64x16 = 2, kTile32x32 = 3, kTile64x8 = 4,
   kSweep32x8 = 5, kSweep32x16 = 6, kSweep64x8 = 7, kPersist32x32 = 8, kPair32x32 = 9,
-  kPairGroups32x32 = 10, kTileCount = 11
+  kPairGroups32x32 = 10, kTileCount = 11,
+  // shapes with more threads per cell that the default choice takes on grids
+  // too small to fill the GPU (hydro_step_tile): 16 x 8 cells by 256 threads,
+  // 32 x 16 by 1024 and by 512
+  kThin16x8 = 11, kThin32x16 = 12, kThin32x16h = 13
 };
+// The tile a step of the production build runs: `tile`, but on small grids of
+// the default configuration (kPairGroups32x32, no grid_limit) or with the open
+// boundary a shape whose phases take fewer rounds of the block's threads.
+int hydro_step_tile(int tile, int n0, int n1, bool open, int device, int grid_limit);
 inline bool hydro_tile_is_persistent(int tile) {
   return tile == kPersist32x32 || tile == kPair32x32 || tile == kPairGroups32x32;
 }

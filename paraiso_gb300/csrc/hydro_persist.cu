@@ -92,8 +92,9 @@ static cudaError_t persist_launch(const HydroStepArgs &a0, const HydroTapeOut *t
   if (a.grid_limit > 0) grid = std::min(grid, a.grid_limit);
   HydroTapeOut t{};
   if (tape) t = *tape;
-  kernel<<<grid, threads, smem, s>>>(a, m[0], m[1], m[2], m[3], t);
   if (grid_out) *grid_out = grid;
+  if (!TAPE) return launch_step(kernel, grid, threads, smem, s, a, m[0], m[1], m[2], m[3], t);
+  kernel<<<grid, threads, smem, s>>>(a, m[0], m[1], m[2], m[3], t);
   return cudaGetLastError();
 }
 

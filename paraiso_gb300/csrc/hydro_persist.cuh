@@ -667,6 +667,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
         sounds(s.box[b ^ 1], hf::consts<float>(args[lo_n].gamma_f), tid - ONE, NTH - ONE);
     }
     if (tile == 0 && tid == 0) {
+      if (A.ts_clear) *ts_at(A, A.ts_clear) = ~0ull;
       A.dt_hist[0] = (double)dtG;
       A.sc->dt_last = (double)dtG;
       A.sc->time = A.sc->time + (double)dtG;
@@ -677,7 +678,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     // publish the CFL minimum when this CTA leaves the instance (the
     // reduction ends with a barrier); else one barrier before the next tile
     if (next >= total || lo_n != lo) {
-      min_to(m, &A.sc->tsmin[1 - A.read_slot]);
+      min_to(m, ts_at(A, A.ts_write));
       m = ~0ull;
     } else {
       sync();
@@ -696,6 +697,7 @@ hydro_persist_kernel(HydroStepArgs a, const __grid_constant__ CUtensorMap m0,
                      const __grid_constant__ CUtensorMap m2,
                      const __grid_constant__ CUtensorMap m3, HydroTapeOut tape) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  hk::step_begin();
   persist_run<TAPE, false, false>(&a, nullptr, 1, nullptr, &m0, &m1, &m2, &m3,
                                   reinterpret_cast<Smem *>(smem_raw), &tape);
 }
@@ -706,6 +708,7 @@ hydro_pair_kernel(HydroStepArgs a, const __grid_constant__ CUtensorMap m0,
                   const __grid_constant__ CUtensorMap m1, const __grid_constant__ CUtensorMap m2,
                   const __grid_constant__ CUtensorMap m3, HydroTapeOut tape) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  hk::step_begin();
   persist_run<TAPE, false, true>(&a, nullptr, 1, nullptr, &m0, &m1, &m2, &m3,
                                  reinterpret_cast<Smem *>(smem_raw), &tape);
 }
@@ -719,6 +722,7 @@ hydro_pair2_kernel(HydroStepArgs a, const __grid_constant__ CUtensorMap m0,
                    const __grid_constant__ CUtensorMap m1, const __grid_constant__ CUtensorMap m2,
                    const __grid_constant__ CUtensorMap m3, HydroTapeOut tape) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  hk::step_begin();
   persist_run<TAPE, false, true, 2>(&a, nullptr, 1, nullptr, &m0, &m1, &m2, &m3,
                                     reinterpret_cast<Smem *>(smem_raw), &tape);
 }

@@ -244,6 +244,7 @@ __device__ __forceinline__ void sweep_segment(const HydroStepArgs &a, int X0, in
 template <class R>
 __device__ __forceinline__ void sweep_advance_time(const HydroStepArgs &a) {
   const R dtG = hk::step_dt<R>(a);
+  if (a.ts_clear) *ts_at(a, a.ts_clear) = ~0ull;
   a.dt_hist[0] = (double)dtG;
   a.sc->dt_last = (double)dtG;
   a.sc->time = a.sc->time + (double)dtG;
@@ -283,7 +284,7 @@ hydro_sweep_kernel(HydroStepArgs a, SweepGeom geo, const __grid_constant__ Hydro
   const int ya = seg * geo.seg, yb = min(a.n1, ya + geo.seg);
   unsigned long long m = ~0ull;
   sweep_segment<R, TX, TY, NT, TAPE, FA>(a, strip * TX, ya, yb, s, m, &t);
-  hk::block_min_to(m, &a.sc->tsmin[1 - a.read_slot], red);
+  hk::block_min_to(m, ts_at(a, a.ts_write), red);
   if (blockIdx.x == 0 && threadIdx.x == 0) sweep_advance_time<R>(a);
 }
 

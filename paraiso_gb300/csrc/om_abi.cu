@@ -240,7 +240,7 @@ om_status create_handle(int kind, const int sizes[2], const om_config &cfg,
   if (s == OM_OK && h->scalar_bytes) {
     const size_t bytes = h->result_offset() + h->result_bytes;
     if (cudaMallocHost(&h->h_scalars, bytes) != cudaSuccess ||
-        (!h->scalars_on_host && cudaMalloc(&h->d_scalars, h->scalar_bytes) != cudaSuccess)) {
+        (!h->scalars_on_host && cudaMalloc(&h->d_scalars, bytes) != cudaSuccess)) {
       cudaGetLastError();
       set_error("om_create: scalar block allocation failed");
       s = OM_ERR_NOMEM;

@@ -124,7 +124,7 @@ struct Handle {
   std::vector<Scalar> scalars;
   std::vector<Kernel> kernels;
   size_t scalar_bytes = 0;
-  // pinned host memory after the scalar block, for a kind's other results
+  // memory after the scalar block (host and device), for a kind's other results
   size_t result_bytes = 0;
   // kernels read and write the host block itself (few accesses per run):
   // nothing is copied before and after a run, d_scalars is h_scalars

@@ -209,11 +209,14 @@ XF_FN double sqrt_rn(double x) {
   return from_bits(q + ((uint64_t)e << 32));
 }
 
+XF_SLOW double half_plain(double x) { return x * 0.5; }
+
 // x / 2
 XF_FN double half(double x) {
   const uint64_t u = bits(x);
   if (plain_exponent(hi32(u))) return from_bits(u - 0x0010000000000000ull);
-  return x * 0.5;
+  if ((u << 1) == 0) return x;
+  return half_plain(x);
 }
 
 // 0 + x: x, but 0 for -0

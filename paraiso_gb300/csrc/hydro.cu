@@ -8,7 +8,7 @@
 // Paths (om_config.precision / .variant):
 //   precision 32, variant 0  fused tiled step, FP32, multiply-add contraction
 //   precision 32, variant 2  fused tiled step, FP32, exact operation order
-//   precision 64, variant 0  fused tiled step, FP64, exact operation order
+//   precision 64, variant 0  two-kernel tiled step, FP64, exact operation order
 //   precision 32/64, variant 1  plain path: the generated structure (timescale
 //                            pass, min-reduce with a host round trip,
 //                            all-Delayed recompute step, manifest copies)
@@ -36,6 +36,7 @@ struct HydroState {
   double ts_ext1 = 0;             // extent1 it was computed with (open grids)
   int lm = 0;                     // margin width: 3 on an open grid, else 0
   unsigned long long *d_margin = nullptr;  // open grid: margin cells' CFL minimum
+  HydroStage1 q{};             // FP64: the stage-1 state (one allocation, q[0] its base)
   double *d_dt = nullptr;      // dt history of the last run
   int dt_cap = 0;
   int last_n = 0;
@@ -151,7 +152,7 @@ static om_status proceed_fused(Handle *h, int n) {
                                                     (long long)(h->size[0] / 32) * (h->size[1] / 32),
                                                     h->device, h->cfg.grid_limit)
                            : -1;
-  const char *kname = st->fp64 ? "hydro_fused_kernel_f64"
+  const char *kname = st->fp64 ? "hydro_stage_kernels_f64"
                       : st->variant == 2 ? "hydro_fused_kernel_f32_exact"
                       : persist          ? (form == 2   ? "hydro_pair2_kernel"
                                             : form == 1 ? "hydro_pair_kernel"
@@ -181,14 +182,14 @@ static om_status proceed_fused(Handle *h, int n) {
     a.margin_min = st->d_margin;
     a.grid_limit = h->cfg.grid_limit;
     cudaEvent_t ev = prof_begin(h);
-    cudaError_t e = st->fp64 ? hydro_fused_f64(a, st->tile, h->stream, nullptr)
+    cudaError_t e = st->fp64 ? hydro_step_f64(a, st->q, h->stream)
                              : hydro_fused_f32(a, stile, st->variant == 2, h->stream, nullptr);
     if (e != cudaSuccess) {
       set_error(std::string("Hydro fused step: ") + cudaGetErrorString(e));
       return OM_ERR_CUDA;
     }
     prof_end(h, ev, kname, cells);
-    h->launches++;
+    h->launches += st->fp64 ? 2 : 1;
     for (int i = 0; i < 4; ++i) h->arrays[i].swap();
     rd = wr;
     wr = third;
@@ -302,6 +303,7 @@ static void hydro_free(Handle *h) {
   if (!st) return;
   adjoint_release(h);
   cudaFree(st->d_dt);
+  cudaFree(st->q.q[0]);
   cudaFree(st->d_ts);
   cudaFree(st->d_min);
   cudaFree(st->d_margin);
@@ -472,6 +474,16 @@ om_status hydro_setup(Handle *h) {
   h->kernels.push_back({"init", hydro_init});
   h->kernels.push_back({"proceed", hydro_proceed});
   const size_t cells = h->memory_size_total();
+  if (st->fp64 && st->variant == 0) {
+    const size_t pitch = (cells * es + 255) / 256 * 256;
+    if (cudaMalloc(&st->q.q[0], 4 * pitch) != cudaSuccess) {
+      cudaGetLastError();
+      st->q.q[0] = nullptr;
+      set_error("Hydro: cannot allocate the stage-1 state");
+      return OM_ERR_NOMEM;
+    }
+    for (int i = 1; i < 4; ++i) st->q.q[i] = (char *)st->q.q[0] + pitch * i;
+  }
   if (cudaMalloc(&st->d_ts, cells * es) != cudaSuccess ||
       cudaMalloc(&st->d_min, sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&st->d_margin, sizeof(unsigned long long)) != cudaSuccess ||

@@ -59,11 +59,27 @@ cudaError_t hydro_fused_tape_exact(int fp64, const HydroStepArgs &a, const Hydro
   return fp64 ? launch_tape<double>(a, t, s) : launch_tape<float>(a, t, s);
 }
 
+// The FP64 step as two kernels on 16 x 16 tiles: small tiles spread a grid
+// evenly over the SMs, whose double pipes are what bounds it (384 x 256 is 192
+// tiles of 32 x 16: some SMs had twice the work of others).
+template <bool OPEN>
+static cudaError_t launch_f64(const HydroStepArgs &a0, const HydroStage1 &q, cudaStream_t s) {
+  constexpr int TX = 16, TY = 16, NT = 256, e = OPEN ? 2 : 0;
+  HydroStepArgs a = a0;
+  a.nt0 = (a.n0 + 2 * e + TX - 1) / TX;
+  const int nt1 = (a.n1 + 2 * e + TY - 1) / TY;
+  cudaError_t err = launch_step(hydro_stage1_kernel<double, TX, TY, NT, OPEN>, a.nt0 * nt1, NT,
+                                sizeof(Stage1Smem<double, TX, TY>), s, a, q);
+  if (err != cudaSuccess) return err;
+  a.nt0 = (a.n0 + TX - 1) / TX;
+  return launch_step(hydro_stage2_kernel<double, TX, TY, NT, OPEN>,
+                     a.nt0 * ((a.n1 + TY - 1) / TY), NT, sizeof(Stage2Smem<double, TX, TY>), s, a,
+                     q);
+}
+
 // a.lm > 0: open grid (margins, jet boundary condition)
-cudaError_t hydro_fused_f64(const HydroStepArgs &a, int tile, cudaStream_t s, int *grid_out) {
-  (void)tile;  // one shape in FP64: 32x16 (104 KB of shared memory)
-  return a.lm > 0 ? launch_fused<double, 32, 16, 256, true>(a, s, grid_out)
-                  : launch_fused<double, 32, 16, 256, false>(a, s, grid_out);
+cudaError_t hydro_step_f64(const HydroStepArgs &a, const HydroStage1 &q, cudaStream_t s) {
+  return a.lm > 0 ? launch_f64<true>(a, q, s) : launch_f64<false>(a, q, s);
 }
 
 // exact FP32 variant (the fast build lives in hydro_fast.cu)

@@ -196,6 +196,37 @@ template <class R> __device__ __forceinline__ R step_dt(const HydroStepArgs &a) 
   return Reals<R>::cfl(a.sc) * tsmin;
 }
 
+// The margin cells of an open grid beside the tile at (X0, Y0) are set to 0:
+// the generated class copies whole manifests, whose margins are zero, into the
+// statics.
+template <class R, int TX, int TY, int NT>
+__device__ __forceinline__ void clear_margins(const HydroStepArgs &a, int X0, int Y0,
+                                              R *const (&out)[4]) {
+  const int n0 = a.n0, n1 = a.n1, lm = a.lm;
+  const int xa = X0 == 0 ? -lm : X0, xb = X0 + TX >= n0 ? n0 + lm : X0 + TX;
+  const int ya = Y0 == 0 ? -lm : Y0, yb = Y0 + TY >= n1 ? n1 + lm : Y0 + TY;
+  if (xa >= 0 && ya >= 0 && xb <= n0 && yb <= n1) return;
+  const int w = xb - xa, cnt = w * (yb - ya);
+  for (int i = threadIdx.x; i < cnt; i += NT) {
+    const int y = ya + i / w, x = xa + i % w;
+    if (x >= 0 && y >= 0 && x < n0 && y < n1) continue;
+    const size_t gi = (size_t)(y + lm) * a.ms0 + (x + lm);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) out[c][gi] = R(0);
+  }
+}
+
+// what a step's tile 0 does for the whole step
+template <class R, bool OPEN>
+__device__ __forceinline__ void step_end(const HydroStepArgs &a, int tile, R dtG) {
+  if (tile != 0 || threadIdx.x != 0) return;
+  if (OPEN) atomicMin(ts_at(a, a.ts_write), *a.margin_min);
+  if (a.ts_clear) *ts_at(a, a.ts_clear) = ~0ull;
+  a.dt_hist[0] = (double)dtG;
+  a.sc->dt_last = (double)dtG;
+  a.sc->time = a.sc->time + (double)dtG;
+}
+
 // 4- or 8-byte asynchronous copy global -> shared, and its group fences
 template <class R> __device__ __forceinline__ void cp_async(R *dst, const R *src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -365,7 +396,7 @@ __device__ __forceinline__ void fused_tile(const HydroStepArgs &a, int tile,
 
   // phase 2: stage-1 cells
   {
-    const R dtdx0 = dtHalf / dR0, dtdx1 = dtHalf / dR1;
+    const R dtdx0 = hs::div(dtHalf, dR0), dtdx1 = hs::div(dtHalf, dR1);
     for (int i = tid; i < S::QY * S::QX; i += NT) {
       const int qy = i / S::QX, qx = i - qy * S::QX;
       const int py = qy + 1, px = qx + 1;
@@ -433,7 +464,7 @@ __device__ __forceinline__ void fused_tile(const HydroStepArgs &a, int tile,
   // phase 4: stage-2 cells, written out, with the CFL minimum of the new state
   unsigned long long m = ~0ull;
   {
-    const R dtdx0 = dtG / dR0, dtdx1 = dtG / dR1;
+    const R dtdx0 = hs::div(dtG, dR0), dtdx1 = hs::div(dtG, dR1);
     R *orho = (R *)a.nrho, *ovx = (R *)a.nv0, *ovy = (R *)a.nv1, *opr = (R *)a.np;
     for (int i = tid; i < TY * TX; i += NT) {
       const int oy = i / TX, ox = i - oy * TX;
@@ -462,33 +493,11 @@ __device__ __forceinline__ void fused_tile(const HydroStepArgs &a, int tile,
     }
   }
   if (OPEN) {
-    // the generated class copies whole manifests, whose margins are zero,
-    // into the statics: tiles on the grid edge clear the adjacent margins
-    const int lm = a.lm;
-    const int xa = X0 == 0 ? -lm : X0, xb = X0 + TX >= n0 ? n0 + lm : X0 + TX;
-    const int ya = Y0 == 0 ? -lm : Y0, yb = Y0 + TY >= n1 ? n1 + lm : Y0 + TY;
-    const int w = xb - xa, cnt = w * (yb - ya);
-    if (xa < 0 || ya < 0 || xb > n0 || yb > n1) {
-      R *orho = (R *)a.nrho, *ovx = (R *)a.nv0, *ovy = (R *)a.nv1, *opr = (R *)a.np;
-      for (int i = tid; i < cnt; i += NT) {
-        const int y = ya + i / w, x = xa + i % w;
-        if (x >= 0 && y >= 0 && x < n0 && y < n1) continue;
-        const size_t gi = (size_t)(y + lm) * a.ms0 + (x + lm);
-        orho[gi] = R(0);
-        ovx[gi] = R(0);
-        ovy[gi] = R(0);
-        opr[gi] = R(0);
-      }
-    }
+    R *out[4] = {(R *)a.nrho, (R *)a.nv0, (R *)a.nv1, (R *)a.np};
+    hk::clear_margins<R, TX, TY, NT>(a, X0, Y0, out);
   }
   hk::block_min_to(m, ts_at(a, a.ts_write), red);
-  if (OPEN && tile == 0 && tid == 0) atomicMin(ts_at(a, a.ts_write), *a.margin_min);
-  if (tile == 0 && tid == 0) {
-    if (a.ts_clear) *ts_at(a, a.ts_clear) = ~0ull;
-    a.dt_hist[0] = (double)dtG;
-    a.sc->dt_last = (double)dtG;
-    a.sc->time = a.sc->time + (double)dtG;
-  }
+  hk::step_end<R, OPEN>(a, tile, dtG);
 }
 
 template <class R, int TX, int TY, int NT, bool OPEN = false, bool FA = false>
@@ -499,6 +508,204 @@ hydro_fused_kernel(HydroStepArgs a) {
   hk::step_begin();
   fused_tile<R, TX, TY, NT, OPEN, false, FA>(
       a, blockIdx.x, *reinterpret_cast<FusedSmem<R, TX, TY> *>(smem_raw), red);
+}
+
+// ---------------------------------------------------------------------------
+// The step as two kernels with the stage-1 state in global memory between them.
+// A double-precision step is bound by its arithmetic (two results a cycle per
+// SM), and the fused tile's halo repeats a third of it: 2.9 stage-1 walls and
+// 1.4 stage-1 cells per cell of a 32 x 16 tile.  Here every cell is advanced
+// once and the walls of a tile's edge twice (2.1 per cell and stage), for 64
+// bytes more per cell, which cost nothing beside that.  1024^2 open: 1.17 ms a
+// step fused, 0.92 so; 384 x 256: 175 us, 141.  16 x 16 tiles by 256 threads:
+// smaller tiles repeat more walls (16 x 8 and 8 x 8 were 10 and 30 % slower),
+// 128 threads leave a small grid too few warps (384 x 256: 206 us).  With a
+// part or all of the products formed on the integer pipes too, the step was 4
+// to 27 % slower: the double instructions' issue gaps are not free.
+// ---------------------------------------------------------------------------
+struct HydroStage1 {
+  void *q[4];  // stage-1 state, memory-sized arrays
+};
+
+namespace hk {
+// What a block's threads share of the quotients that are the same for all of
+// them (formed by each thread they were a fifth of a step's double operations).
+template <class R> struct alignas(16) StageConsts {
+  hs::Gas<R> gas;
+  R dtdx0, dtdx1;
+  StageConsts() = default;
+  __device__ StageConsts(R g, R dt, R dR0, R dR1)
+      : gas(hs::gas(g)), dtdx0(hs::div(dt, dR0)), dtdx1(hs::div(dt, dR1)) {}
+};
+}  // namespace hk
+
+template <class R, int TX, int TY> struct Stage1Smem {
+  static constexpr int PX = TX + 2, PY = TY + 2;
+  hk::StageConsts<R> c;
+  R P[4][PY][PX];
+  R C[PY][PX];
+  hs::Flux<R> fx[TY * (TX + 1)];
+  hs::Flux<R> fy[(TY + 1) * TX];
+};
+template <class R, int TX, int TY> struct Stage2Smem {
+  static constexpr int QX = TX + 4, QY = TY + 4;
+  hk::StageConsts<R> c;
+  R Q[4][QY][QX];
+  hs::Flux<R> fx[TY * (TX + 1)];
+  hs::Flux<R> fy[(TY + 1) * TX];
+};
+
+// Stage 1 of the cells [-e, n + e) of both axes (e = 2 on an open grid, whose
+// margin cells step from the jet state; else 0); a.nt0 tiles along x of that
+// range.
+template <class R, int TX, int TY, int NT, bool OPEN>
+__global__ void __launch_bounds__(NT)
+hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
+  using S = Stage1Smem<R, TX, TY>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  S &s = *reinterpret_cast<S *>(smem_raw);
+  hk::step_begin();
+  const int tid = threadIdx.x, tile = blockIdx.x;
+  const int t0 = tile % a.nt0, t1 = tile / a.nt0;
+  constexpr int e = OPEN ? 2 : 0;
+  const int X0 = t0 * TX - e, Y0 = t1 * TY - e;
+  const int n0 = a.n0, n1 = a.n1;
+  const R g = hk::Reals<R>::gamma(a);
+  const R dR0 = hk::Reals<R>::dR0(a.sc), dR1 = hk::Reals<R>::dR1(a.sc);
+  if (tid == 0) s.c = hk::StageConsts<R>(g, hk::step_dt<R>(a) / R(2), dR0, dR1);
+  const R *f[4] = {(const R *)a.rho, (const R *)a.v0, (const R *)a.v1, (const R *)a.p};
+  const bool near = n0 >= TX + 2 && n1 >= TY + 2;
+  for (int i = tid; i < S::PY * S::PX; i += NT) {
+    const int py = i / S::PX, px = i - py * S::PX;
+    const int ix = X0 + px - 1, iy = Y0 + py - 1;
+    hs::Prim<R> w;
+    if (OPEN) {
+      if (ix < 0 || iy < 0 || ix >= n0 || iy >= n1) {
+        w = hk::jet_state<R>(g, dR0, dR1, hk::Reals<R>::ext1(a.sc), ix, iy);
+      } else {
+        const size_t gi = (size_t)(iy + a.lm) * a.ms0 + (ix + a.lm);
+        w = hs::Prim<R>{f[0][gi], f[1][gi], f[2][gi], f[3][gi]};
+      }
+    } else {
+      const int gy = near ? hk::wrap_near(iy, n1) : hk::wrap<R>(iy, n1);
+      const int gx = near ? hk::wrap_near(ix, n0) : hk::wrap<R>(ix, n0);
+      const size_t gi = (size_t)gy * n0 + gx;
+      w = hs::Prim<R>{f[0][gi], f[1][gi], f[2][gi], f[3][gi]};
+    }
+    s.P[0][py][px] = w.rho;
+    s.P[1][py][px] = w.v0;
+    s.P[2][py][px] = w.v1;
+    s.P[3][py][px] = w.p;
+    s.C[py][px] = hs::sound(g, w.rho, w.p);
+  }
+  __syncthreads();
+  const hs::Gas<R> k = s.c.gas;
+  auto cell = [&](int py, int px) {
+    return hs::Prim<R>{s.P[0][py][px], s.P[1][py][px], s.P[2][py][px], s.P[3][py][px]};
+  };
+  constexpr int NX = TY * (TX + 1), NY = (TY + 1) * TX;
+  for (int i = tid; i < NX + NY; i += NT) {
+    if (i < NX) {
+      const int sy = i / (TX + 1), sx = i - sy * (TX + 1);
+      s.fx[i] = hs::hllc<0>(k, cell(sy + 1, sx), s.C[sy + 1][sx], cell(sy + 1, sx + 1),
+                            s.C[sy + 1][sx + 1]);
+    } else {
+      const int j = i - NX, sy = j / TX, sx = j - sy * TX;
+      s.fy[j] = hs::hllc<1>(k, cell(sy, sx + 1), s.C[sy][sx + 1], cell(sy + 1, sx + 1),
+                            s.C[sy + 1][sx + 1]);
+    }
+  }
+  __syncthreads();
+  const R dtdx0 = s.c.dtdx0, dtdx1 = s.c.dtdx1;
+  for (int i = tid; i < TY * TX; i += NT) {
+    const int oy = i / TX, ox = i - oy * TX;
+    const int iy = Y0 + oy, ix = X0 + ox;
+    if (iy >= n1 + e || ix >= n0 + e) continue;
+    const hs::Prim<R> q = hs::update(k, cell(oy + 1, ox + 1), dtdx0, dtdx1,
+                                     s.fx[oy * (TX + 1) + ox], s.fx[oy * (TX + 1) + ox + 1],
+                                     s.fy[oy * TX + ox], s.fy[(oy + 1) * TX + ox]);
+    const size_t gi = OPEN ? (size_t)(iy + a.lm) * a.ms0 + (ix + a.lm) : (size_t)iy * n0 + ix;
+    ((R *)o.q[0])[gi] = q.rho;
+    ((R *)o.q[1])[gi] = q.v0;
+    ((R *)o.q[2])[gi] = q.v1;
+    ((R *)o.q[3])[gi] = q.p;
+  }
+}
+
+// Stage 2, the new state and its CFL minimum.
+template <class R, int TX, int TY, int NT, bool OPEN>
+__global__ void __launch_bounds__(NT)
+hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
+  using S = Stage2Smem<R, TX, TY>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned long long red[32];
+  S &s = *reinterpret_cast<S *>(smem_raw);
+  hk::step_begin();
+  const int tid = threadIdx.x, tile = blockIdx.x;
+  const int t0 = tile % a.nt0, t1 = tile / a.nt0;
+  const int X0 = t0 * TX, Y0 = t1 * TY;
+  const int n0 = a.n0, n1 = a.n1, lm = a.lm;
+  const R dR0 = hk::Reals<R>::dR0(a.sc), dR1 = hk::Reals<R>::dR1(a.sc);
+  const R dtG = hk::step_dt<R>(a);
+  if (tid == 0) s.c = hk::StageConsts<R>(hk::Reals<R>::gamma(a), dtG, dR0, dR1);
+  const bool near = n0 >= TX + 4 && n1 >= TY + 4;
+  for (int i = tid; i < S::QY * S::QX; i += NT) {
+    const int qy = i / S::QX, qx = i - qy * S::QX;
+    const int ix = X0 + qx - 2, iy = Y0 + qy - 2;
+    size_t gi;
+    if (OPEN) {  // rows and columns beyond the last margin cell feed no cell
+      gi = (size_t)(min(iy, n1 + 1) + lm) * a.ms0 + (min(ix, n0 + 1) + lm);
+    } else {
+      const int gy = near ? hk::wrap_near(iy, n1) : hk::wrap<R>(iy, n1);
+      const int gx = near ? hk::wrap_near(ix, n0) : hk::wrap<R>(ix, n0);
+      gi = (size_t)gy * n0 + gx;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s.Q[c][qy][qx] = ((const R *)o.q[c])[gi];
+  }
+  __syncthreads();
+  const hs::Gas<R> k = s.c.gas;
+  constexpr int NX = TY * (TX + 1), NY = (TY + 1) * TX;
+  for (int i = tid; i < NX + NY; i += NT) {
+    const bool x = i < NX;
+    const int j = x ? i : i - NX;
+    const int sy = x ? j / (TX + 1) : j / TX, sx = x ? j - sy * (TX + 1) : j - sy * TX;
+    // the wall lies between cells 1 and 2 of four along its axis
+    const int qy = x ? sy + 2 : sy, qx = x ? sx : sx + 2, dy = x ? 0 : 1, dx = x ? 1 : 0;
+    hs::Prim<R> L, Rt;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      hs::muscl(s.Q[c][qy][qx], s.Q[c][qy + dy][qx + dx], s.Q[c][qy + 2 * dy][qx + 2 * dx],
+                s.Q[c][qy + 3 * dy][qx + 3 * dx], (&L.rho)[c], (&Rt.rho)[c]);
+    const R cl = hs::sound(k.g, L.rho, L.p), cr = hs::sound(k.g, Rt.rho, Rt.p);
+    if (x) s.fx[j] = hs::hllc<0>(k, L, cl, Rt, cr);
+    else s.fy[j] = hs::hllc<1>(k, L, cl, Rt, cr);
+  }
+  __syncthreads();
+  unsigned long long m = ~0ull;
+  const R dtdx0 = s.c.dtdx0, dtdx1 = s.c.dtdx1;
+  const R *f[4] = {(const R *)a.rho, (const R *)a.v0, (const R *)a.v1, (const R *)a.p};
+  R *out[4] = {(R *)a.nrho, (R *)a.nv0, (R *)a.nv1, (R *)a.np};
+  for (int i = tid; i < TY * TX; i += NT) {
+    const int oy = i / TX, ox = i - oy * TX;
+    const int gy = Y0 + oy, gx = X0 + ox;
+    if (gy >= n1 || gx >= n0) continue;
+    const size_t gi = OPEN ? (size_t)(gy + lm) * a.ms0 + (gx + lm) : (size_t)gy * n0 + gx;
+    const hs::Prim<R> b{f[0][gi], f[1][gi], f[2][gi], f[3][gi]};
+    const hs::Prim<R> q = hs::update(k, b, dtdx0, dtdx1, s.fx[oy * (TX + 1) + ox],
+                                     s.fx[oy * (TX + 1) + ox + 1], s.fy[oy * TX + ox],
+                                     s.fy[(oy + 1) * TX + ox]);
+    out[0][gi] = q.rho;
+    out[1][gi] = q.v0;
+    out[2][gi] = q.v1;
+    out[3][gi] = q.p;
+    const unsigned long long bits =
+        hk::ts_bits<R>(hs::timescale(k.g, dR0, dR1, q.rho, q.v0, q.v1, q.p));
+    m = bits < m ? bits : m;
+  }
+  if (OPEN) hk::clear_margins<R, TX, TY, NT>(a, X0, Y0, out);
+  hk::block_min_to(m, ts_at(a, a.ts_write), red);
+  hk::step_end<R, OPEN>(a, tile, dtG);
 }
 
 // the fused step that also writes the tape of the reverse sweep (periodic)

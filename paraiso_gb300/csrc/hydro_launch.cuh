@@ -85,7 +85,8 @@ inline int hydro_tile_of(int tile_x, int tile_y, bool production) {
 // fused two-stage step; `exact` selects the no-contraction build
 cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaStream_t s,
                             int *grid_out);
-cudaError_t hydro_fused_f64(const HydroStepArgs &a, int tile, cudaStream_t s, int *grid_out);
+// the FP64 step, its stage-1 state in q
+cudaError_t hydro_step_f64(const HydroStepArgs &a, const HydroStage1 &q, cudaStream_t s);
 // one fused step of a periodic grid that also writes the tape of the
 // reverse sweep (32x16 tiles; the build of the handle's variant)
 cudaError_t hydro_fused_tape(int fp64, bool exact, const HydroStepArgs &a, const HydroTapeOut &t,

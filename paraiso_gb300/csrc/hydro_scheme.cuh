@@ -62,8 +62,8 @@ template <class R> __device__ __forceinline__ Gas<R> gas(R g) {
   Gas<R> k;
   k.g = g;
   k.gm1 = g - R(1);
-  k.gm1inv = R(1) / k.gm1;
-  k.qc = (g + R(1)) / (R(2) * g);
+  k.gm1inv = div(R(1), k.gm1);
+  k.qc = div(g + R(1), R(2) * g);
   return k;
 }
 

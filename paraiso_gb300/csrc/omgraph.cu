@@ -734,6 +734,7 @@ struct StagePlan {
   std::vector<int> reduces;    // reduce node ids
   std::vector<int> manifests;  // manifest node ids computed by this stage
   std::string fn;
+  long long items = 1;  // work items (row chunks or tiles), one a block at a time
 };
 
 struct KernelPlan {
@@ -743,6 +744,12 @@ struct KernelPlan {
   std::vector<int> stored_arrays;  // static indices of arrays written
   std::string commit_fn;
 };
+
+// Every kernel of a machine is launched so that its blocks may be scheduled
+// while the kernel before drains; they wait for its completion first.
+static const char *kBegin =
+    "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
+    "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n";
 
 static const char *kPrelude =
     "struct OMPtrs { const void *cur[32]; void *nxt[32]; void *tmp[64]; };\n"
@@ -1057,7 +1064,7 @@ static std::string generate(const Graph &g, const Layout &L, std::vector<KernelP
       std::ostringstream body;
       src << "extern \"C\" __global__ void __launch_bounds__(256)\n" << sp.fn
           << "(OMPtrs P, const unsigned char *SC, unsigned char *slots, unsigned char *part,\n"
-          << "     unsigned int *done) {\n";
+          << "     unsigned int *done) {\n" << kBegin;
       for (size_t r = 0; r < sp.reduces.size(); ++r) {
         const Node &n = k.node(sp.reduces[r]);
         src << "  " << ctype(n.type) << " acc" << r << " = " << ident(n.type, n.sarg) << ";\n";
@@ -1103,11 +1110,14 @@ static std::string generate(const Graph &g, const Layout &L, std::vector<KernelP
       const bool tiled = V == 1 && shared && !L.open && g.ndim == 2 &&
                          plan_tiles(g, k, L, slots, man, st, sp, &tiles, &shape);
       if (tiled) {
+        sp.items = (long long)((L.ms[0] + shape.tx - 1) / shape.tx) *
+                   ((L.ms[1] + shape.ty - 1) / shape.ty);
         emit_tiled(src, g, k, L, slots, man, st, sp, tiles, shape, em);
       } else {
         // work items: chunks of 256 V cells of a memory row, rows in order; a
         // block takes items blockIdx.x, blockIdx.x + gridDim.x, ...
         const int chunk = 256 * V;
+        sp.items = (long long)L.ms[1] * ((L.ms[0] + chunk - 1) / chunk);
         src << "  constexpr int CX = " << (L.ms[0] + chunk - 1) / chunk << ";\n"
             << "  const long long NW = (long long)" << L.ms[1] << " * CX;\n"
             << "  for (long long w = blockIdx.x; w < NW; w += gridDim.x) {\n"
@@ -1235,7 +1245,7 @@ static std::string generate(const Graph &g, const Layout &L, std::vector<KernelP
     kp.commit_fn = "om_k" + std::to_string(ki) + "_commit";
     {
       src << "extern \"C\" __global__ void " << kp.commit_fn
-          << "(OMPtrs P, unsigned char *SC, unsigned char *slots) {\n"
+          << "(OMPtrs P, unsigned char *SC, unsigned char *slots) {\n" << kBegin
           << "  if (threadIdx.x != 0 || blockIdx.x != 0) return;\n"
           << "  const int c0 = 0, c1 = 0; (void)c0; (void)c1; (void)P;\n";
       Emitter e(g, k, L, slots);
@@ -1278,7 +1288,7 @@ struct GraphState {
   unsigned char *part = nullptr;   // per reduce of a stage: 8 bytes per block
   unsigned int *done = nullptr;    // one counter per (kernel, stage)
   std::vector<std::vector<int>> done_index;
-  int grid = 1;
+  std::vector<std::vector<int>> stage_grid;  // blocks per (kernel, stage)
   std::string source;
   bool owned = false;  // freed with the handle once setup has started
 };
@@ -1303,6 +1313,20 @@ struct OMPtrs {
   void *tmp[kMaxManifests];
 };
 
+static cudaError_t launch_dependent(const void *kernel, int grid, int threads, void **args,
+                                    cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
 static om_status graph_run(Handle *h, int n) {
   GraphState *st = gst(h);
   const int ki = h->current_kernel;
@@ -1319,14 +1343,13 @@ static om_status graph_run(Handle *h, int n) {
     for (size_t s = 0; s < kp.stages.size(); ++s) {
       unsigned int *done = st->done + st->done_index[ki][s];
       void *args[] = {&P, &SC, &st->slots, &st->part, &done};
-      OM_CUDA_CHECK(cudaLaunchKernel((const void *)st->stage_k[ki][s], dim3(st->grid), dim3(256),
-                                     args, 0, h->stream));
+      OM_CUDA_CHECK(launch_dependent((const void *)st->stage_k[ki][s], st->stage_grid[ki][s], 256,
+                                     args, h->stream));
       h->launches++;
     }
     if (!kp.scalar_stores.empty()) {
       void *args[] = {&P, &SC, &st->slots};
-      OM_CUDA_CHECK(cudaLaunchKernel((const void *)st->commit_k[ki], dim3(1), dim3(32), args, 0,
-                                     h->stream));
+      OM_CUDA_CHECK(launch_dependent((const void *)st->commit_k[ki], 1, 32, args, h->stream));
       h->launches++;
     }
     for (int s : kp.stored_arrays) {
@@ -1468,14 +1491,28 @@ static om_status graph_setup(Handle *h, void *ctx) {
   h->scalar_bytes = scalar_end;
   for (const KernelDef &k : g.kernels) h->kernels.push_back({k.name, graph_run});
   const long long cells = (long long)L.ms[0] * L.ms[1];
-  st->grid = (int)std::max<long long>(
-      1, std::min<long long>((cells + 255) / 256, 8LL * sm_count(h->device)));
-  int maxred = 1, nstages = 0;
+  // blocks of a stage: eight per SM walk the items, or one block an item where
+  // that is at most 32 per SM, so that the hardware evens out their times (the
+  // walls of a 1024^2 Hydro graph are 4096 tiles: 1216 blocks took three or four
+  // each).  Sums of floating values keep the first form at every size: their
+  // rounding follows the blocks.
+  const long long sms = sm_count(h->device);
+  const int walk = (int)std::max<long long>(1, std::min<long long>((cells + 255) / 256, 8 * sms));
+  auto ordered = [](const KernelDef &k, const StagePlan &sp) {
+    for (int id : sp.reduces)
+      if (k.node(id).sarg == "sum" && k.node(id).type != TInt) return true;
+    return false;
+  };
+  int maxred = 1, nstages = 0, maxgrid = walk;
   st->done_index.resize(st->plans.size());
+  st->stage_grid.resize(st->plans.size());
   for (size_t k = 0; k < st->plans.size(); ++k)
     for (const StagePlan &sp : st->plans[k].stages) {
       maxred = std::max(maxred, (int)sp.reduces.size());
       st->done_index[k].push_back(nstages++);
+      const bool each = sp.items <= 32 * sms && !ordered(g.kernels[k], sp);
+      st->stage_grid[k].push_back(each ? (int)std::max<long long>(1, sp.items) : walk);
+      maxgrid = std::max(maxgrid, st->stage_grid[k].back());
     }
   for (Type t : st->tmp_types) {
     void *p = nullptr;
@@ -1488,7 +1525,7 @@ static om_status graph_setup(Handle *h, void *ctx) {
     st->tmp.push_back(p);
   }
   if (cudaMalloc(&st->slots, 8 * (size_t)std::max(nslots, 1)) != cudaSuccess ||
-      cudaMalloc(&st->part, 8 * (size_t)maxred * st->grid) != cudaSuccess ||
+      cudaMalloc(&st->part, 8 * (size_t)maxred * maxgrid) != cudaSuccess ||
       cudaMalloc(&st->done, sizeof(unsigned int) * std::max(nstages, 1)) != cudaSuccess ||
       cudaMemset(st->done, 0, sizeof(unsigned int) * std::max(nstages, 1)) != cudaSuccess ||
       cudaMemset(st->slots, 0, 8 * (size_t)std::max(nslots, 1)) != cudaSuccess) {

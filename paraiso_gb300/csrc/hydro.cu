@@ -146,10 +146,13 @@ static om_status proceed_fused(Handle *h, int n) {
                         : st->tile;
   const bool persist = !st->fp64 && st->variant != 2 && st->lm == 0 &&
                        hydro_tile_is_persistent(stile) &&
-                       hydro_persist_fits(h->size[0], h->size[1]);
+                       (hydro_persist_fits(h->size[0], h->size[1]) ||
+                        (hydro_tile_takes_any(stile) &&
+                         hydro_persist_any(h->size[0], h->size[1])));
   // the persistent kernel's form that runs (the profile name follows it)
   const int form = persist ? hydro_persist_form_for(hydro_persist_form(stile),
-                                                    (long long)(h->size[0] / 32) * (h->size[1] / 32),
+                                                    (long long)((h->size[0] + 31) / 32) *
+                                                        ((h->size[1] + 31) / 32),
                                                     h->device, h->cfg.grid_limit)
                            : -1;
   const char *kname = st->fp64 ? "hydro_stage_kernels_f64"

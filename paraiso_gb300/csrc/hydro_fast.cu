@@ -89,10 +89,12 @@ template <int TX, int TY, int NT> static int occ_fast() {
 }
 
 cudaError_t hydro_ensemble_f32(const HydroStepArgs *args, const int *prefix, int count, int tile,
-                               bool exact, int grid, cudaStream_t s, const CUtensorMap *table) {
+                               bool exact, int grid, cudaStream_t s, const CUtensorMap *table,
+                               bool general) {
   if (exact) return hydro_ensemble_f32_exact(args, prefix, count, grid, s);
   if (hydro_tile_is_persistent(tile) && table)
-    return hydro_persist_ensemble(args, prefix, count, table, hydro_persist_form(tile), grid, s);
+    return hydro_persist_ensemble(args, prefix, count, table, hydro_persist_form(tile), general,
+                                  grid, s);
   switch (tile) {
     case kTile32x8: return launch_ens<32, 8, 256>(args, prefix, count, grid, s);
     case kTile64x16: return launch_ens<64, 16, 512>(args, prefix, count, grid, s);
@@ -177,8 +179,9 @@ int hydro_step_tile(int tile, int n0, int n1, bool open, int device, int grid_li
   if (!open && tiles(16, 8) <= sms) return kThin16x8;
   if (tiles(32, 16) <= sms) return kThin32x16;
   if (tiles(32, 16) <= 2 * sms) return kThin32x16h;
-  if (!open && !hydro_persist_fits(n0, n1) && tiles(32, 16) <= 6 * sms) return kThin32x16h;
-  return tile;
+  if (open || hydro_persist_fits(n0, n1)) return tile;
+  if (tiles(32, 16) <= 6 * sms) return kThin32x16h;
+  return hydro_persist_partial(n0, n1, device) ? tile : kTile32x32;
 }
 
 cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaStream_t s,
@@ -197,7 +200,8 @@ cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaSt
     case kPersist32x32:
     case kPair32x32:
     case kPairGroups32x32:
-      if (hydro_persist_fits(a.n0, a.n1))
+      if (hydro_persist_fits(a.n0, a.n1) ||
+          (hydro_tile_takes_any(tile) && hydro_persist_any(a.n0, a.n1)))
         return hydro_persist_step(a, hydro_persist_form(tile), s, grid_out);
       return launch_fast<32, 32, 512>(a, s, grid_out);
     case kTile32x8: return launch_fast<32, 8, 256>(a, s, grid_out);

@@ -199,15 +199,15 @@ template <class R> __device__ __forceinline__ R step_dt(const HydroStepArgs &a) 
 // The margin cells of an open grid beside the tile at (X0, Y0) are set to 0:
 // the generated class copies whole manifests, whose margins are zero, into the
 // statics.
-template <class R, int TX, int TY, int NT>
+template <class R, int TX, int TY>
 __device__ __forceinline__ void clear_margins(const HydroStepArgs &a, int X0, int Y0,
-                                              R *const (&out)[4]) {
+                                              R *const (&out)[4], int tid, int threads) {
   const int n0 = a.n0, n1 = a.n1, lm = a.lm;
   const int xa = X0 == 0 ? -lm : X0, xb = X0 + TX >= n0 ? n0 + lm : X0 + TX;
   const int ya = Y0 == 0 ? -lm : Y0, yb = Y0 + TY >= n1 ? n1 + lm : Y0 + TY;
   if (xa >= 0 && ya >= 0 && xb <= n0 && yb <= n1) return;
   const int w = xb - xa, cnt = w * (yb - ya);
-  for (int i = threadIdx.x; i < cnt; i += NT) {
+  for (int i = tid; i < cnt; i += threads) {
     const int y = ya + i / w, x = xa + i % w;
     if (x >= 0 && y >= 0 && x < n0 && y < n1) continue;
     const size_t gi = (size_t)(y + lm) * a.ms0 + (x + lm);
@@ -494,7 +494,7 @@ __device__ __forceinline__ void fused_tile(const HydroStepArgs &a, int tile,
   }
   if (OPEN) {
     R *out[4] = {(R *)a.nrho, (R *)a.nv0, (R *)a.nv1, (R *)a.np};
-    hk::clear_margins<R, TX, TY, NT>(a, X0, Y0, out);
+    hk::clear_margins<R, TX, TY>(a, X0, Y0, out, tid, NT);
   }
   hk::block_min_to(m, ts_at(a, a.ts_write), red);
   hk::step_end<R, OPEN>(a, tile, dtG);
@@ -703,7 +703,7 @@ hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
         hk::ts_bits<R>(hs::timescale(k.g, dR0, dR1, q.rho, q.v0, q.v1, q.p));
     m = bits < m ? bits : m;
   }
-  if (OPEN) hk::clear_margins<R, TX, TY, NT>(a, X0, Y0, out);
+  if (OPEN) hk::clear_margins<R, TX, TY>(a, X0, Y0, out, tid, NT);
   hk::block_min_to(m, ts_at(a, a.ts_write), red);
   hk::step_end<R, OPEN>(a, tile, dtG);
 }

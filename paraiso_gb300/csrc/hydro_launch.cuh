@@ -98,11 +98,18 @@ cudaError_t hydro_fused_tape(int fp64, bool exact, const HydroStepArgs &a, const
 // the instance's args) and fall back to the 32 x 32 tile kernel without one.
 cudaError_t hydro_ensemble_f32(const HydroStepArgs *args, const int *prefix, int count, int tile,
                                bool exact, int grid, cudaStream_t s,
-                               const CUtensorMap *table = nullptr);
+                               const CUtensorMap *table = nullptr, bool general = false);
 
 // the persistent 32 x 32 production step (hydro_persist.cu): grids whose
 // sides are multiples of 32 and at least 64 (periodic)
 bool hydro_persist_fits(int n0, int n1);
+// and, in its paired forms, sides of any size from 64 with rows of a multiple
+// of 4 cells (partial tiles); `partial` also says whether it is worth it
+bool hydro_persist_any(int n0, int n1);
+bool hydro_persist_partial(int n0, int n1, int device);
+inline bool hydro_tile_takes_any(int tile) {
+  return tile == kPair32x32 || tile == kPairGroups32x32;
+}
 // the four field tensor maps of a's current state
 bool hydro_persist_encode(CUtensorMap *maps4, const HydroStepArgs &a);
 // the form that runs for `tiles` tiles: two groups per CTA only when every
@@ -116,7 +123,7 @@ cudaError_t hydro_persist_step(const HydroStepArgs &a, int form, cudaStream_t s,
 cudaError_t hydro_persist_tape(const HydroStepArgs &a, int form, const HydroTapeOut &t,
                                cudaStream_t s);
 cudaError_t hydro_persist_ensemble(const HydroStepArgs *args, const int *prefix, int count,
-                                   const CUtensorMap *table, int form, int grid,
+                                   const CUtensorMap *table, int form, bool general, int grid,
                                    cudaStream_t s);
 cudaError_t hydro_ensemble_f64(const HydroStepArgs *args, const int *prefix, int count, int tile,
                                int grid, cudaStream_t s);

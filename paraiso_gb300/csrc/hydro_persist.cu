@@ -27,6 +27,21 @@ bool hydro_persist_fits(int n0, int n1) {
   return n0 % hp::TX == 0 && n1 % hp::TY == 0 && n0 >= 2 * hp::TX && n1 >= 2 * hp::TY;
 }
 
+// The partial tiles of such a grid cost it a few per cent: 1000 x 700 (704
+// tiles) takes 30.9 us a step against 28.4 with the tile kernel, 1500 x 1100
+// (1645) 57.8 against 59.3, 3000 x 2500 244.7 against 257.1, 4000^2 488 against
+// 529.  Rows that TMA cannot take, and open grids, were slower copied cell by
+// cell than with the tile kernel at every size (3001 x 2500: 265.6 against
+// 257.5; open 4000^2: 552 against 541).
+bool hydro_persist_partial(int n0, int n1, int device) {
+  const long long tiles =
+      (long long)((n0 + hp::TX - 1) / hp::TX) * ((n1 + hp::TY - 1) / hp::TY);
+  return hydro_persist_any(n0, n1) && tiles >= 8LL * sm_count(device);
+}
+bool hydro_persist_any(int n0, int n1) {
+  return n0 % 4 == 0 && n0 >= 2 * hp::TX && n1 >= 2 * hp::TY;
+}
+
 // one field of an n0 x n1 FP32 grid as a 2-D tensor of 40 x 38 boxes
 static bool encode_field(CUtensorMap *m, const void *base, int n0, int n1) {
   const uint64_t dims[2] = {(uint64_t)n0, (uint64_t)n1};
@@ -62,18 +77,19 @@ int hydro_persist_occupancy(int form) {
   static int n[3] = {-1, -1, -1};
   int &v = n[form];
   if (v < 0)
-    v = form == 2 ? resident_per_sm(hp::hydro_pair2_ensemble_kernel, 2 * hp::NT2, 2)
-        : form == 1 ? resident_per_sm(hp::hydro_persist_ensemble_kernel<true>, hp::NT2)
-                    : resident_per_sm(hp::hydro_persist_ensemble_kernel<false>, hp::NT);
+    v = form == 2 ? resident_per_sm(hp::hydro_pair2_ensemble_kernel<false>, 2 * hp::NT2, 2)
+        : form == 1 ? resident_per_sm(hp::hydro_persist_ensemble_kernel<true, false>, hp::NT2)
+                    : resident_per_sm(hp::hydro_persist_ensemble_kernel<false, false>, hp::NT);
   return v > 0 ? v : 1;
 }
 
-// FORM 0: one wall or cell per thread; 1: paired; 2: paired, two groups per CTA
-template <bool TAPE, int FORM>
+// FORM 0: one wall or cell per thread (GEN false); 1: paired; 2: paired, two
+// groups per CTA
+template <bool TAPE, int FORM, bool GEN>
 static cudaError_t persist_launch(const HydroStepArgs &a0, const HydroTapeOut *tape,
                                   cudaStream_t s, int *grid_out) {
-  auto kernel = FORM == 2 ? hp::hydro_pair2_kernel<TAPE>
-                : FORM == 1 ? hp::hydro_pair_kernel<TAPE> : hp::hydro_persist_kernel<TAPE>;
+  auto kernel = FORM == 2 ? hp::hydro_pair2_kernel<TAPE, GEN>
+                : FORM == 1 ? hp::hydro_pair_kernel<TAPE, GEN> : hp::hydro_persist_kernel<TAPE>;
   const int groups = FORM == 2 ? 2 : 1;
   const int threads = (FORM == 0 ? hp::NT : hp::NT2) * groups;
   const size_t smem = sizeof(hp::Smem) * groups;
@@ -81,12 +97,12 @@ static cudaError_t persist_launch(const HydroStepArgs &a0, const HydroTapeOut *t
   if (occ < 0) occ = resident_per_sm(kernel, threads, groups);
   if (occ <= 0) return cudaErrorInvalidConfiguration;
   HydroStepArgs a = a0;
-  a.nt0 = a.n0 / hp::TX;
+  a.nt0 = (a.n0 + hp::TX - 1) / hp::TX;
   CUtensorMap m[4];
   if (!hydro_persist_encode(m, a)) return cudaErrorInvalidValue;
   int dev = 0;
   cudaGetDevice(&dev);
-  const int tiles = a.nt0 * (a.n1 / hp::TY);
+  const int tiles = a.nt0 * ((a.n1 + hp::TY - 1) / hp::TY);
   // every group of a CTA takes at least one tile
   int grid = std::min((tiles + groups - 1) / groups, occ * sm_count(dev));
   if (a.grid_limit > 0) grid = std::min(grid, a.grid_limit);
@@ -98,41 +114,52 @@ static cudaError_t persist_launch(const HydroStepArgs &a0, const HydroTapeOut *t
   return cudaGetLastError();
 }
 
-cudaError_t hydro_persist_step(const HydroStepArgs &a, int form, cudaStream_t s, int *grid_out) {
+static int form_for(const HydroStepArgs &a, int form) {
   int dev = 0;
   cudaGetDevice(&dev);
-  form = hydro_persist_form_for(form, (long long)(a.n0 / hp::TX) * (a.n1 / hp::TY), dev,
-                                a.grid_limit);
-  return form == 2 ? persist_launch<false, 2>(a, nullptr, s, grid_out)
-         : form == 1 ? persist_launch<false, 1>(a, nullptr, s, grid_out)
-                     : persist_launch<false, 0>(a, nullptr, s, grid_out);
+  const long long tiles =
+      (long long)((a.n0 + hp::TX - 1) / hp::TX) * ((a.n1 + hp::TY - 1) / hp::TY);
+  return hydro_persist_form_for(form, tiles, dev, a.grid_limit);
+}
+
+cudaError_t hydro_persist_step(const HydroStepArgs &a, int form, cudaStream_t s, int *grid_out) {
+  form = form_for(a, form);
+  if (!hydro_persist_fits(a.n0, a.n1))
+    return form == 2 ? persist_launch<false, 2, true>(a, nullptr, s, grid_out)
+                     : persist_launch<false, 1, true>(a, nullptr, s, grid_out);
+  return form == 2 ? persist_launch<false, 2, false>(a, nullptr, s, grid_out)
+         : form == 1 ? persist_launch<false, 1, false>(a, nullptr, s, grid_out)
+                     : persist_launch<false, 0, false>(a, nullptr, s, grid_out);
 }
 
 cudaError_t hydro_persist_tape(const HydroStepArgs &a, int form, const HydroTapeOut &t,
                                cudaStream_t s) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  form = hydro_persist_form_for(form, (long long)(a.n0 / hp::TX) * (a.n1 / hp::TY), dev,
-                                a.grid_limit);
-  return form == 2 ? persist_launch<true, 2>(a, &t, s, nullptr)
-         : form == 1 ? persist_launch<true, 1>(a, &t, s, nullptr)
-                     : persist_launch<true, 0>(a, &t, s, nullptr);
+  form = form_for(a, form);
+  return form == 2 ? persist_launch<true, 2, false>(a, &t, s, nullptr)
+         : form == 1 ? persist_launch<true, 1, false>(a, &t, s, nullptr)
+                     : persist_launch<true, 0, false>(a, &t, s, nullptr);
+}
+
+template <bool GEN>
+static cudaError_t ensemble_launch(const HydroStepArgs *args, const int *prefix, int count,
+                                   const CUtensorMap *table, int form, int grid, cudaStream_t s) {
+  const int groups = form == 2 ? 2 : 1;
+  const int threads = (form == 0 ? hp::NT : hp::NT2) * groups;
+  auto kernel = form == 2   ? hp::hydro_pair2_ensemble_kernel<GEN>
+                : form == 1 ? hp::hydro_persist_ensemble_kernel<true, GEN>
+                            : hp::hydro_persist_ensemble_kernel<false, false>;
+  static int occ[3] = {-1, -1, -1};
+  if (occ[form] < 0) occ[form] = resident_per_sm(kernel, threads, groups);
+  if (occ[form] < 1) return cudaErrorInvalidConfiguration;
+  kernel<<<grid, threads, groups * sizeof(hp::Smem), s>>>(args, prefix, count, table);
+  return cudaGetLastError();
 }
 
 cudaError_t hydro_persist_ensemble(const HydroStepArgs *args, const int *prefix, int count,
-                                   const CUtensorMap *table, int form, int grid,
+                                   const CUtensorMap *table, int form, bool general, int grid,
                                    cudaStream_t s) {
-  if (hydro_persist_occupancy(form) < 1) return cudaErrorInvalidConfiguration;
-  if (form == 2)
-    hp::hydro_pair2_ensemble_kernel<<<grid, 2 * hp::NT2, 2 * sizeof(hp::Smem), s>>>(
-        args, prefix, count, table);
-  else if (form == 1)
-    hp::hydro_persist_ensemble_kernel<true><<<grid, hp::NT2, sizeof(hp::Smem), s>>>(
-        args, prefix, count, table);
-  else
-    hp::hydro_persist_ensemble_kernel<false><<<grid, hp::NT, sizeof(hp::Smem), s>>>(
-        args, prefix, count, table);
-  return cudaGetLastError();
+  return general ? ensemble_launch<true>(args, prefix, count, table, form, grid, s)
+                 : ensemble_launch<false>(args, prefix, count, table, form, grid, s);
 }
 
 }  // namespace om

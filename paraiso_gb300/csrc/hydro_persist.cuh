@@ -123,8 +123,8 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 // Start the copy of a tile's box into `dst`.  Inside the grid: thread 0
 // posts the byte count on *bar and issues the four TMA boxes (maps[k]
 // describes field k of this grid).  Else every thread copies 16-byte
-// chunks with wrapped coordinates (grid sizes are multiples of 32, so a
-// wrapped chunk stays 16-byte aligned).
+// chunks with wrapped coordinates (rows are multiples of 4 cells, so a
+// wrapped chunk stays 16-byte aligned and whole).
 // The four fields of a grid: their tensor maps (m, for boxes inside the
 // grid) and base pointers (f).
 struct FieldRefs {
@@ -343,7 +343,9 @@ __device__ __forceinline__ void wall_run2(const float4 *q, int xb, int yb, Flux 
 // alternate items; group 1 starts once group 0 has passed the second phase
 // of its first tile, so the two groups' phases run about half a tile apart
 // and one group's barrier tails overlap the other's arithmetic.
-template <bool TAPE, bool ENS, bool PAIR, int GROUPS = 1>
+// GEN: sides of any size from 64 cells whose rows are whole 16-byte chunks
+// (partial tiles); else sides are multiples of 32.
+template <bool TAPE, bool ENS, bool PAIR, int GROUPS = 1, bool GEN = false>
 __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ args,
                                             const int *__restrict__ pf, int count,
                                             const CUtensorMap *table, const CUtensorMap *m0,
@@ -426,12 +428,12 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
         s.cq.c[i] = hf::sound(Kx, Bx[i], Bx[3 * PLANE + i]);
     }
   };
-  // wait until the box of tile (X0, Y0) of an n0 x n1 grid has landed in
+  // wait until the box of tile (X0, Y0) of a grid has landed in
   // buffer bb (the caller synchronises the block afterwards)
   uint32_t parity = 0;  // bit k: parity of the next completed phase of bar[k]
-  auto await_box = [&](int bb, int X0, int Y0, int n0, int n1, uint32_t *err) {
-    if (box_inside(X0, Y0, n0, n1)) {
-      tma::mbar_wait(&s.bar[bb], (parity >> bb) & 1u, err);
+  auto await_box = [&](int bb, int X0, int Y0, const HydroStepArgs &A) {
+    if (box_inside(X0, Y0, A.n0, A.n1)) {
+      tma::mbar_wait(&s.bar[bb], (parity >> bb) & 1u, &A.sc->wait_error);
       parity ^= 1u << bb;
     } else {
       hk::cp_async_wait_all();
@@ -453,7 +455,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
   {
     int X0, Y0;
     tile_origin(item, lo, X0, Y0);
-    await_box(0, X0, Y0, args[lo].n0, args[lo].n1, &args[lo].sc->wait_error);
+    await_box(0, X0, Y0, args[lo]);
     sync();
     sounds(s.box[0], hf::consts<float>(args[lo].gamma_f), tid, NTH);
   }
@@ -598,7 +600,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     if (next < total) {
       int Xn, Yn;
       tile_origin(next, lo_n, Xn, Yn);
-      await_box(b ^ 1, Xn, Yn, args[lo_n].n0, args[lo_n].n1, &args[lo_n].sc->wait_error);
+      await_box(b ^ 1, Xn, Yn, args[lo_n]);
     }
     sync();
 
@@ -613,6 +615,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
       float *out[4] = {(float *)A.nrho, (float *)A.nv0, (float *)A.nv1, (float *)A.np};
       auto put = [&](int oy, int ox, const float *q, const float *cons, const Flux &l0,
                      const Flux &r0, const Flux &l1, const Flux &r1) {
+        if (GEN && (X0 + ox >= n0 || Y0 + oy >= A.n1)) return;
         const size_t gi = (size_t)(Y0 + oy) * n0 + (X0 + ox);
         if (TAPE) {
           hk::tape_diffs<float>(tape->d2, gi, l0, r0, l1, r1);
@@ -702,50 +705,51 @@ hydro_persist_kernel(HydroStepArgs a, const __grid_constant__ CUtensorMap m0,
                                   reinterpret_cast<Smem *>(smem_raw), &tape);
 }
 
-template <bool TAPE>
+template <bool TAPE, bool GEN>
 __global__ void __launch_bounds__(NT2, 2)
 hydro_pair_kernel(HydroStepArgs a, const __grid_constant__ CUtensorMap m0,
                   const __grid_constant__ CUtensorMap m1, const __grid_constant__ CUtensorMap m2,
                   const __grid_constant__ CUtensorMap m3, HydroTapeOut tape) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   hk::step_begin();
-  persist_run<TAPE, false, true>(&a, nullptr, 1, nullptr, &m0, &m1, &m2, &m3,
-                                 reinterpret_cast<Smem *>(smem_raw), &tape);
+  persist_run<TAPE, false, true, 1, GEN>(&a, nullptr, 1, nullptr, &m0, &m1, &m2, &m3,
+                                         reinterpret_cast<Smem *>(smem_raw), &tape);
 }
 
 // the paired form as one CTA per SM of two groups half a tile apart (two
 // shared-memory blocks); 80 registers keep the 22 warps within the SM
 // sub-partitions' register files
-template <bool TAPE>
+template <bool TAPE, bool GEN>
 __global__ void __maxnreg__(80)
 hydro_pair2_kernel(HydroStepArgs a, const __grid_constant__ CUtensorMap m0,
                    const __grid_constant__ CUtensorMap m1, const __grid_constant__ CUtensorMap m2,
                    const __grid_constant__ CUtensorMap m3, HydroTapeOut tape) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   hk::step_begin();
-  persist_run<TAPE, false, true, 2>(&a, nullptr, 1, nullptr, &m0, &m1, &m2, &m3,
-                                    reinterpret_cast<Smem *>(smem_raw), &tape);
+  persist_run<TAPE, false, true, 2, GEN>(&a, nullptr, 1, nullptr, &m0, &m1, &m2, &m3,
+                                         reinterpret_cast<Smem *>(smem_raw), &tape);
 }
 
 // the paired ensemble step as one CTA per SM of two groups half an item apart
+template <bool GEN>
 __global__ void __maxnreg__(80)
 hydro_pair2_ensemble_kernel(const HydroStepArgs *__restrict__ args,
                             const int *__restrict__ prefix, int count,
                             const CUtensorMap *__restrict__ table) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  persist_run<false, true, true, 2>(args, prefix, count, table, nullptr, nullptr, nullptr, nullptr,
-                                    reinterpret_cast<Smem *>(smem_raw), nullptr);
+  persist_run<false, true, true, 2, GEN>(args, prefix, count, table, nullptr, nullptr, nullptr,
+                                         nullptr, reinterpret_cast<Smem *>(smem_raw), nullptr);
 }
 
 // table: 4 tensor maps per instance for the buffers `args` reads
-template <bool PAIR>
+template <bool PAIR, bool GEN>
 __global__ void __launch_bounds__(PAIR ? NT2 : NT, 2)
 hydro_persist_ensemble_kernel(const HydroStepArgs *__restrict__ args,
                               const int *__restrict__ prefix, int count,
                               const CUtensorMap *__restrict__ table) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  persist_run<false, true, PAIR>(args, prefix, count, table, nullptr, nullptr, nullptr, nullptr,
-                                 reinterpret_cast<Smem *>(smem_raw), nullptr);
+  persist_run<false, true, PAIR, 1, GEN>(args, prefix, count, table, nullptr, nullptr, nullptr,
+                                         nullptr, reinterpret_cast<Smem *>(smem_raw), nullptr);
 }
 
 }  // namespace hp

@@ -91,7 +91,7 @@ struct alignas(128) Smem {
   } fl;
   uint64_t bar[2];
   uint64_t go;  // two groups per CTA: group 0 releases group 1 (in group 0's block)
-  unsigned long long red[32];
+  unsigned red[32];
   // ensembles: the arguments of the current and the next item's instance
   // (read from shared memory rather than held in registers across phases)
   HydroStepArgs args[2];
@@ -361,20 +361,13 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     else asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(NTH) : "memory");
   };
   // block-wide (group-wide) min of CFL bit patterns folded into *dst
-  auto min_to = [&](unsigned long long v, unsigned long long *dst) {
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-      v = w < v ? w : v;
-    }
+  auto min_to = [&](unsigned v, unsigned long long *dst) {
+    v = __reduce_min_sync(0xffffffffu, v);
     if (lane == 0) s.red[warp] = v;
     sync();
     if (warp == 0) {
-      v = lane < NTH / 32 ? s.red[lane] : ~0ull;
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w < v ? w : v;
-      }
-      if (lane == 0) atomicMin(dst, v);
+      v = __reduce_min_sync(0xffffffffu, lane < NTH / 32 ? s.red[lane] : ~0u);
+      if (lane == 0) atomicMin(dst, (unsigned long long)v);
     }
   };
   const int total =
@@ -461,7 +454,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
   }
   sync();
   int b = 0;
-  unsigned long long m = ~0ull;
+  unsigned m = ~0u;
 
   for (;;) {
     const HydroStepArgs &A = ENS ? s.args[b] : args[lo];
@@ -625,8 +618,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
 #pragma unroll
         for (int f = 0; f < 4; ++f) out[f][gi] = q[f];
         const float t = hs::timescale(g, dR0, dR1, q[0], q[1], q[2], q[3]);
-        const unsigned long long bits = hk::ts_bits<float>(t);
-        m = bits < m ? bits : m;
+        m = min(m, __float_as_uint(t));
       };
       if (PAIR) {
         const hf::K<f2> k2 = hf::kconsts<f2>(K);
@@ -682,7 +674,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     // reduction ends with a barrier); else one barrier before the next tile
     if (next >= total || lo_n != lo) {
       min_to(m, ts_at(A, A.ts_write));
-      m = ~0ull;
+      m = ~0u;
     } else {
       sync();
     }

@@ -324,6 +324,13 @@ __device__ __forceinline__ float sqrt_(float a) {
   return d;
 }
 
+// the larger; the other one where one is not a number
+__device__ __forceinline__ float max_(float a, float b) {
+  float d;
+  asm("max.ftz.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+
 __device__ __forceinline__ f2 add(f2 a, f2 b) {
   f2 d;
   asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
@@ -355,13 +362,19 @@ __device__ __forceinline__ f2 sqrt_(f2 a) {
   return pack(sqrt_(x), sqrt_(y));
 }
 
+__device__ __forceinline__ f2 max_(f2 a, f2 b) {
+  float a0, a1, b0, b1;
+  unpack(a, a0, a1);
+  unpack(b, b0, b1);
+  return pack(max_(a0, b0), max_(a1, b1));
+}
+
 // comparisons, selections and predicate logic
 __device__ __forceinline__ bool lt(float a, float b) { return a < b; }
 __device__ __forceinline__ bool le(float a, float b) { return a <= b; }
 __device__ __forceinline__ float sel(bool m, float a, float b) { return m ? a : b; }
 __device__ __forceinline__ bool mor(bool a, bool b) { return a || b; }
-__device__ __forceinline__ bool mnot(bool a) { return !a; }
-__device__ __forceinline__ bool msel(bool c, bool a, bool b) { return c ? a : b; }
+__device__ __forceinline__ bool mxor(bool a, bool b) { return a != b; }
 
 __device__ __forceinline__ m2 lt(f2 a, f2 b) {
   float a0, a1, b0, b1;
@@ -382,10 +395,7 @@ __device__ __forceinline__ f2 sel(m2 m, f2 a, f2 b) {
   return pack(m.x ? a0 : b0, m.y ? a1 : b1);
 }
 __device__ __forceinline__ m2 mor(m2 a, m2 b) { return m2{a.x || b.x, a.y || b.y}; }
-__device__ __forceinline__ m2 mnot(m2 a) { return m2{!a.x, !a.y}; }
-__device__ __forceinline__ m2 msel(m2 c, m2 a, m2 b) {
-  return m2{c.x ? a.x : b.x, c.y ? a.y : b.y};
-}
+__device__ __forceinline__ m2 mxor(m2 a, m2 b) { return m2{a.x != b.x, a.y != b.y}; }
 
 template <class T> __device__ __forceinline__ T splat(float c);
 template <> __device__ __forceinline__ float splat<float>(float c) { return c; }
@@ -424,12 +434,13 @@ template <class T> struct NF {
 };
 
 // minmod of two differences (hs::absmaller's value: the one of smaller
-// magnitude when both have the same sign, else zero) in four bit and
-// min/max operations: sign(a) max(0, min(|a|, sign(a) b))
+// magnitude when both have the same sign, else zero) in three operations: the
+// smaller magnitude under the product of the signs, not below zero, under a's
+// sign
 __device__ __forceinline__ float minmod(float a, float b) {
-  const unsigned sa = __float_as_uint(a) & 0x80000000u;
-  const float m = fmaxf(0.0f, fminf(fabsf(a), __uint_as_float(__float_as_uint(b) ^ sa)));
-  return __uint_as_float(__float_as_uint(m) | sa);
+  float m;
+  asm("min.ftz.xorsign.abs.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return __uint_as_float(__float_as_uint(max_(m, 0.0f)) | (__float_as_uint(a) & 0x80000000u));
 }
 __device__ __forceinline__ f2 minmod(f2 a, f2 b) {
   float a0, a1, b0, b1;
@@ -457,7 +468,7 @@ __device__ __forceinline__ NF<T> hllc_ns(const K<T> &k, const NS<T> &L, T cl, co
   // densMid * soundMid = (rhoL + rhoR)(cL + cR) / 4
   const T ds = mul(mul(add(L.rho, R.rho), add(cl, cr)), k.quarter);
   const T psraw = fma(ds, sub(L.un, R.un), mul(add(L.p, R.p), k.half));
-  const T presStar = sel(lt(k.zero, psraw), psraw, k.zero);
+  const T presStar = max_(psraw, k.zero);
   const T tL = sqrt_(fma(mul(k.qc, rcp(L.p)), presStar, k.omqc));
   const T tR = sqrt_(fma(mul(k.qc, rcp(R.p)), presStar, k.omqc));
   const T qL = sel(le(L.p, presStar), k.one, tL);
@@ -468,13 +479,11 @@ __device__ __forceinline__ NF<T> hllc_ns(const K<T> &k, const NS<T> &L, T cl, co
   const T shockStar =
       mul(fma(mR, R.un, fma(mL, L.un, sub(L.p, R.p))), rcp(add(mL, mR)));
   // select (0 < SL) L (select (0 < S*) L* (select (0 < SR) R* R))
-  const auto posL = lt(k.zero, shockLeft), posS = lt(k.zero, shockStar),
-             posR = lt(k.zero, shockRight);
-  const auto useL = mor(posL, posS);
-  const auto star = msel(useL, mnot(posL), posR);
+  const auto useL = mor(lt(k.zero, shockLeft), lt(k.zero, shockStar));
   const T r = sel(useL, L.rho, R.rho), p = sel(useL, L.p, R.p);
   const T un = sel(useL, L.un, R.un), ut = sel(useL, L.ut, R.ut);
   const T shock = sel(useL, shockLeft, shockRight);
+  const auto star = mxor(useL, lt(k.zero, shock));
   const T E = fma(mul(k.half, r), fma(un, un, mul(ut, ut)), mul(k.gm1inv, p));
   const T su = sub(shock, un);
   const T idS = rcp(sub(shock, shockStar));
@@ -523,10 +532,10 @@ __device__ __forceinline__ void update_t(const K<T> &k, T rho, T v0, T v1, T p, 
   const T rd = rcp(d2);
   const T u0 = mul(b0, rd), u1 = mul(b1, rd);
   const T pn = mul(k.gm1, fma(k.neghalf, fma(u0, b0, mul(u1, b1)), e2));
-  q[0] = sel(lt(k.floor, d2), d2, k.floor);
+  q[0] = max_(d2, k.floor);
   q[1] = u0;
   q[2] = u1;
-  q[3] = sel(lt(k.floor, pn), pn, k.floor);
+  q[3] = max_(pn, k.floor);
 }
 
 // one-wall forms on the axis-ordered records of the tile kernels

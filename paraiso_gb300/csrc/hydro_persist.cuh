@@ -23,12 +23,12 @@
 //    of a row (or column) are 11 runs, so the 704 wall runs of a tile are
 //    exactly one per thread of the 704-thread CTA.
 //  * The paired form (PAIR, 352 threads) evaluates two walls or two cells
-//    per thread with packed f32x2 instructions (hf::f2): a wall and the
-//    wall 1344 items later, a cell and the cell 672 (stage 1) or 512
-//    (stage 2) later (whole warps, so both halves of a warp run along
-//    rows), a row's x-wall run with a column's y-wall run.  Walls of either
-//    axis share the arithmetic in the frame of the wall; an item without a
-//    partner is paired with itself and stored once.
+//    per thread with packed f32x2 instructions (hf::f2): an x wall and a y
+//    wall, a cell and the cell 672 (stage 1) or 512 (stage 2) later (whole
+//    warps, so both halves of a warp run along rows), a row's x-wall run
+//    with a column's y-wall run.  Walls of either axis share the arithmetic
+//    in the frame of the wall; a cell without a partner is paired with
+//    itself and stored once.
 //  * On large grids the paired form runs as one CTA per SM of two groups
 //    (persist_run's GROUPS), each with its own shared-memory block and
 //    named barrier, whose phases are offset by about half a tile.
@@ -64,14 +64,28 @@ constexpr uint32_t kBoxBytes = 4u * BH * BW * 4u;  // bytes the four TMA boxes d
 constexpr int kS1XMain = 36 * 32, kS1YMain = 37 * 32, kS1XRem = 36 * 5, kS1YRem = 37 * 4;
 constexpr int kS1Items = kS1XMain + kS1YMain + kS1XRem + kS1YRem;  // 2664
 constexpr int kQMain = 36 * 32, kQItems = 36 * 36;                  // stage-1 cells
-// the paired form's second items start a whole number of warps later, so a
-// warp's second items begin a row as its first ones do: wall i pairs with
-// wall i + kS1Half (when that exists), cell i with cell i + kQHalf
-constexpr int kS1Half = (kS1Items / 2 + 31) / 32 * 32;  // 1344
+constexpr int kS1Pairs = kS1Items / 2;  // paired form: an x and a y wall each
+static_assert(kS1XMain + kS1XRem == kS1Pairs && kS1YMain + kS1YRem == kS1Pairs, "");
+// the paired form's second cells start a whole number of warps later, so a
+// warp's second items begin a row as its first ones do
 constexpr int kQHalf = (kQItems / 2 + 31) / 32 * 32;    // 672
 
 using Flux = hs::Flux<float>;
 using Prim = hs::Prim<float>;
+
+// What the items of one instance share, formed by one warp when the CTA (or
+// group) comes to it and read from shared memory instead of being held in
+// registers across phases.  Read and formed by every thread for every tile (with
+// the tile's place), it took 453 us of a 4096^2 step where 438 do, and 3.16 ms
+// of 64 instances of 256 to 2048 cells a side where 2.86 do: there each tile
+// began with a chain of loads from global memory.
+struct Inst {
+  HydroStepArgs a;  // ensembles only
+  int first, end;   // its items
+  float dt, dR0, dR1;
+  float h0, h1, f0, f1;  // dt/2 and dt over dR0 and dR1
+  hf::Consts<float> K;
+};
 
 struct alignas(128) Smem {
   float box[2][4 * PLANE];  // two boxes: planes rho, v0, v1, p (128-byte aligned)
@@ -92,9 +106,11 @@ struct alignas(128) Smem {
   uint64_t bar[2];
   uint64_t go;  // two groups per CTA: group 0 releases group 1 (in group 0's block)
   unsigned red[32];
-  // ensembles: the arguments of the current and the next item's instance
-  // (read from shared memory rather than held in registers across phases)
-  HydroStepArgs args[2];
+  // of the items in box[0] and box[1]: the tile's origin and whether its box
+  // lies inside the grid
+  int4 pos[2];
+  // the current item's instance and the next one's
+  Inst inst[2];
 };
 
 // two CTAs per SM, or one CTA of two groups, within the SM's shared memory
@@ -108,6 +124,28 @@ __device__ __forceinline__ void copy_args(HydroStepArgs *dst, const HydroStepArg
   const uint32_t *s = reinterpret_cast<const uint32_t *>(src);
   uint32_t *d = reinterpret_cast<uint32_t *>(dst);
   for (int i = lane; i < (int)(sizeof(HydroStepArgs) / 4); i += 32) d[i] = s[i];
+}
+
+// a warp fills an instance's block; args: its arguments in global memory (ENS)
+// or among the kernel's parameters
+template <bool ENS>
+__device__ __forceinline__ void fill_inst(Inst &o, const HydroStepArgs &A, int first, int end,
+                                          int lane) {
+  if (ENS) copy_args(&o.a, &A, lane);
+  const float dt = hk::step_dt<float>(A), dR0 = A.sc->dR0_f, dR1 = A.sc->dR1_f;
+  const float half = dt / 2.0f;
+  if (lane == 0) {
+    o.first = first;
+    o.end = end;
+    o.dt = dt;
+    o.dR0 = dR0;
+    o.dR1 = dR1;
+    o.h0 = half / dR0;
+    o.h1 = half / dR1;
+    o.f0 = dt / dR0;
+    o.f1 = dt / dR1;
+    o.K = hf::consts<float>(A.gamma_f);
+  }
 }
 
 // a box lies inside the grid (no periodic image needed)
@@ -172,7 +210,7 @@ __device__ __forceinline__ Prim rec(const float4 v) { return Prim{v.x, v.y, v.z,
 // state of wall j+1.
 template <int AX>
 __device__ __forceinline__ void wall_run(const float4 *q, int base, int st, Flux *out, int ost,
-                                         float g, const hf::Consts<float> &K) {
+                                         const hf::Consts<float> &K) {
   Prim L;
   {
     const Prim x0 = rec(q[base]), x1 = rec(q[base + st]), x2 = rec(q[base + 2 * st]);
@@ -231,6 +269,27 @@ __device__ __forceinline__ void s1_item(int i, int &ax, int &c, int &w) {
   w = ax == 0 ? fy * F1X + fx : fy * F1Y + fx;
 }
 
+// stage-1 wall pair i of the paired form, an x wall and a y wall: box index of
+// the cell left of (below) each and its index in s1.x or s1.y.  Their axes are
+// known where the code is compiled and rows of 32 pair with rows of 32; the
+// last row of 32 y walls and the y remainder go with the x remainder.  (Wall i
+// with the wall 1344 items on, of whatever axis, chose between the velocities
+// of each state and flux: 4096^2 took 485 us a step, 453 so.)
+__device__ __forceinline__ void s1_pair(int i, int &cx, int &wx, int &cy, int &wy) {
+  int fyx = i >> 5, fxx = i & 31, fyy = fyx, fxy = fxx;
+  if (i >= kS1XMain) {
+    const int j = i - kS1XMain, k = j - (kS1YMain - kS1XMain);
+    fyx = j / 5;
+    fxx = 32 + (j - fyx * 5);
+    fyy = k < 0 ? 36 : k >> 2;
+    fxy = k < 0 ? j : 32 + (k & 3);
+  }
+  cx = (fyx + 1) * BW + fxx + 1;
+  wx = fyx * F1X + fxx;
+  cy = fyy * BW + fxy + 2;
+  wy = fyy * F1Y + fxy;
+}
+
 // stage-1 cell item i: (qy, qx) of the 36 x 36 cells
 __device__ __forceinline__ void q_item(int i, int &qy, int &qx) {
   if (i < kQMain) {
@@ -251,37 +310,24 @@ __device__ __forceinline__ hf::NF<f2> pack_flux(const Flux &a, const Flux &b) {
                     hf::pack(a.fe, b.fe)};
 }
 
-// a wall's flux from the frame of the wall back to axis order
-__device__ __forceinline__ Flux axis_order(float fd, float fn, float ft, float fe, int ax) {
-  Flux o;
-  o.fd = fd;
-  o.fm0 = ax == 0 ? fn : ft;
-  o.fm1 = ax == 0 ? ft : fn;
-  o.fe = fe;
-  return o;
-}
-
-__device__ __forceinline__ void store_pair(const hf::NF<f2> &f, Flux *da, int axa, Flux *db,
-                                           int axb) {
+// the fluxes of an x wall and a y wall, back in axis order
+__device__ __forceinline__ void store_pair(const hf::NF<f2> &f, Flux *dx, Flux *dy) {
   float d0, d1, n0, n1, t0, t1, e0, e1;
   hf::unpack(f.fd, d0, d1);
   hf::unpack(f.fn, n0, n1);
   hf::unpack(f.ft, t0, t1);
   hf::unpack(f.fe, e0, e1);
-  *da = axis_order(d0, n0, t0, e0, axa);
-  *db = axis_order(d1, n1, t1, e1, axb);
+  *dx = Flux{d0, n0, t0, e0};
+  *dy = Flux{d1, t1, n1, e1};
 }
 
-// a box cell of wall a and one of wall b in the frames of their walls
-__device__ __forceinline__ hf::NS<f2> pair_state(const float *B, int ca, int axa, int cb,
-                                                 int axb) {
-  const float va0 = B[PLANE + ca], va1 = B[2 * PLANE + ca];
-  const float vb0 = B[PLANE + cb], vb1 = B[2 * PLANE + cb];
-  return hf::NS<f2>{hf::pack(B[ca], B[cb]), hf::pack(axa == 0 ? va0 : va1, axb == 0 ? vb0 : vb1),
-                    hf::pack(axa == 0 ? va1 : va0, axb == 0 ? vb1 : vb0),
-                    hf::pack(B[3 * PLANE + ca], B[3 * PLANE + cb])};
+// box cell cx beside an x wall and box cell cy beside a y wall, in the frames
+// of their walls
+__device__ __forceinline__ hf::NS<f2> pair_state(const float *B, int cx, int cy) {
+  return hf::NS<f2>{hf::pack(B[cx], B[cy]), hf::pack(B[PLANE + cx], B[2 * PLANE + cy]),
+                    hf::pack(B[2 * PLANE + cx], B[PLANE + cy]),
+                    hf::pack(B[3 * PLANE + cx], B[3 * PLANE + cy])};
 }
-
 
 // record k of the x run (row) and of the y run (column), in their walls'
 // frames: (rho, un, ut, p)
@@ -321,7 +367,7 @@ __device__ __forceinline__ void wall_run2(const float4 *q, int xb, int yb, Flux 
       (&Ln.rho)[f] = hf::fma(sl, k.half, c);
     }
     const f2 cr = hf::sound(k, R.rho, R.p);
-    store_pair(hf::hllc_ns<f2>(k, L, cl, R, cr), &xo[j], 0, &yo[j * F2Y], 1);
+    store_pair(hf::hllc_ns<f2>(k, L, cl, R, cr), &xo[j], &yo[j * F2Y]);
     if (j < 2) {
       L = Ln;
       cl = hf::sound(k, L.rho, L.p);
@@ -388,10 +434,13 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
   }
   if (GROUPS == 2 && grp == 1) tma::mbar_wait(&sm[0].go, 0, &args[0].sc->wait_error);
 
-  auto issue = [&](int it, int k, float *dst, uint64_t *bar) {
-    const HydroStepArgs &A = args[k];
-    const int tile = it - (ENS ? pf[k] : 0);
-    const int t1 = tile / A.nt0, t0 = tile - t1 * A.nt0;
+  // start the copy of item `it` of instance k (items from `first` on,
+  // arguments A) into box bb, and leave its place in s.pos[bb]
+  auto issue = [&](int it, int k, int first, const HydroStepArgs &A, int bb) {
+    const int tile = it - first, n0 = A.n0, n1 = A.n1;
+    const int t1 = tile / A.nt0, X0 = (tile - t1 * A.nt0) * TX, Y0 = t1 * TY;
+    const bool inside = box_inside(X0, Y0, n0, n1);
+    if (tid == 0) s.pos[bb] = make_int4(X0, Y0, inside, 0);
     const CUtensorMap *tk = ENS ? table + (size_t)k * 4 : nullptr;
     const FieldRefs r{ENS ? tk : m0,
                       ENS ? tk + 1 : m1,
@@ -401,8 +450,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
                       (const float *)A.v0,
                       (const float *)A.v1,
                       (const float *)A.p};
-    issue_box<NTH>(dst, box_inside(t0 * TX, t1 * TY, A.n0, A.n1), r, A.n0, A.n1, t0 * TX,
-                   t1 * TY, bar, tid);
+    issue_box<NTH>(s.box[bb], inside, r, n0, n1, X0, Y0, &s.bar[bb], tid);
   };
 
   // sound speeds of the box cells into s.cq.c: items [i0, BH*BW/ (PAIR ? 2 : 1))
@@ -421,84 +469,74 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
         s.cq.c[i] = hf::sound(Kx, Bx[i], Bx[3 * PLANE + i]);
     }
   };
-  // wait until the box of tile (X0, Y0) of a grid has landed in
-  // buffer bb (the caller synchronises the block afterwards)
+  // wait until the box of the item in s.pos[bb] has landed (the caller
+  // synchronises the block before, so that s.pos holds, and afterwards)
   uint32_t parity = 0;  // bit k: parity of the next completed phase of bar[k]
-  auto await_box = [&](int bb, int X0, int Y0, const HydroStepArgs &A) {
-    if (box_inside(X0, Y0, A.n0, A.n1)) {
+  auto await_box = [&](int bb, const HydroStepArgs &A) {
+    if (s.pos[bb].z) {
       tma::mbar_wait(&s.bar[bb], (parity >> bb) & 1u, &A.sc->wait_error);
       parity ^= 1u << bb;
     } else {
       hk::cp_async_wait_all();
     }
   };
-  auto tile_origin = [&](int it, int k, int &X0, int &Y0) {
-    const HydroStepArgs &A = args[k];
-    const int tile = it - (ENS ? pf[k] : 0);
-    const int t1 = tile / A.nt0;
-    X0 = (tile - t1 * A.nt0) * TX;
-    Y0 = t1 * TY;
-  };
 
   int lo = 0;  // instance of `item`
-  if (ENS)
-    while (lo < count - 1 && pf[lo + 1] <= item) ++lo;
-  issue(item, lo, s.box[0], &s.bar[0]);
-  if (ENS && warp == 0) copy_args(&s.args[0], &args[lo], lane);
+  int ai = 0;  // its slot in s.inst
   {
-    int X0, Y0;
-    tile_origin(item, lo, X0, Y0);
-    await_box(0, X0, Y0, args[lo]);
+    if (ENS)
+      while (lo < count - 1 && pf[lo + 1] <= item) ++lo;
+    const int first = ENS ? pf[lo] : 0, end = ENS ? pf[lo + 1] : total;
+    issue(item, lo, first, args[lo], 0);
+    if (warp == 0) fill_inst<ENS>(s.inst[0], args[lo], first, end, lane);
     sync();
-    sounds(s.box[0], hf::consts<float>(args[lo].gamma_f), tid, NTH);
+    await_box(0, args[lo]);
+    sync();
+    sounds(s.box[0], s.inst[0].K, tid, NTH);
   }
   sync();
   int b = 0;
   unsigned m = ~0u;
 
   for (;;) {
-    const HydroStepArgs &A = ENS ? s.args[b] : args[lo];
-    const int n0 = A.n0, n1 = A.n1;
-    const int tile = item - (ENS ? pf[lo] : 0);
-    int X0, Y0;
-    tile_origin(item, lo, X0, Y0);
-    const float g = A.gamma_f;
-    const hf::Consts<float> K = hf::consts<float>(g);
-    const float dR0 = A.sc->dR0_f, dR1 = A.sc->dR1_f;
-    const float dtG = hk::step_dt<float>(A);
-    const float dtHalf = dtG / 2.0f;
+    Inst &I = s.inst[ai];
+    const HydroStepArgs &A = ENS ? I.a : args[0];
+    const int n0 = A.n0;
+    const int X0 = s.pos[b].x, Y0 = s.pos[b].y;
     const float *B = s.box[b];
 
     // the next item's box goes into the other buffer while this one computes
     // (that buffer's last reader, the previous tile's stage 2, is behind the
-    // last barrier)
+    // last barrier, and so is the last reader of the other instance slot)
     const int next = item + stride;
     int lo_n = lo;
     if (next < total) {
-      if (ENS)
-        while (lo_n < count - 1 && pf[lo_n + 1] <= next) ++lo_n;
-      issue(next, lo_n, s.box[b ^ 1], &s.bar[b ^ 1]);
+      if (!ENS || next < I.end) {
+        issue(next, lo, ENS ? I.first : 0, A, b ^ 1);
+      } else {
+        do ++lo_n;
+        while (lo_n < count - 1 && pf[lo_n + 1] <= next);
+        const int first = pf[lo_n];
+        issue(next, lo_n, first, args[lo_n], b ^ 1);
+        if (warp == NTH / 32 - 1)
+          fill_inst<ENS>(s.inst[ai ^ 1], args[lo_n], first, pf[lo_n + 1], lane);
+      }
     }
+    const int an = lo_n == lo ? ai : ai ^ 1;  // the next item's instance
 
     // stage-1 walls, order-1 reconstruction
     if (PAIR) {
-      const hf::K<f2> k2 = hf::kconsts<f2>(K);
-      for (int i = tid; i < kS1Half; i += NTH) {
-        int axa, ca, wa, axb, cb, wb;
-        s1_item(i, axa, ca, wa);
-        const bool two = i + kS1Half < kS1Items;
-        s1_item(two ? i + kS1Half : i, axb, cb, wb);
-        const int da = axa == 0 ? 1 : BW, db = axb == 0 ? 1 : BW;
-        const hf::NS<f2> L = pair_state(B, ca, axa, cb, axb);
-        const hf::NS<f2> R = pair_state(B, ca + da, axa, cb + db, axb);
-        const f2 cl = hf::pack(s.cq.c[ca], s.cq.c[cb]);
-        const f2 cr = hf::pack(s.cq.c[ca + da], s.cq.c[cb + db]);
-        Flux fa, fb;
-        store_pair(hf::hllc_ns<f2>(k2, L, cl, R, cr), &fa, axa, &fb, axb);
-        (axa == 0 ? s.fl.s1.x[wa] : s.fl.s1.y[wa]) = fa;
-        if (two) (axb == 0 ? s.fl.s1.x[wb] : s.fl.s1.y[wb]) = fb;
+      const hf::K<f2> k2 = hf::kconsts<f2>(I.K);
+      for (int i = tid; i < kS1Pairs; i += NTH) {
+        int cx, wx, cy, wy;
+        s1_pair(i, cx, wx, cy, wy);
+        const hf::NS<f2> L = pair_state(B, cx, cy), R = pair_state(B, cx + 1, cy + BW);
+        const f2 cl = hf::pack(s.cq.c[cx], s.cq.c[cy]);
+        const f2 cr = hf::pack(s.cq.c[cx + 1], s.cq.c[cy + BW]);
+        store_pair(hf::hllc_ns<f2>(k2, L, cl, R, cr), &s.fl.s1.x[wx], &s.fl.s1.y[wy]);
       }
     } else {
+      const hf::Consts<float> K = I.K;
       for (int i = tid; i < kS1Items; i += NTH) {
         int ax, c, w;
         s1_item(i, ax, c, w);
@@ -514,7 +552,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
 
     // stage-1 cells (qy, qx) = box cell (qy+1, qx+2), advanced by dt/2
     {
-      const float dtdx0 = dtHalf / dR0, dtdx1 = dtHalf / dR1;
+      const float dtdx0 = I.h0, dtdx1 = I.h1;
       auto tape_cell = [&](int qy, int qx, const float *q, const Flux &l0, const Flux &r0,
                            const Flux &l1, const Flux &r1) {
         const int ty = qy - 2, tx = qx - 2;
@@ -526,7 +564,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
         }
       };
       if (PAIR) {
-        const hf::K<f2> k2 = hf::kconsts<f2>(K);
+        const hf::K<f2> k2 = hf::kconsts<f2>(I.K);
         const f2 t0 = hf::splat<f2>(dtdx0), t1 = hf::splat<f2>(dtdx1);
         for (int i = tid; i < kQHalf; i += NTH) {
           int qya, qxa, qyb, qxb;
@@ -555,6 +593,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
           if (two) s.cq.q[qyb * QP + qxb] = make_float4(qb[0], qb[1], qb[2], qb[3]);
         }
       } else {
+        const hf::Consts<float> K = I.K;
         for (int i = tid; i < kQItems; i += NTH) {
           int qy, qx;
           q_item(i, qy, qx);
@@ -581,20 +620,15 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     if (PAIR) {
       wall_run2(s.cq.q, (lane + 2) * QP + 3 * warp, 3 * warp * QP + lane + 2,
                 &s.fl.s2.x[lane * F2X + 3 * warp], &s.fl.s2.y[3 * warp * F2Y + lane],
-                hf::kconsts<f2>(K));
+                hf::kconsts<f2>(I.K));
     } else if (warp < 11) {
-      wall_run<0>(s.cq.q, (lane + 2) * QP + 3 * warp, 1, &s.fl.s2.x[lane * F2X + 3 * warp], 1, g,
-                  K);
+      wall_run<0>(s.cq.q, (lane + 2) * QP + 3 * warp, 1, &s.fl.s2.x[lane * F2X + 3 * warp], 1, I.K);
     } else {
       const int t = warp - 11;
-      wall_run<1>(s.cq.q, 3 * t * QP + lane + 2, QP, &s.fl.s2.y[3 * t * F2Y + lane], F2Y, g, K);
+      wall_run<1>(s.cq.q, 3 * t * QP + lane + 2, QP, &s.fl.s2.y[3 * t * F2Y + lane], F2Y, I.K);
     }
     // the next box must have landed before its sound speeds are formed
-    if (next < total) {
-      int Xn, Yn;
-      tile_origin(next, lo_n, Xn, Yn);
-      await_box(b ^ 1, Xn, Yn, args[lo_n]);
-    }
+    if (next < total) await_box(b ^ 1, ENS ? s.inst[an].a : args[0]);
     sync();
 
     // stage-2 cells (oy, ox) = box cell (oy+3, ox+4), advanced by dt and
@@ -604,7 +638,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     {
       constexpr int P4 = PAIR ? TX * TY / 2 : TX * TY;  // stage-2 items
       constexpr int ONE = P4 - NTH;  // threads from here on take one item
-      const float dtdx0 = dtG / dR0, dtdx1 = dtG / dR1;
+      const float dtdx0 = I.f0, dtdx1 = I.f1, g = I.K.g, dR0 = I.dR0, dR1 = I.dR1;
       float *out[4] = {(float *)A.nrho, (float *)A.nv0, (float *)A.nv1, (float *)A.np};
       auto put = [&](int oy, int ox, const float *q, const float *cons, const Flux &l0,
                      const Flux &r0, const Flux &l1, const Flux &r1) {
@@ -621,7 +655,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
         m = min(m, __float_as_uint(t));
       };
       if (PAIR) {
-        const hf::K<f2> k2 = hf::kconsts<f2>(K);
+        const hf::K<f2> k2 = hf::kconsts<f2>(I.K);
         const f2 t0 = hf::splat<f2>(dtdx0), t1 = hf::splat<f2>(dtdx1);
         for (int i = tid; i < P4; i += NTH) {
           const int oya = i >> 5, ox = i & 31, oyb = oya + TY / 2;
@@ -646,6 +680,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
           put(oyb, ox, qb, cb4, l0b, r0b, l1b, r1b);
         }
       } else {
+        const hf::Consts<float> K = I.K;
         for (int i = tid; i < P4; i += NTH) {
           const int oy = i >> 5, ox = i & 31;
           const int c = (oy + 3) * BW + ox + 4;
@@ -659,17 +694,15 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
         }
       }
       if (next < total && tid >= ONE)
-        sounds(s.box[b ^ 1], hf::consts<float>(args[lo_n].gamma_f), tid - ONE, NTH - ONE);
+        sounds(s.box[b ^ 1], s.inst[an].K, tid - ONE, NTH - ONE);
     }
-    if (tile == 0 && tid == 0) {
+    if (X0 == 0 && Y0 == 0 && tid == 0) {
+      const float dtG = I.dt;
       if (A.ts_clear) *ts_at(A, A.ts_clear) = ~0ull;
       A.dt_hist[0] = (double)dtG;
       A.sc->dt_last = (double)dtG;
       A.sc->time = A.sc->time + (double)dtG;
     }
-    // the next item's arguments into the other slot (its last reader, the
-    // previous item, is behind the last barrier)
-    if (ENS && next < total && warp == NTH / 32 - 1) copy_args(&s.args[b ^ 1], &args[lo_n], lane);
     // publish the CFL minimum when this CTA leaves the instance (the
     // reduction ends with a barrier); else one barrier before the next tile
     if (next >= total || lo_n != lo) {
@@ -681,6 +714,7 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     if (next >= total) break;
     item = next;
     lo = lo_n;
+    ai = an;
     b ^= 1;
   }
 }

@@ -23,12 +23,10 @@
 //    of a row (or column) are 11 runs, so the 704 wall runs of a tile are
 //    exactly one per thread of the 704-thread CTA.
 //  * The paired form (PAIR, 352 threads) evaluates two walls or two cells
-//    per thread with packed f32x2 instructions (hf::f2): an x wall and a y
-//    wall, a cell and the cell 672 (stage 1) or 512 (stage 2) later (whole
-//    warps, so both halves of a warp run along rows), a row's x-wall run
-//    with a column's y-wall run.  Walls of either axis share the arithmetic
-//    in the frame of the wall; a cell without a partner is paired with
-//    itself and stored once.
+//    per thread with packed f32x2 instructions (hf::f2): the x wall left of a
+//    cell with the y wall below it, a cell with the one above it, a row's
+//    x-wall run with a column's y-wall run.  Walls of either axis share the
+//    arithmetic in the frame of the wall.
 //  * On large grids the paired form runs as one CTA per SM of two groups
 //    (persist_run's GROUPS), each with its own shared-memory block and
 //    named barrier, whose phases are offset by about half a tile.
@@ -64,11 +62,8 @@ constexpr uint32_t kBoxBytes = 4u * BH * BW * 4u;  // bytes the four TMA boxes d
 constexpr int kS1XMain = 36 * 32, kS1YMain = 37 * 32, kS1XRem = 36 * 5, kS1YRem = 37 * 4;
 constexpr int kS1Items = kS1XMain + kS1YMain + kS1XRem + kS1YRem;  // 2664
 constexpr int kQMain = 36 * 32, kQItems = 36 * 36;                  // stage-1 cells
-constexpr int kS1Pairs = kS1Items / 2;  // paired form: an x and a y wall each
-static_assert(kS1XMain + kS1XRem == kS1Pairs && kS1YMain + kS1YRem == kS1Pairs, "");
-// the paired form's second cells start a whole number of warps later, so a
-// warp's second items begin a row as its first ones do
-constexpr int kQHalf = (kQItems / 2 + 31) / 32 * 32;    // 672
+constexpr int kS1PairMain = 37 * 32, kS1Pairs = 37 * 37;  // paired form
+constexpr int kQPairMain = 18 * 32, kQPairs = 18 * 36;    // paired form
 
 using Flux = hs::Flux<float>;
 using Prim = hs::Prim<float>;
@@ -269,25 +264,23 @@ __device__ __forceinline__ void s1_item(int i, int &ax, int &c, int &w) {
   w = ax == 0 ? fy * F1X + fx : fy * F1Y + fx;
 }
 
-// stage-1 wall pair i of the paired form, an x wall and a y wall: box index of
-// the cell left of (below) each and its index in s1.x or s1.y.  Their axes are
-// known where the code is compiled and rows of 32 pair with rows of 32; the
-// last row of 32 y walls and the y remainder go with the x remainder.  (Wall i
-// with the wall 1344 items on, of whatever axis, chose between the velocities
-// of each state and flux: 4096^2 took 485 us a step, 453 so.)
-__device__ __forceinline__ void s1_pair(int i, int &cx, int &wx, int &cy, int &wy) {
-  int fyx = i >> 5, fxx = i & 31, fyy = fyx, fxy = fxx;
-  if (i >= kS1XMain) {
-    const int j = i - kS1XMain, k = j - (kS1YMain - kS1XMain);
-    fyx = j / 5;
-    fxx = 32 + (j - fyx * 5);
-    fyy = k < 0 ? 36 : k >> 2;
-    fxy = k < 0 ? j : 32 + (k & 3);
+// stage-1 wall pair i of the paired form: the x wall left of a cell and the y
+// wall below it, for the 37 x 37 cells that are right of or above a wall (rows
+// of 32, then the remainder).  The pair's axes are known where the code is
+// compiled and it reads three cells; the x walls of the last row and the y walls
+// of the last column are no walls of the tile (their cells lie in the box): not
+// stored.  (Wall i with the wall 1344 items on, of whatever axis, chose between
+// the velocities of each state and flux: 4096^2 took 485 us a step, 438 so, and
+// 434 with the common cell and the wall between two paired cells read once; the
+// ensembles below 2.86 ms, 2.75.)
+__device__ __forceinline__ void s1_pair(int i, int &fy, int &fx) {
+  fy = i >> 5;
+  fx = i & 31;
+  if (i >= kS1PairMain) {
+    const int j = i - kS1PairMain;
+    fy = j / 5;
+    fx = 32 + (j - fy * 5);
   }
-  cx = (fyx + 1) * BW + fxx + 1;
-  wx = fyx * F1X + fxx;
-  cy = fyy * BW + fxy + 2;
-  wy = fyy * F1Y + fxy;
 }
 
 // stage-1 cell item i: (qy, qx) of the 36 x 36 cells
@@ -297,6 +290,16 @@ __device__ __forceinline__ void q_item(int i, int &qy, int &qx) {
   } else {
     const int j = i - kQMain;
     qy = j >> 2; qx = 32 + (j & 3);
+  }
+}
+
+// stage-1 cell pair i: cells (qy, qx) and (qy + 1, qx), qy even
+__device__ __forceinline__ void q_pair(int i, int &qy, int &qx) {
+  if (i < kQPairMain) {
+    qy = i >> 5 << 1; qx = i & 31;
+  } else {
+    const int j = i - kQPairMain;
+    qy = j >> 2 << 1; qx = 32 + (j & 3);
   }
 }
 
@@ -311,14 +314,14 @@ __device__ __forceinline__ hf::NF<f2> pack_flux(const Flux &a, const Flux &b) {
 }
 
 // the fluxes of an x wall and a y wall, back in axis order
-__device__ __forceinline__ void store_pair(const hf::NF<f2> &f, Flux *dx, Flux *dy) {
+__device__ __forceinline__ void split_pair(const hf::NF<f2> &f, Flux &x, Flux &y) {
   float d0, d1, n0, n1, t0, t1, e0, e1;
   hf::unpack(f.fd, d0, d1);
   hf::unpack(f.fn, n0, n1);
   hf::unpack(f.ft, t0, t1);
   hf::unpack(f.fe, e0, e1);
-  *dx = Flux{d0, n0, t0, e0};
-  *dy = Flux{d1, t1, n1, e1};
+  x = Flux{d0, n0, t0, e0};
+  y = Flux{d1, t1, n1, e1};
 }
 
 // box cell cx beside an x wall and box cell cy beside a y wall, in the frames
@@ -367,7 +370,7 @@ __device__ __forceinline__ void wall_run2(const float4 *q, int xb, int yb, Flux 
       (&Ln.rho)[f] = hf::fma(sl, k.half, c);
     }
     const f2 cr = hf::sound(k, R.rho, R.p);
-    store_pair(hf::hllc_ns<f2>(k, L, cl, R, cr), &xo[j], &yo[j * F2Y]);
+    split_pair(hf::hllc_ns<f2>(k, L, cl, R, cr), xo[j], yo[j * F2Y]);
     if (j < 2) {
       L = Ln;
       cl = hf::sound(k, L.rho, L.p);
@@ -528,12 +531,17 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
     if (PAIR) {
       const hf::K<f2> k2 = hf::kconsts<f2>(I.K);
       for (int i = tid; i < kS1Pairs; i += NTH) {
-        int cx, wx, cy, wy;
-        s1_pair(i, cx, wx, cy, wy);
-        const hf::NS<f2> L = pair_state(B, cx, cy), R = pair_state(B, cx + 1, cy + BW);
-        const f2 cl = hf::pack(s.cq.c[cx], s.cq.c[cy]);
-        const f2 cr = hf::pack(s.cq.c[cx + 1], s.cq.c[cy + BW]);
-        store_pair(hf::hllc_ns<f2>(k2, L, cl, R, cr), &s.fl.s1.x[wx], &s.fl.s1.y[wy]);
+        int fy, fx;
+        s1_pair(i, fy, fx);
+        const int c = (fy + 1) * BW + fx + 2;
+        // the cell left of, the one below, and the one right of and above
+        const hf::NS<f2> L = pair_state(B, c - 1, c - BW), R = pair_state(B, c, c);
+        const f2 cl = hf::pack(s.cq.c[c - 1], s.cq.c[c - BW]);
+        const f2 cr = hf::pack(s.cq.c[c], s.cq.c[c]);
+        Flux x, y;
+        split_pair(hf::hllc_ns<f2>(k2, L, cl, R, cr), x, y);
+        if (fy < 36) s.fl.s1.x[fy * F1X + fx] = x;
+        if (fx < 36) s.fl.s1.y[fy * F1Y + fx] = y;
       }
     } else {
       const hf::Consts<float> K = I.K;
@@ -566,31 +574,31 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
       if (PAIR) {
         const hf::K<f2> k2 = hf::kconsts<f2>(I.K);
         const f2 t0 = hf::splat<f2>(dtdx0), t1 = hf::splat<f2>(dtdx1);
-        for (int i = tid; i < kQHalf; i += NTH) {
-          int qya, qxa, qyb, qxb;
-          q_item(i, qya, qxa);
-          const bool two = i + kQHalf < kQItems;
-          q_item(two ? i + kQHalf : i, qyb, qxb);
-          const int ca = (qya + 1) * BW + qxa + 2, cb = (qyb + 1) * BW + qxb + 2;
-          const Flux &l0a = s.fl.s1.x[qya * F1X + qxa], &r0a = s.fl.s1.x[qya * F1X + qxa + 1];
-          const Flux &l1a = s.fl.s1.y[qya * F1Y + qxa], &r1a = s.fl.s1.y[(qya + 1) * F1Y + qxa];
-          const Flux &l0b = s.fl.s1.x[qyb * F1X + qxb], &r0b = s.fl.s1.x[qyb * F1X + qxb + 1];
-          const Flux &l1b = s.fl.s1.y[qyb * F1Y + qxb], &r1b = s.fl.s1.y[(qyb + 1) * F1Y + qxb];
+        for (int i = tid; i < kQPairs; i += NTH) {
+          int qy, qx;
+          q_pair(i, qy, qx);
+          const int ca = (qy + 1) * BW + qx + 2, cb = ca + BW;
+          const Flux &l0a = s.fl.s1.x[qy * F1X + qx], &r0a = s.fl.s1.x[qy * F1X + qx + 1];
+          const Flux &l0b = s.fl.s1.x[(qy + 1) * F1X + qx],
+                     &r0b = s.fl.s1.x[(qy + 1) * F1X + qx + 1];
+          // the wall between the two cells is read once
+          const Flux &l1a = s.fl.s1.y[qy * F1Y + qx], &r1b = s.fl.s1.y[(qy + 2) * F1Y + qx];
+          const Flux mid = s.fl.s1.y[(qy + 1) * F1Y + qx];
           f2 q[4];
           hf::update_t<f2>(k2, hf::pack(B[ca], B[cb]), hf::pack(B[PLANE + ca], B[PLANE + cb]),
                            hf::pack(B[2 * PLANE + ca], B[2 * PLANE + cb]),
                            hf::pack(B[3 * PLANE + ca], B[3 * PLANE + cb]), t0, t1,
-                           pack_flux(l0a, l0b), pack_flux(r0a, r0b), pack_flux(l1a, l1b),
-                           pack_flux(r1a, r1b), q);
+                           pack_flux(l0a, l0b), pack_flux(r0a, r0b), pack_flux(l1a, mid),
+                           pack_flux(mid, r1b), q);
           float qa[4], qb[4];
 #pragma unroll
           for (int f = 0; f < 4; ++f) hf::unpack(q[f], qa[f], qb[f]);
           if (TAPE) {
-            tape_cell(qya, qxa, qa, l0a, r0a, l1a, r1a);
-            if (two) tape_cell(qyb, qxb, qb, l0b, r0b, l1b, r1b);
+            tape_cell(qy, qx, qa, l0a, r0a, l1a, mid);
+            tape_cell(qy + 1, qx, qb, l0b, r0b, mid, r1b);
           }
-          s.cq.q[qya * QP + qxa] = make_float4(qa[0], qa[1], qa[2], qa[3]);
-          if (two) s.cq.q[qyb * QP + qxb] = make_float4(qb[0], qb[1], qb[2], qb[3]);
+          s.cq.q[qy * QP + qx] = make_float4(qa[0], qa[1], qa[2], qa[3]);
+          s.cq.q[(qy + 1) * QP + qx] = make_float4(qb[0], qb[1], qb[2], qb[3]);
         }
       } else {
         const hf::Consts<float> K = I.K;
@@ -658,26 +666,27 @@ __device__ __forceinline__ void persist_run(const HydroStepArgs *__restrict__ ar
         const hf::K<f2> k2 = hf::kconsts<f2>(I.K);
         const f2 t0 = hf::splat<f2>(dtdx0), t1 = hf::splat<f2>(dtdx1);
         for (int i = tid; i < P4; i += NTH) {
-          const int oya = i >> 5, ox = i & 31, oyb = oya + TY / 2;
-          const int ca = (oya + 3) * BW + ox + 4, cb = ca + (TY / 2) * BW;
-          const Flux &l0a = s.fl.s2.x[oya * F2X + ox], &r0a = s.fl.s2.x[oya * F2X + ox + 1];
-          const Flux &l1a = s.fl.s2.y[oya * F2Y + ox], &r1a = s.fl.s2.y[(oya + 1) * F2Y + ox];
-          const Flux &l0b = s.fl.s2.x[oyb * F2X + ox], &r0b = s.fl.s2.x[oyb * F2X + ox + 1];
-          const Flux &l1b = s.fl.s2.y[oyb * F2Y + ox], &r1b = s.fl.s2.y[(oyb + 1) * F2Y + ox];
+          const int oy = i >> 5 << 1, ox = i & 31;
+          const int ca = (oy + 3) * BW + ox + 4, cb = ca + BW;
+          const Flux &l0a = s.fl.s2.x[oy * F2X + ox], &r0a = s.fl.s2.x[oy * F2X + ox + 1];
+          const Flux &l0b = s.fl.s2.x[(oy + 1) * F2X + ox],
+                     &r0b = s.fl.s2.x[(oy + 1) * F2X + ox + 1];
+          const Flux &l1a = s.fl.s2.y[oy * F2Y + ox], &r1b = s.fl.s2.y[(oy + 2) * F2Y + ox];
+          const Flux mid = s.fl.s2.y[(oy + 1) * F2Y + ox];
           f2 q[4], cons[4];
           hf::update_t<f2>(k2, hf::pack(B[ca], B[cb]), hf::pack(B[PLANE + ca], B[PLANE + cb]),
                            hf::pack(B[2 * PLANE + ca], B[2 * PLANE + cb]),
                            hf::pack(B[3 * PLANE + ca], B[3 * PLANE + cb]), t0, t1,
-                           pack_flux(l0a, l0b), pack_flux(r0a, r0b), pack_flux(l1a, l1b),
-                           pack_flux(r1a, r1b), q, TAPE ? cons : nullptr);
+                           pack_flux(l0a, l0b), pack_flux(r0a, r0b), pack_flux(l1a, mid),
+                           pack_flux(mid, r1b), q, TAPE ? cons : nullptr);
           float qa[4], qb[4], ca4[4], cb4[4];
 #pragma unroll
           for (int f = 0; f < 4; ++f) {
             hf::unpack(q[f], qa[f], qb[f]);
             if (TAPE) hf::unpack(cons[f], ca4[f], cb4[f]);
           }
-          put(oya, ox, qa, ca4, l0a, r0a, l1a, r1a);
-          put(oyb, ox, qb, cb4, l0b, r0b, l1b, r1b);
+          put(oy, ox, qa, ca4, l0a, r0a, l1a, mid);
+          put(oy + 1, ox, qb, cb4, l0b, r0b, mid, r1b);
         }
       } else {
         const hf::Consts<float> K = I.K;

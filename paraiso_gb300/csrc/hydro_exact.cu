@@ -72,9 +72,12 @@ static cudaError_t launch_f64(const HydroStepArgs &a0, const HydroStage1 &q, cud
                                 sizeof(Stage1Smem<double, TX, TY>), s, a, q);
   if (err != cudaSuccess) return err;
   a.nt0 = (a.n0 + TX - 1) / TX;
+  const size_t smem = sizeof(Stage2Smem<double, TX, TY>);
+  err = cudaFuncSetAttribute(hydro_stage2_kernel<double, TX, TY, NT, OPEN>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return err;
   return launch_step(hydro_stage2_kernel<double, TX, TY, NT, OPEN>,
-                     a.nt0 * ((a.n1 + TY - 1) / TY), NT, sizeof(Stage2Smem<double, TX, TY>), s, a,
-                     q);
+                     a.nt0 * ((a.n1 + TY - 1) / TY), NT, smem, s, a, q);
 }
 
 // a.lm > 0: open grid (margins, jet boundary condition)

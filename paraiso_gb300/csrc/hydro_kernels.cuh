@@ -544,13 +544,27 @@ template <class R, int TX, int TY> struct Stage1Smem {
   hk::StageConsts<R> c;
   R P[4][PY][PX];
   R C[PY][PX];
+  R M[3][PY][PX];  // momenta and energy
   hs::Flux<R> fx[TY * (TX + 1)];
   hs::Flux<R> fy[(TY + 1) * TX];
+  // the momenta and energies of a wall's cells, m and m + step
+  template <int AX> struct Wall {
+    const R *m;
+    int step;
+    __device__ __forceinline__ R momL() const { return m[AX * PY * PX]; }
+    __device__ __forceinline__ R momR() const { return m[AX * PY * PX + step]; }
+    __device__ __forceinline__ hs::Cons<R> side(bool left, R, R, R, R) const {
+      const R *x = left ? m : m + step;
+      return hs::Cons<R>{x[0], x[PY * PX], x[2 * PY * PX]};
+    }
+  };
 };
 template <class R, int TX, int TY> struct Stage2Smem {
   static constexpr int QX = TX + 4, QY = TY + 4;
   hk::StageConsts<R> c;
   R Q[4][QY][QX];
+  R dx[4][TY][TX + 3];  // differences of a tile row's cells, and of a column's
+  R dy[4][TY + 3][TX];
   hs::Flux<R> fx[TY * (TX + 1)];
   hs::Flux<R> fy[(TY + 1) * TX];
 };
@@ -603,16 +617,27 @@ hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
   auto cell = [&](int py, int px) {
     return hs::Prim<R>{s.P[0][py][px], s.P[1][py][px], s.P[2][py][px], s.P[3][py][px]};
   };
+  for (int i = tid; i < S::PY * S::PX; i += NT) {
+    const int py = i / S::PX, px = i - py * S::PX;
+    const hs::Prim<R> w = cell(py, px);
+    const hs::Cons<R> c = hs::cons_of(k, w.rho, w.v0, w.v1, w.p);
+    s.M[0][py][px] = c.m0;
+    s.M[1][py][px] = c.m1;
+    s.M[2][py][px] = c.e;
+  }
+  __syncthreads();
   constexpr int NX = TY * (TX + 1), NY = (TY + 1) * TX;
   for (int i = tid; i < NX + NY; i += NT) {
     if (i < NX) {
       const int sy = i / (TX + 1), sx = i - sy * (TX + 1);
       s.fx[i] = hs::hllc<0>(k, cell(sy + 1, sx), s.C[sy + 1][sx], cell(sy + 1, sx + 1),
-                            s.C[sy + 1][sx + 1]);
+                            s.C[sy + 1][sx + 1],
+                            typename S::template Wall<0>{&s.M[0][sy + 1][sx], 1});
     } else {
       const int j = i - NX, sy = j / TX, sx = j - sy * TX;
       s.fy[j] = hs::hllc<1>(k, cell(sy, sx + 1), s.C[sy][sx + 1], cell(sy + 1, sx + 1),
-                            s.C[sy + 1][sx + 1]);
+                            s.C[sy + 1][sx + 1],
+                            typename S::template Wall<1>{&s.M[0][sy][sx + 1], S::PX});
     }
   }
   __syncthreads();
@@ -621,9 +646,10 @@ hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
     const int oy = i / TX, ox = i - oy * TX;
     const int iy = Y0 + oy, ix = X0 + ox;
     if (iy >= n1 + e || ix >= n0 + e) continue;
-    const hs::Prim<R> q = hs::update(k, cell(oy + 1, ox + 1), dtdx0, dtdx1,
-                                     s.fx[oy * (TX + 1) + ox], s.fx[oy * (TX + 1) + ox + 1],
-                                     s.fy[oy * TX + ox], s.fy[(oy + 1) * TX + ox]);
+    const hs::Cons<R> c{s.M[0][oy + 1][ox + 1], s.M[1][oy + 1][ox + 1], s.M[2][oy + 1][ox + 1]};
+    const hs::Prim<R> q = hs::update_cons<R>(
+        k, s.P[0][oy + 1][ox + 1], c, dtdx0, dtdx1, s.fx[oy * (TX + 1) + ox],
+        s.fx[oy * (TX + 1) + ox + 1], s.fy[oy * TX + ox], s.fy[(oy + 1) * TX + ox], nullptr);
     const size_t gi = OPEN ? (size_t)(iy + a.lm) * a.ms0 + (ix + a.lm) : (size_t)iy * n0 + ix;
     ((R *)o.q[0])[gi] = q.rho;
     ((R *)o.q[1])[gi] = q.v0;
@@ -664,6 +690,18 @@ hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
     for (int c = 0; c < 4; ++c) s.Q[c][qy][qx] = ((const R *)o.q[c])[gi];
   }
   __syncthreads();
+  for (int i = tid; i < TY * (TX + 3) + (TY + 3) * TX; i += NT) {
+    const bool x = i < TY * (TX + 3);
+    const int j = x ? i : i - TY * (TX + 3), r = x ? j / (TX + 3) : j / TX,
+              q = x ? j - r * (TX + 3) : j - r * TX;
+    const int y0 = x ? r + 2 : r, x0 = x ? q : q + 2;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const R d = s.Q[c][y0 + !x][x0 + x] - s.Q[c][y0][x0];
+      (x ? s.dx[c][r][q] : s.dy[c][r][q]) = d;
+    }
+  }
+  __syncthreads();
   const hs::Gas<R> k = s.c.gas;
   constexpr int NX = TY * (TX + 1), NY = (TY + 1) * TX;
   for (int i = tid; i < NX + NY; i += NT) {
@@ -671,12 +709,14 @@ hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
     const int j = x ? i : i - NX;
     const int sy = x ? j / (TX + 1) : j / TX, sx = x ? j - sy * (TX + 1) : j - sy * TX;
     // the wall lies between cells 1 and 2 of four along its axis
-    const int qy = x ? sy + 2 : sy, qx = x ? sx : sx + 2, dy = x ? 0 : 1, dx = x ? 1 : 0;
+    const int qy = x ? sy + 2 : sy + 1, qx = x ? sx + 1 : sx + 2, dy = x ? 0 : 1, dx = x ? 1 : 0;
+    const int step = x ? 1 : TX, field = x ? TY * (TX + 3) : (TY + 3) * TX;
+    const R *d = x ? &s.dx[0][sy][sx] : &s.dy[0][sy][sx];
     hs::Prim<R> L, Rt;
 #pragma unroll
     for (int c = 0; c < 4; ++c)
-      hs::muscl(s.Q[c][qy][qx], s.Q[c][qy + dy][qx + dx], s.Q[c][qy + 2 * dy][qx + 2 * dx],
-                s.Q[c][qy + 3 * dy][qx + 3 * dx], (&L.rho)[c], (&Rt.rho)[c]);
+      hs::muscl_of(s.Q[c][qy][qx], s.Q[c][qy + dy][qx + dx], d[c * field], d[c * field + step],
+                   d[c * field + 2 * step], (&L.rho)[c], (&Rt.rho)[c]);
     const R cl = hs::sound(k.g, L.rho, L.p), cr = hs::sound(k.g, Rt.rho, Rt.p);
     if (x) s.fx[j] = hs::hllc<0>(k, L, cl, Rt, cr);
     else s.fy[j] = hs::hllc<1>(k, L, cl, Rt, cr);

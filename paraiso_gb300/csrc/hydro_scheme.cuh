@@ -77,11 +77,12 @@ template <class R> __device__ __forceinline__ R kinetic(R v0, R v1, R m0, R m1) 
   return half(plus_zero(v0 * m0) + v1 * m1);
 }
 
-// energy of a primitive record: Ek + 1/(gamma-1) * p
+// momenta and energy (Ek + 1/(gamma-1) * p) of a primitive record
+template <class R> struct Cons { R m0, m1, e; };
 template <class R>
-__device__ __forceinline__ R energy_prim(const Gas<R> &k, R rho, R v0, R v1, R p) {
+__device__ __forceinline__ Cons<R> cons_of(const Gas<R> &k, R rho, R v0, R v1, R p) {
   const R m0 = rho * v0, m1 = rho * v1;
-  return kinetic(v0, v1, m0, m1) + k.gm1inv * p;
+  return Cons<R>{m0, m1, kinetic(v0, v1, m0, m1) + k.gm1inv * p};
 }
 
 // m va + p [the axis is AX]
@@ -89,17 +90,15 @@ template <bool ON, class R> __device__ __forceinline__ R mome_flux(R m, R va, R 
   return ON ? m * va + p : plus_none(m * va, p);
 }
 
-// fluxes along axis AX of a primitive record
+// fluxes along axis AX of a primitive record with momenta and energy c
 template <int AX, class R>
-__device__ __forceinline__ Flux<R> flux_prim(const Gas<R> &k, R rho, R v0, R v1, R p) {
-  const R m0 = rho * v0, m1 = rho * v1;
-  const R e = kinetic(v0, v1, m0, m1) + k.gm1inv * p;
-  const R h = e + p;
+__device__ __forceinline__ Flux<R> flux_prim(const Cons<R> &c, R v0, R v1, R p) {
+  const R h = c.e + p;
   const R va = AX == 0 ? v0 : v1;
   Flux<R> f;
-  f.fd = AX == 0 ? m0 : m1;
-  f.fm0 = mome_flux<AX == 0>(m0, va, p);
-  f.fm1 = mome_flux<AX == 1>(m1, va, p);
+  f.fd = AX == 0 ? c.m0 : c.m1;
+  f.fm0 = mome_flux<AX == 0>(c.m0, va, p);
+  f.fm1 = mome_flux<AX == 1>(c.m1, va, p);
   f.fe = h * va;
   return f;
 }
@@ -133,23 +132,34 @@ template <class R> __device__ __forceinline__ R hllc_q(const Gas<R> &k, R sp, R 
 
 template <int AX, class R>
 __device__ __forceinline__ Flux<R> star_flux(const Gas<R> &k, R sstar, R shock, R rho, R v0, R v1,
-                                             R p) {
+                                             R p, R e) {
   const R speed = AX == 0 ? v0 : v1;
   const R ds = shock - speed;
   const Divisor<R> d(rho);
   const R dens = div(rho * ds, shock - sstar);
   const R mome0 = dens * (AX == 0 ? sstar : v0);
   const R mome1 = dens * (AX == 1 ? sstar : v1);
-  const R e = energy_prim(k, rho, v0, v1, p);
   const R enrg = dens * (d.under(e) + (sstar - speed) * (sstar + div(d.under(p), ds)));
   return flux_cons<AX>(k, dens, mome0, mome1, enrg);
 }
 
+// The momentum along AX of a wall's two states and the momenta and energy of
+// the one whose flux is taken, formed from the states.
+template <int AX, class R> struct WallCons {
+  const Gas<R> &k;
+  const Prim<R> &L, &Rt;
+  __device__ __forceinline__ R momL() const { return L.rho * (AX == 0 ? L.v0 : L.v1); }
+  __device__ __forceinline__ R momR() const { return Rt.rho * (AX == 0 ? Rt.v0 : Rt.v1); }
+  __device__ __forceinline__ Cons<R> side(bool, R rho, R v0, R v1, R p) const {
+    return cons_of(k, rho, v0, v1, p);
+  }
+};
+
 // The wall record's fluxes of hllc i left right (HydroMain.hs:237-268).
-// cl, cr: sound speeds of the two states.
-template <int AX, class R>
+// cl, cr: sound speeds of the two states; C: a WallCons, or what has them ready.
+template <int AX, class R, class C>
 __device__ __forceinline__ Flux<R> hllc(const Gas<R> &k, const Prim<R> &L, R cl,
-                                        const Prim<R> &Rt, R cr) {
+                                        const Prim<R> &Rt, R cr, const C &cons) {
   const R densMid = half(L.rho + Rt.rho);
   const R soundMid = half(cl + cr);
   const R uL = AX == 0 ? L.v0 : L.v1;
@@ -160,7 +170,7 @@ __device__ __forceinline__ Flux<R> hllc(const Gas<R> &k, const Prim<R> &L, R cl,
   const R shockLeft = uL - cl * qL;
   const R shockRight = uR + cr * qR;
   const R dL = shockLeft - uL, dR = shockRight - uR;
-  const R shockStar = div(Rt.p - L.p + L.rho * uL * dL - Rt.rho * uR * dR,
+  const R shockStar = div(Rt.p - L.p + cons.momL() * dL - cons.momR() * dR,
                           L.rho * dL - Rt.rho * dR);
   // select (0 < SL) L (select (0 < S*) L* (select (0 < SR) R* R)): pick the
   // side first, then evaluate one physical or star flux on it, so a warp
@@ -171,8 +181,14 @@ __device__ __forceinline__ Flux<R> hllc(const Gas<R> &k, const Prim<R> &L, R cl,
   const R xr = useL ? L.rho : Rt.rho, x0 = useL ? L.v0 : Rt.v0, x1 = useL ? L.v1 : Rt.v1,
           xp = useL ? L.p : Rt.p;
   const R shock = useL ? shockLeft : shockRight;
-  if (star) return star_flux<AX>(k, shockStar, shock, xr, x0, x1, xp);
-  return flux_prim<AX>(k, xr, x0, x1, xp);
+  const Cons<R> c = cons.side(useL, xr, x0, x1, xp);
+  if (star) return star_flux<AX>(k, shockStar, shock, xr, x0, x1, xp, c.e);
+  return flux_prim<AX>(c, x0, x1, xp);
+}
+template <int AX, class R>
+__device__ __forceinline__ Flux<R> hllc(const Gas<R> &k, const Prim<R> &L, R cl,
+                                        const Prim<R> &Rt, R cr) {
+  return hllc<AX>(k, L, cl, Rt, cr, WallCons<AX, R>{k, L, Rt});
 }
 
 template <class R> __device__ __forceinline__ R absmaller(R a, R b) {
@@ -182,31 +198,33 @@ template <> __device__ __forceinline__ double absmaller(double a, double b) {
   return xf::absmaller(a, b);
 }
 
-// interpolateSingle 2 (minmod MUSCL): face value left (l) and right (r)
+// interpolateSingle 2 (minmod MUSCL): face value left (l) and right (r) of the
+// wall between x1 and x2, from the differences of four neighbours
 template <class R>
-__device__ __forceinline__ void muscl(R x0, R x1, R x2, R x3, R &l, R &r) {
-  const R d01 = x1 - x0, d12 = x2 - x1, d23 = x3 - x2;
+__device__ __forceinline__ void muscl_of(R x1, R x2, R d01, R d12, R d23, R &l, R &r) {
   const R d1 = absmaller(d01, d12);
   const R d2 = absmaller(d12, d23);
   l = x1 + half(d1);
   r = x2 - half(d2);
+}
+template <class R>
+__device__ __forceinline__ void muscl(R x0, R x1, R x2, R x3, R &l, R &r) {
+  muscl_of(x1, x2, x1 - x0, x2 - x1, x3 - x2, l, r);
 }
 
 // Conservative update of base state b by the axis-1 walls, then the axis-0
 // walls (foldl1 (.) over the axes applies axis 1 first), then
 // bindPrimitive (max 1e-2 rho) v (max 1e-2 p).  cons (optional): the new
 // conserved state (rho, m0, m1, E) before the primitive recovery.
+// rho, c: of the base state.
 template <class R>
-__device__ __forceinline__ Prim<R> update(const Gas<R> &k, const Prim<R> &b, R dtdx0, R dtdx1,
-                                          const Flux<R> &l0, const Flux<R> &r0,
-                                          const Flux<R> &l1, const Flux<R> &r1,
-                                          R *cons = nullptr) {
-  const R m0 = b.rho * b.v0, m1 = b.rho * b.v1;
-  const R e = kinetic(b.v0, b.v1, m0, m1) + k.gm1inv * b.p;
-  const R d1 = b.rho + dtdx1 * (l1.fd - r1.fd);
-  const R a0 = m0 + dtdx1 * (l1.fm0 - r1.fm0);
-  const R a1 = m1 + dtdx1 * (l1.fm1 - r1.fm1);
-  const R e1 = e + dtdx1 * (l1.fe - r1.fe);
+__device__ __forceinline__ Prim<R> update_cons(const Gas<R> &k, R rho, const Cons<R> &c, R dtdx0,
+                                               R dtdx1, const Flux<R> &l0, const Flux<R> &r0,
+                                               const Flux<R> &l1, const Flux<R> &r1, R *cons) {
+  const R d1 = rho + dtdx1 * (l1.fd - r1.fd);
+  const R a0 = c.m0 + dtdx1 * (l1.fm0 - r1.fm0);
+  const R a1 = c.m1 + dtdx1 * (l1.fm1 - r1.fm1);
+  const R e1 = c.e + dtdx1 * (l1.fe - r1.fe);
   const R d2 = d1 + dtdx0 * (l0.fd - r0.fd);
   const R b0 = a0 + dtdx0 * (l0.fm0 - r0.fm0);
   const R b1 = a1 + dtdx0 * (l0.fm1 - r0.fm1);
@@ -226,6 +244,14 @@ __device__ __forceinline__ Prim<R> update(const Gas<R> &k, const Prim<R> &b, R d
   q.v1 = v1;
   q.p = omax(R(1e-2), pn);
   return q;
+}
+template <class R>
+__device__ __forceinline__ Prim<R> update(const Gas<R> &k, const Prim<R> &b, R dtdx0, R dtdx1,
+                                          const Flux<R> &l0, const Flux<R> &r0,
+                                          const Flux<R> &l1, const Flux<R> &r1,
+                                          R *cons = nullptr) {
+  return update_cons(k, b.rho, cons_of(k, b.rho, b.v0, b.v1, b.p), dtdx0, dtdx1, l0, r0, l1, r1,
+                     cons);
 }
 
 // per-cell CFL timescale min_i dR_i / (c + |v_i|)   (HydroMain.hs:150-153)

@@ -486,6 +486,7 @@ om_status hydro_setup(Handle *h) {
       return OM_ERR_NOMEM;
     }
     for (int i = 1; i < 4; ++i) st->q.q[i] = (char *)st->q.q[0] + pitch * i;
+    hydro_f64_tile(st->q, h->size[0], h->size[1], h->device);
   }
   if (cudaMalloc(&st->d_ts, cells * es) != cudaSuccess ||
       cudaMalloc(&st->d_min, sizeof(unsigned long long)) != cudaSuccess ||

@@ -59,25 +59,49 @@ cudaError_t hydro_fused_tape_exact(int fp64, const HydroStepArgs &a, const Hydro
   return fp64 ? launch_tape<double>(a, t, s) : launch_tape<float>(a, t, s);
 }
 
-// The FP64 step as two kernels on 16 x 16 tiles: small tiles spread a grid
-// evenly over the SMs, whose double pipes are what bounds it (384 x 256 is 192
-// tiles of 32 x 16: some SMs had twice the work of others).
+// The tile of an FP64 step: what its double operations cost on the SM that gets
+// most tiles, in thousands, is least (the counts are those of the two kernels;
+// 4000 stand for a tile's start and its barriers: 8 x 8 tiles of a large grid
+// were 30 % slower than 16 x 16).  Large grids take 16 x 16; 384 x 256 takes 448
+// tiles of 14 x 16, three to an SM, 116 us a step where 384 of 16 x 16 take 131;
+// 256 x 256 115 us and not 129, 100 x 80 (7 x 8) 33 and not 57, 40 x 40 (4 x 4) 31
+// and not 59.
+void hydro_f64_tile(HydroStage1 &q, int n0, int n1, int device) {
+  const long long sms = sm_count(device);
+  double best = 0;
+  for (int th = kF64Tile; th >= 4; --th)
+    for (int tw = kF64Tile; tw >= 4; --tw) {
+      const long long tiles =
+          (long long)((n0 + tw - 1) / tw) * ((n1 + th - 1) / th);
+      const int walls = (tw + 1) * th + (th + 1) * tw;
+      const double ops = 115.0 * walls + 68.0 * tw * th + 8.0 * (tw + 2) * (th + 2) +
+                         4.0 * ((tw + 3) * th + (th + 3) * tw) + 4000.0;
+      const double cost = (double)((tiles + sms - 1) / sms) * ops;
+      if (best == 0 || cost < best) {
+        best = cost;
+        q.tw = tw;
+        q.th = th;
+      }
+    }
+  for (int k = 0; k < 5; ++k) q.inv[k] = 65535u / (unsigned)(q.tw + k) + 1;
+}
+
 template <bool OPEN>
 static cudaError_t launch_f64(const HydroStepArgs &a0, const HydroStage1 &q, cudaStream_t s) {
-  constexpr int TX = 16, TY = 16, NT = 256, e = OPEN ? 2 : 0;
+  constexpr int NT = 256, e = OPEN ? 2 : 0;
   HydroStepArgs a = a0;
-  a.nt0 = (a.n0 + 2 * e + TX - 1) / TX;
-  const int nt1 = (a.n1 + 2 * e + TY - 1) / TY;
-  cudaError_t err = launch_step(hydro_stage1_kernel<double, TX, TY, NT, OPEN>, a.nt0 * nt1, NT,
-                                sizeof(Stage1Smem<double, TX, TY>), s, a, q);
+  a.nt0 = (a.n0 + 2 * e + q.tw - 1) / q.tw;
+  const int nt1 = (a.n1 + 2 * e + q.th - 1) / q.th;
+  cudaError_t err = launch_step(hydro_stage1_kernel<double, NT, OPEN>, a.nt0 * nt1, NT,
+                                sizeof(Stage1Smem<double>), s, a, q);
   if (err != cudaSuccess) return err;
-  a.nt0 = (a.n0 + TX - 1) / TX;
-  const size_t smem = sizeof(Stage2Smem<double, TX, TY>);
-  err = cudaFuncSetAttribute(hydro_stage2_kernel<double, TX, TY, NT, OPEN>,
+  a.nt0 = (a.n0 + q.tw - 1) / q.tw;
+  constexpr size_t smem = sizeof(Stage2Smem<double>);
+  err = cudaFuncSetAttribute(hydro_stage2_kernel<double, NT, OPEN>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return err;
-  return launch_step(hydro_stage2_kernel<double, TX, TY, NT, OPEN>,
-                     a.nt0 * ((a.n1 + TY - 1) / TY), NT, smem, s, a, q);
+  return launch_step(hydro_stage2_kernel<double, NT, OPEN>, a.nt0 * ((a.n1 + q.th - 1) / q.th), NT,
+                     smem, s, a, q);
 }
 
 // a.lm > 0: open grid (margins, jet boundary condition)

@@ -199,12 +199,12 @@ template <class R> __device__ __forceinline__ R step_dt(const HydroStepArgs &a) 
 // The margin cells of an open grid beside the tile at (X0, Y0) are set to 0:
 // the generated class copies whole manifests, whose margins are zero, into the
 // statics.
-template <class R, int TX, int TY>
-__device__ __forceinline__ void clear_margins(const HydroStepArgs &a, int X0, int Y0,
-                                              R *const (&out)[4], int tid, int threads) {
+template <class R>
+__device__ __forceinline__ void clear_margins(const HydroStepArgs &a, int X0, int Y0, int tw,
+                                              int th, R *const (&out)[4], int tid, int threads) {
   const int n0 = a.n0, n1 = a.n1, lm = a.lm;
-  const int xa = X0 == 0 ? -lm : X0, xb = X0 + TX >= n0 ? n0 + lm : X0 + TX;
-  const int ya = Y0 == 0 ? -lm : Y0, yb = Y0 + TY >= n1 ? n1 + lm : Y0 + TY;
+  const int xa = X0 == 0 ? -lm : X0, xb = X0 + tw >= n0 ? n0 + lm : X0 + tw;
+  const int ya = Y0 == 0 ? -lm : Y0, yb = Y0 + th >= n1 ? n1 + lm : Y0 + th;
   if (xa >= 0 && ya >= 0 && xb <= n0 && yb <= n1) return;
   const int w = xb - xa, cnt = w * (yb - ya);
   for (int i = tid; i < cnt; i += threads) {
@@ -494,7 +494,7 @@ __device__ __forceinline__ void fused_tile(const HydroStepArgs &a, int tile,
   }
   if (OPEN) {
     R *out[4] = {(R *)a.nrho, (R *)a.nv0, (R *)a.nv1, (R *)a.np};
-    hk::clear_margins<R, TX, TY>(a, X0, Y0, out, tid, NT);
+    hk::clear_margins<R>(a, X0, Y0, TX, TY, out, tid, NT);
   }
   hk::block_min_to(m, ts_at(a, a.ts_write), red);
   hk::step_end<R, OPEN>(a, tile, dtG);
@@ -517,15 +517,24 @@ hydro_fused_kernel(HydroStepArgs a) {
 // 1.4 stage-1 cells per cell of a 32 x 16 tile.  Here every cell is advanced
 // once and the walls of a tile's edge twice (2.1 per cell and stage), for 64
 // bytes more per cell, which cost nothing beside that.  1024^2 open: 1.17 ms a
-// step fused, 0.92 so; 384 x 256: 175 us, 141.  16 x 16 tiles by 256 threads:
-// smaller tiles repeat more walls (16 x 8 and 8 x 8 were 10 and 30 % slower),
-// 128 threads leave a small grid too few warps (384 x 256: 206 us).  With a
-// part or all of the products formed on the integer pipes too, the step was 4
-// to 27 % slower: the double instructions' issue gaps are not free.
+// step fused, 0.92 so, 0.85 with the momenta, energies and differences that
+// several walls use formed per cell; 384 x 256: 175 us, 140, 132, and 116 with
+// tiles that suit the grid (hydro_f64_tile).  256 threads: 128 leave a small
+// grid too few warps (384 x 256: 206 us against 141).  With a part or all of the
+// products formed on the integer pipes too, the step was 4 to 27 % slower: the
+// double instructions' issue gaps are not free.
 // ---------------------------------------------------------------------------
 struct HydroStage1 {
-  void *q[4];  // stage-1 state, memory-sized arrays
+  void *q[4];       // stage-1 state, memory-sized arrays
+  int tw, th;       // tile, at most kF64Tile a side
+  unsigned inv[5];  // 65535 / (tw + k) + 1
+  // i / (tw + k) for i < 2000 (exact: the excess of inv over 2^16 / (tw + k)
+  // times i stays below 2^16)
+  __device__ __forceinline__ int row(int i, int k) const {
+    return (int)((unsigned)i * inv[k] >> 16);
+  }
 };
+constexpr int kF64Tile = 16;
 
 namespace hk {
 // What a block's threads share of the quotients that are the same for all of
@@ -539,7 +548,8 @@ template <class R> struct alignas(16) StageConsts {
 };
 }  // namespace hk
 
-template <class R, int TX, int TY> struct Stage1Smem {
+template <class R> struct Stage1Smem {
+  static constexpr int TX = kF64Tile, TY = kF64Tile;
   static constexpr int PX = TX + 2, PY = TY + 2;
   hk::StageConsts<R> c;
   R P[4][PY][PX];
@@ -559,7 +569,8 @@ template <class R, int TX, int TY> struct Stage1Smem {
     }
   };
 };
-template <class R, int TX, int TY> struct Stage2Smem {
+template <class R> struct Stage2Smem {
+  static constexpr int TX = kF64Tile, TY = kF64Tile;
   static constexpr int QX = TX + 4, QY = TY + 4;
   hk::StageConsts<R> c;
   R Q[4][QY][QX];
@@ -572,25 +583,26 @@ template <class R, int TX, int TY> struct Stage2Smem {
 // Stage 1 of the cells [-e, n + e) of both axes (e = 2 on an open grid, whose
 // margin cells step from the jet state; else 0); a.nt0 tiles along x of that
 // range.
-template <class R, int TX, int TY, int NT, bool OPEN>
+template <class R, int NT, bool OPEN>
 __global__ void __launch_bounds__(NT)
 hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
-  using S = Stage1Smem<R, TX, TY>;
+  using S = Stage1Smem<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   S &s = *reinterpret_cast<S *>(smem_raw);
   hk::step_begin();
   const int tid = threadIdx.x, tile = blockIdx.x;
   const int t0 = tile % a.nt0, t1 = tile / a.nt0;
   constexpr int e = OPEN ? 2 : 0;
-  const int X0 = t0 * TX - e, Y0 = t1 * TY - e;
+  const int tw = o.tw, th = o.th;
+  const int X0 = t0 * tw - e, Y0 = t1 * th - e;
   const int n0 = a.n0, n1 = a.n1;
   const R g = hk::Reals<R>::gamma(a);
   const R dR0 = hk::Reals<R>::dR0(a.sc), dR1 = hk::Reals<R>::dR1(a.sc);
   if (tid == 0) s.c = hk::StageConsts<R>(g, hk::step_dt<R>(a) / R(2), dR0, dR1);
   const R *f[4] = {(const R *)a.rho, (const R *)a.v0, (const R *)a.v1, (const R *)a.p};
-  const bool near = n0 >= TX + 2 && n1 >= TY + 2;
-  for (int i = tid; i < S::PY * S::PX; i += NT) {
-    const int py = i / S::PX, px = i - py * S::PX;
+  const bool near = n0 >= tw + 2 && n1 >= th + 2;
+  for (int i = tid; i < (th + 2) * (tw + 2); i += NT) {
+    const int py = o.row(i, 2), px = i - py * (tw + 2);
     const int ix = X0 + px - 1, iy = Y0 + py - 1;
     hs::Prim<R> w;
     if (OPEN) {
@@ -617,8 +629,8 @@ hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
   auto cell = [&](int py, int px) {
     return hs::Prim<R>{s.P[0][py][px], s.P[1][py][px], s.P[2][py][px], s.P[3][py][px]};
   };
-  for (int i = tid; i < S::PY * S::PX; i += NT) {
-    const int py = i / S::PX, px = i - py * S::PX;
+  for (int i = tid; i < (th + 2) * (tw + 2); i += NT) {
+    const int py = o.row(i, 2), px = i - py * (tw + 2);
     const hs::Prim<R> w = cell(py, px);
     const hs::Cons<R> c = hs::cons_of(k, w.rho, w.v0, w.v1, w.p);
     s.M[0][py][px] = c.m0;
@@ -626,15 +638,15 @@ hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
     s.M[2][py][px] = c.e;
   }
   __syncthreads();
-  constexpr int NX = TY * (TX + 1), NY = (TY + 1) * TX;
+  const int NX = th * (tw + 1), NY = (th + 1) * tw;
   for (int i = tid; i < NX + NY; i += NT) {
     if (i < NX) {
-      const int sy = i / (TX + 1), sx = i - sy * (TX + 1);
+      const int sy = o.row(i, 1), sx = i - sy * (tw + 1);
       s.fx[i] = hs::hllc<0>(k, cell(sy + 1, sx), s.C[sy + 1][sx], cell(sy + 1, sx + 1),
                             s.C[sy + 1][sx + 1],
                             typename S::template Wall<0>{&s.M[0][sy + 1][sx], 1});
     } else {
-      const int j = i - NX, sy = j / TX, sx = j - sy * TX;
+      const int j = i - NX, sy = o.row(j, 0), sx = j - sy * tw;
       s.fy[j] = hs::hllc<1>(k, cell(sy, sx + 1), s.C[sy][sx + 1], cell(sy + 1, sx + 1),
                             s.C[sy + 1][sx + 1],
                             typename S::template Wall<1>{&s.M[0][sy][sx + 1], S::PX});
@@ -642,14 +654,14 @@ hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
   }
   __syncthreads();
   const R dtdx0 = s.c.dtdx0, dtdx1 = s.c.dtdx1;
-  for (int i = tid; i < TY * TX; i += NT) {
-    const int oy = i / TX, ox = i - oy * TX;
+  for (int i = tid; i < th * tw; i += NT) {
+    const int oy = o.row(i, 0), ox = i - oy * tw;
     const int iy = Y0 + oy, ix = X0 + ox;
     if (iy >= n1 + e || ix >= n0 + e) continue;
     const hs::Cons<R> c{s.M[0][oy + 1][ox + 1], s.M[1][oy + 1][ox + 1], s.M[2][oy + 1][ox + 1]};
     const hs::Prim<R> q = hs::update_cons<R>(
-        k, s.P[0][oy + 1][ox + 1], c, dtdx0, dtdx1, s.fx[oy * (TX + 1) + ox],
-        s.fx[oy * (TX + 1) + ox + 1], s.fy[oy * TX + ox], s.fy[(oy + 1) * TX + ox], nullptr);
+        k, s.P[0][oy + 1][ox + 1], c, dtdx0, dtdx1, s.fx[oy * (tw + 1) + ox],
+        s.fx[oy * (tw + 1) + ox + 1], s.fy[oy * tw + ox], s.fy[(oy + 1) * tw + ox], nullptr);
     const size_t gi = OPEN ? (size_t)(iy + a.lm) * a.ms0 + (ix + a.lm) : (size_t)iy * n0 + ix;
     ((R *)o.q[0])[gi] = q.rho;
     ((R *)o.q[1])[gi] = q.v0;
@@ -659,24 +671,26 @@ hydro_stage1_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
 }
 
 // Stage 2, the new state and its CFL minimum.
-template <class R, int TX, int TY, int NT, bool OPEN>
+template <class R, int NT, bool OPEN>
 __global__ void __launch_bounds__(NT)
 hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
-  using S = Stage2Smem<R, TX, TY>;
+  using S = Stage2Smem<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned long long red[32];
   S &s = *reinterpret_cast<S *>(smem_raw);
   hk::step_begin();
+  constexpr int T = kF64Tile;
   const int tid = threadIdx.x, tile = blockIdx.x;
   const int t0 = tile % a.nt0, t1 = tile / a.nt0;
-  const int X0 = t0 * TX, Y0 = t1 * TY;
+  const int tw = o.tw, th = o.th;
+  const int X0 = t0 * tw, Y0 = t1 * th;
   const int n0 = a.n0, n1 = a.n1, lm = a.lm;
   const R dR0 = hk::Reals<R>::dR0(a.sc), dR1 = hk::Reals<R>::dR1(a.sc);
   const R dtG = hk::step_dt<R>(a);
   if (tid == 0) s.c = hk::StageConsts<R>(hk::Reals<R>::gamma(a), dtG, dR0, dR1);
-  const bool near = n0 >= TX + 4 && n1 >= TY + 4;
-  for (int i = tid; i < S::QY * S::QX; i += NT) {
-    const int qy = i / S::QX, qx = i - qy * S::QX;
+  const bool near = n0 >= tw + 4 && n1 >= th + 4;
+  for (int i = tid; i < (th + 4) * (tw + 4); i += NT) {
+    const int qy = o.row(i, 4), qx = i - qy * (tw + 4);
     const int ix = X0 + qx - 2, iy = Y0 + qy - 2;
     size_t gi;
     if (OPEN) {  // rows and columns beyond the last margin cell feed no cell
@@ -690,10 +704,10 @@ hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
     for (int c = 0; c < 4; ++c) s.Q[c][qy][qx] = ((const R *)o.q[c])[gi];
   }
   __syncthreads();
-  for (int i = tid; i < TY * (TX + 3) + (TY + 3) * TX; i += NT) {
-    const bool x = i < TY * (TX + 3);
-    const int j = x ? i : i - TY * (TX + 3), r = x ? j / (TX + 3) : j / TX,
-              q = x ? j - r * (TX + 3) : j - r * TX;
+  for (int i = tid; i < th * (tw + 3) + (th + 3) * tw; i += NT) {
+    const bool x = i < th * (tw + 3);
+    const int j = x ? i : i - th * (tw + 3), r = o.row(j, x ? 3 : 0),
+              q = j - r * (x ? tw + 3 : tw);
     const int y0 = x ? r + 2 : r, x0 = x ? q : q + 2;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -703,14 +717,14 @@ hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
   }
   __syncthreads();
   const hs::Gas<R> k = s.c.gas;
-  constexpr int NX = TY * (TX + 1), NY = (TY + 1) * TX;
+  const int NX = th * (tw + 1), NY = (th + 1) * tw;
   for (int i = tid; i < NX + NY; i += NT) {
     const bool x = i < NX;
     const int j = x ? i : i - NX;
-    const int sy = x ? j / (TX + 1) : j / TX, sx = x ? j - sy * (TX + 1) : j - sy * TX;
+    const int sy = o.row(j, x ? 1 : 0), sx = j - sy * (x ? tw + 1 : tw);
     // the wall lies between cells 1 and 2 of four along its axis
     const int qy = x ? sy + 2 : sy + 1, qx = x ? sx + 1 : sx + 2, dy = x ? 0 : 1, dx = x ? 1 : 0;
-    const int step = x ? 1 : TX, field = x ? TY * (TX + 3) : (TY + 3) * TX;
+    const int step = x ? 1 : T, field = x ? T * (T + 3) : (T + 3) * T;
     const R *d = x ? &s.dx[0][sy][sx] : &s.dy[0][sy][sx];
     hs::Prim<R> L, Rt;
 #pragma unroll
@@ -726,15 +740,15 @@ hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
   const R dtdx0 = s.c.dtdx0, dtdx1 = s.c.dtdx1;
   const R *f[4] = {(const R *)a.rho, (const R *)a.v0, (const R *)a.v1, (const R *)a.p};
   R *out[4] = {(R *)a.nrho, (R *)a.nv0, (R *)a.nv1, (R *)a.np};
-  for (int i = tid; i < TY * TX; i += NT) {
-    const int oy = i / TX, ox = i - oy * TX;
+  for (int i = tid; i < th * tw; i += NT) {
+    const int oy = o.row(i, 0), ox = i - oy * tw;
     const int gy = Y0 + oy, gx = X0 + ox;
     if (gy >= n1 || gx >= n0) continue;
     const size_t gi = OPEN ? (size_t)(gy + lm) * a.ms0 + (gx + lm) : (size_t)gy * n0 + gx;
     const hs::Prim<R> b{f[0][gi], f[1][gi], f[2][gi], f[3][gi]};
-    const hs::Prim<R> q = hs::update(k, b, dtdx0, dtdx1, s.fx[oy * (TX + 1) + ox],
-                                     s.fx[oy * (TX + 1) + ox + 1], s.fy[oy * TX + ox],
-                                     s.fy[(oy + 1) * TX + ox]);
+    const hs::Prim<R> q = hs::update(k, b, dtdx0, dtdx1, s.fx[oy * (tw + 1) + ox],
+                                     s.fx[oy * (tw + 1) + ox + 1], s.fy[oy * tw + ox],
+                                     s.fy[(oy + 1) * tw + ox]);
     out[0][gi] = q.rho;
     out[1][gi] = q.v0;
     out[2][gi] = q.v1;
@@ -743,7 +757,7 @@ hydro_stage2_kernel(HydroStepArgs a, const __grid_constant__ HydroStage1 o) {
         hk::ts_bits<R>(hs::timescale(k.g, dR0, dR1, q.rho, q.v0, q.v1, q.p));
     m = bits < m ? bits : m;
   }
-  if (OPEN) hk::clear_margins<R, TX, TY>(a, X0, Y0, out, tid, NT);
+  if (OPEN) hk::clear_margins<R>(a, X0, Y0, tw, th, out, tid, NT);
   hk::block_min_to(m, ts_at(a, a.ts_write), red);
   hk::step_end<R, OPEN>(a, tile, dtG);
 }

@@ -164,6 +164,9 @@ om_status om_ensemble_create(int count, const int *sizes, const om_config *cfg,
     for (int k = 0; k < count; ++k)
       if (!hydro_persist_fits(sizes[2 * k], sizes[2 * k + 1])) {
         if (hydro_tile_takes_any(E->tile) && hydro_persist_any(sizes[2 * k], sizes[2 * k + 1]))
+          // (8 instances of 64 to 200 cells a side, multiples of 4: 13.7 us a
+          // step against 13.9 with 32 x 32 tiles; 13 of 212 to 276 31.1 against
+          // 34.9; 64 of 256 to 2048 2.31 ms against 3.05)
           E->general = true;
         else
           E->tile = kTile32x32;
@@ -172,13 +175,6 @@ om_status om_ensemble_create(int count, const int *sizes, const om_config *cfg,
     long long items = 0;
     for (int k = 0; k < count; ++k) items += (long long)((sizes[2 * k] + 31) / 32) * ((sizes[2 * k + 1] + 31) / 32);
     if (hydro_persist_form_for(2, items, c.device, c.grid_limit) != 2) E->tile = kPair32x32;
-    // partial tiles pay from about eight tiles per SM on, as on single grids (64
-    // instances of 256 to 2048, multiples of 4: 2.79 ms a step against 3.14; 8 of
-    // 64 to 200: 14.6 us against 14.0)
-    if (E->general && items < 8LL * sm_count(c.device) && c.grid_limit == 0) {
-      E->tile = kTile32x32;
-      E->general = false;
-    }
   }
   hydro_tile_dims(E->tile, &E->tx, &E->ty);
   E->gamma = c.gamma;

@@ -169,19 +169,24 @@ cudaError_t hydro_fused_tape(int fp64, bool exact, const HydroStepArgs &a0, cons
 //   256^2  11.4, 32 x 16 by 1024 5.56, by 512 11.6, 32 x 8 by 512 7.5
 //   384 x 256 (192 tiles of 32 x 16 on 152 SMs)  12.0, by 512 8.2, by 1024 9.3
 //   500 x 300 (304)  12.2, by 512 8.5, by 1024 9.8
-//   512^2 (512)  persistent 12.3, 32 x 16 by 512 13.3
-//   500 x 700 (704, not persistent)  17.6, 32 x 16 by 512 15.9
-//   1000 x 700 (1408)  27.4, 32 x 16 by 512 28.4
+//   560 x 400 (450)  32 x 32 11.8, persistent 11.2, 32 x 16 by 512 10.4
+//   600 x 400 (475: more than three to an SM)  12.0, 11.2, 13.1
+//   700 x 500 (704)  17.4, 14.7, 16.1;  900 x 500 (928)  21.2, 19.4
+//   1000 x 700 (1408)  26.8, 25.6, 28.4;  1200 x 900  40.3, 36.4
+//   1500 x 1100  55.5, 47.7;  3000 x 2500  245, 205
+// Rows that are no multiples of 4 cells go cell by cell or in pairs into the
+// persistent kernel's boxes, which costs what it gains: 1501 x 1100 55.9 with
+// 32 x 32 tiles, 58.4; 2002 x 1500 100.2, 99.0; 3001 x 2500 246, 257.
 int hydro_step_tile(int tile, int n0, int n1, bool open, int device, int grid_limit) {
   if (grid_limit > 0 || !(open || tile == kPairGroups32x32)) return tile;
   const long long sms = sm_count(device);
   auto tiles = [&](int tx, int ty) { return (long long)((n0 + tx - 1) / tx) * ((n1 + ty - 1) / ty); };
   if (!open && tiles(16, 8) <= sms) return kThin16x8;
   if (tiles(32, 16) <= sms) return kThin32x16;
-  if (tiles(32, 16) <= 2 * sms) return kThin32x16h;
-  if (open || hydro_persist_fits(n0, n1)) return tile;
-  if (tiles(32, 16) <= 6 * sms) return kThin32x16h;
-  return hydro_persist_partial(n0, n1, device) ? tile : kTile32x32;
+  if (tiles(32, 16) <= (open ? 2 : 3) * sms) return kThin32x16h;
+  if (open || hydro_persist_any(n0, n1)) return tile;
+  if (tiles(32, 32) <= 2 * sms) return kTile32x32;
+  return tiles(32, 16) <= 6 * sms ? kThin32x16h : kTile32x32;
 }
 
 cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaStream_t s,

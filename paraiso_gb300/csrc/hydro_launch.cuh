@@ -105,9 +105,8 @@ cudaError_t hydro_ensemble_f32(const HydroStepArgs *args, const int *prefix, int
 // sides are multiples of 32 and at least 64 (periodic)
 bool hydro_persist_fits(int n0, int n1);
 // and, in its paired forms, sides of any size from 64 with rows of a multiple
-// of 4 cells (partial tiles); `partial` also says whether it is worth it
+// of 4 cells (partial tiles)
 bool hydro_persist_any(int n0, int n1);
-bool hydro_persist_partial(int n0, int n1, int device);
 inline bool hydro_tile_takes_any(int tile) {
   return tile == kPair32x32 || tile == kPairGroups32x32;
 }

@@ -27,17 +27,6 @@ bool hydro_persist_fits(int n0, int n1) {
   return n0 % hp::TX == 0 && n1 % hp::TY == 0 && n0 >= 2 * hp::TX && n1 >= 2 * hp::TY;
 }
 
-// The partial tiles of such a grid cost it a few per cent: 1000 x 700 (704
-// tiles) takes 30.9 us a step against 28.4 with the tile kernel, 1500 x 1100
-// (1645) 57.8 against 59.3, 3000 x 2500 244.7 against 257.1, 4000^2 488 against
-// 529.  Rows that TMA cannot take, and open grids, were slower copied cell by
-// cell than with the tile kernel at every size (3001 x 2500: 265.6 against
-// 257.5; open 4000^2: 552 against 541).
-bool hydro_persist_partial(int n0, int n1, int device) {
-  const long long tiles =
-      (long long)((n0 + hp::TX - 1) / hp::TX) * ((n1 + hp::TY - 1) / hp::TY);
-  return hydro_persist_any(n0, n1) && tiles >= 8LL * sm_count(device);
-}
 bool hydro_persist_any(int n0, int n1) {
   return n0 % 4 == 0 && n0 >= 2 * hp::TX && n1 >= 2 * hp::TY;
 }

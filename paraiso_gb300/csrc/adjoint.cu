@@ -51,7 +51,7 @@ template <class R> struct Fields {
   }
 };
 
-// Indices reach at most a tile (32 x 16) plus 3 cells beyond the mesh; with
+// Indices reach at most a tile (32 x 15) plus 3 cells beyond the mesh; with
 // both extents at least this, a single add or subtract wraps them.
 constexpr int kCheapWrap = 40;
 
@@ -156,10 +156,15 @@ __device__ __forceinline__ double block_sum_of(const double *x, int n, double *s
   return block_sum(acc, sh);
 }
 
-// Tile shapes of the tile kernels
+// Tile shapes of the stage-2 (TX x TY) and stage-1 (TX x TY1) kernels.  A phase
+// ends when the warps with most of its faces are through: of 16 rows, the 17.5
+// and 19 warps' worth of x and y faces of stage 2 and the 33.5 of stage 1 took
+// the 8 warps three, three and five rounds; 13 rows make them 14.2 and 16, two
+// rounds each, 15 rows 31.5, four.  1024^2, 200 steps: 46.9 ms with 16 rows, 45.8
+// so (12 and 14 rows of stage 2: 46.7, 45.8; 9: 48.3).
 template <class R> struct AdjTile;
-template <> struct AdjTile<float> { static constexpr int TX = 32, TY = 16; };
-template <> struct AdjTile<double> { static constexpr int TX = 32, TY = 8; };
+template <> struct AdjTile<float> { static constexpr int TX = 32, TY = 13, TY1 = 15; };
+template <> struct AdjTile<double> { static constexpr int TX = 32, TY = 8, TY1 = 8; };
 
 __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
   for (int o = 16; o > 0; o >>= 1) {
@@ -661,7 +666,7 @@ struct AdjointScratch {
   double *partials = nullptr;
   unsigned long long *argmin = nullptr;
   int nparts = 0;   // blocks of the grid-stride kernels
-  int ntiles = 0;   // tiles of the reverse kernels (one dt partial each)
+  int ntiles = 0;   // tiles of the stage-2 kernel (one dt partial each)
   std::vector<void *> all;
 };
 
@@ -684,14 +689,14 @@ static std::vector<std::pair<Handle *, AdjointScratch *>> g_scratch;
 static std::mutex g_scratch_mu;
 
 template <class R> static cudaError_t allow_tile_smem() {
-  constexpr int TX = adj::AdjTile<R>::TX, TY = adj::AdjTile<R>::TY;
+  constexpr int TX = adj::AdjTile<R>::TX, TY = adj::AdjTile<R>::TY, TY1 = adj::AdjTile<R>::TY1;
   const cudaError_t e = cudaFuncSetAttribute(adj::adj_stage2_tile<R, TX, TY>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(adj::Stage2Smem<R, TX, TY>));
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(adj::adj_stage1_tile<R, TX, TY>,
+  return cudaFuncSetAttribute(adj::adj_stage1_tile<R, TX, TY1>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(adj::Stage1Smem<R, TX, TY>));
+                              (int)sizeof(adj::Stage1Smem<R, TX, TY1>));
 }
 
 static om_status get_scratch(Handle *h, int fp64, AdjointScratch **out) {
@@ -806,7 +811,8 @@ static om_status vjp_kernels(Handle *h, AdjointScratch *s, const adj::StepIn *re
   adj::Geo<R> G{h->size[0], h->size[1], (R)h->cfg.gamma, (R)hs_->dR0, (R)hs_->dR1, R(0), rec,
                 cheap};
   const int nt = s->ntiles;
-  constexpr int TX = adj::AdjTile<R>::TX, TY = adj::AdjTile<R>::TY;
+  constexpr int TX = adj::AdjTile<R>::TX, TY = adj::AdjTile<R>::TY, TY1 = adj::AdjTile<R>::TY1;
+  const int nt1 = ((G.n0 + TX - 1) / TX) * ((G.n1 + TY1 - 1) / TY1);
   const auto U = F4<R>(ub), U1b = F4<R>(s->u1b), Pbase = F4<R>(s->pbase), Pb = F4<R>(pb_out);
   // argmin[2 par]: arg-min cell, argmin[2 par + 1]: minimum timescale bits
   unsigned long long *am = s->argmin + 2 * par;
@@ -818,8 +824,8 @@ static om_status vjp_kernels(Handle *h, AdjointScratch *s, const adj::StepIn *re
   OM_CUDA_CHECK(launch_after(adj::adj_stage2_tile<R, TX, TY>, nt,
                              sizeof(adj::Stage2Smem<R, TX, TY>), st, U, U1b, Pbase, G, part,
                              am + 1, pend));
-  OM_CUDA_CHECK(launch_after(adj::adj_stage1_tile<R, TX, TY>, nt,
-                             sizeof(adj::Stage1Smem<R, TX, TY>), st, U1b, Pbase, Pb, G, am + 1,
+  OM_CUDA_CHECK(launch_after(adj::adj_stage1_tile<R, TX, TY1>, nt1,
+                             sizeof(adj::Stage1Smem<R, TX, TY1>), st, U1b, Pbase, Pb, G, am + 1,
                              am, other));
   h->launches += kVjpLaunches;
   return OM_OK;

@@ -62,15 +62,17 @@ typedef struct {
   int depth;        /* Life: generations per temporally blocked launch (0 = tuned) */
   int tile_x;       /* Life: tile width in 32-cell words; Hydro: tile width in cells (0 = tuned) */
   int tile_y;       /* tile height in cells (0 = tuned; Hydro FP32: 0 = the persistent
-                       32 x 32 kernel on grids whose sides are multiples of 32 and
-                       at least 64 (else the 32 x 32 tile kernel): with tile_x 0
-                       paired, as one CTA per SM of two groups half a tile apart
-                       when every group gets at least 16 tiles, else two CTAs per
-                       SM; with tile_x 16 paired, two CTAs per SM; with tile_x 32
-                       one wall per thread.  8, 16 and 32 with tile_x 0 or 32, 8
+                       32 x 32 kernel on grids of at least 64 cells a side whose
+                       rows are multiples of 4 cells (else the 32 x 32 tile
+                       kernel): with tile_x 0 paired, as one CTA per SM of two
+                       groups half a tile apart when every group gets at least 16
+                       tiles, else two CTAs per SM, and without a grid_limit on
+                       grids that one wave of smaller tiles holds those; with
+                       tile_x 16 paired, two CTAs per SM; with tile_x 32 one wall
+                       per thread (sides that are multiples of 32).  8, 16 and 32 with tile_x 0 or 32, 8
                        and 16 with tile_x 64 are tile kernels; a negative -k
                        selects the column sweep of k rows per chunk, 8 or 16) */
-  int use_graph;    /* capture om_run_n in a CUDA graph (default 1) */
+  int use_graph;    /* capture om_run_n in a CUDA graph when it repeats (default 1) */
   int variant;      /* 0 = fastest path.  Life 1: integer one-cell-per-thread kernel only.
                        Hydro 1: plain unfused FP64-structured grid-stride kernels */
   int life_io;      /* Life cell I/O of the packed kernels: 0 = 128-bit, 1 = 32-bit */
@@ -79,8 +81,12 @@ typedef struct {
                        by TMA and need rows of at least 1024 cells; in 14 and 15
                        each consumer warp synchronises with its two neighbours
                        only); 0 = automatic:
-                       with tile_y 0, that kernel on grids of at least 1.5 of its
-                       tiles per SM, else register-resident blocks */
+                       with tile_y 0, that kernel at the ends of a run on grids of
+                       at least 1.5 of its tiles per SM and register-resident blocks
+                       of packed cells between and on smaller grids.  On grids of
+                       up to 4096 words of 32 cells depth, tile_x, tile_y, life_io,
+                       life_kernel and grid_limit have no effect: what suits the
+                       grid runs, one block for all generations where that is best */
   int grid_limit;   /* persistent kernels (Life warp-specialised, the persistent
                        Hydro FP32 step, Hydro ensembles): at most this many
                        CTAs (0 = as many as the GPU keeps resident) */
@@ -122,7 +128,8 @@ om_status om_kernel_id(om_handle h, const char *name, int *id);
 /* Runs one kernel: `void init()` / `void proceed()` of the generated class. */
 om_status om_run(om_handle h, int kernel_id);
 /* Runs a kernel n times back to back (a driver's step loop), captured in a
- * CUDA graph when cfg.use_graph is set.  Scalars are synced once at the end. */
+ * CUDA graph the second time when cfg.use_graph is set.  Scalars are synced once
+ * at the end. */
 om_status om_run_n(om_handle h, int kernel_id, int n);
 
 /* ---- static variable accessors (PlanTrans.hs:117-157) ------------------ */

@@ -1901,16 +1901,19 @@ static om_status launch_ws_tiles(Handle *h, int v, int io, const void *in, void 
 // Generations per launch at the two ends of a packed run on the
 // warp-specialised kernel: fewer leave it waiting for the cells' 4 bytes each
 // (16384^2 x 100 generations: 1280 us at 8, 1230 at 12, 1176 at 22), more only
-// add halo rows (1189 at 26, 1207 at 30).
+// add halo rows (1189 at 26, 1207 at 30).  These and the block heights' figures
+// were taken with each row's sums formed alone; shared by two rows
+// (life_two_rows), 22 takes 1133.
 static const int kWsEdgeDepth = 22;
 
 // Generations g .. n - 1 of a run through the packed grid.  With every launch
 // reading and writing int32 cells a 16384^2 run of 100 generations moved 9 GB
 // in four launches (1955 us); with the cells read once and written once it
-// takes 1176 us, bound by the ALU's bit operations (76 % of its cycles) between
-// the ends.  2048^2 x 100: 205 -> 128 us.  Rows of 1000 cells (1000 x 700 x
+// takes 1133 us, bound by the ALU's bit operations (78 % of its cycles) between
+// the ends.  2048^2 x 100: 205 -> 102 us.  Rows of 1000 cells (1000 x 700 x
 // 100) no longer take a launch of the one-cell kernel per generation: 496 ->
-// 95 us.
+// 72 us.  A kernel of the warp-specialised form between the ends too was no
+// faster (1144 to 1208 us over its row counts, warps and depths).
 static om_status proceed_packed(Handle *h, int n, int g) {
   LifeState *st = life_state(h);
   if (!st->packed[0]) {

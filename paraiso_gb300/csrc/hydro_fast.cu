@@ -167,11 +167,16 @@ cudaError_t hydro_fused_tape(int fp64, bool exact, const HydroStepArgs &a0, cons
 //   64^2   8.5, 16 x 8 by 256 threads 4.3      100^2 8.3, 4.8
 //   128^2  8.3, 16 x 8 5.65, 32 x 16 by 1024 5.56
 //   256^2  11.4, 32 x 16 by 1024 5.56, by 512 11.6, 32 x 8 by 512 7.5
-//   384 x 256 (192 tiles of 32 x 16 on 152 SMs)  12.0, by 512 8.2, by 1024 9.3
-//   500 x 300 (304)  12.2, by 512 8.5, by 1024 9.8
-//   560 x 400 (450)  32 x 32 11.8, persistent 11.2, 32 x 16 by 512 10.4
+//   384 x 256 (192 tiles of 32 x 16 on 152 SMs)  12.0, by 512 8.9, by 544 7.8
+//   450 x 300 (285)  by 512 10.0, by 544 7.8;  500 x 300 (304)  12.2, 7.7, 7.8
+//   560 x 400 (450)  32 x 32 11.8, persistent 11.2, by 512 10.1, by 544 11.5
+// (544 threads take the walls of stage 2 in two rounds, and two blocks fill an
+// SM; of 512 three do, which evens out only when there are as many.)  Open
+// grids: 384 x 256 by 512 10.3, by 544 8.4; 560 x 400 10.5, 12.4, and 12.9 by
+// 288; larger ones by 288 threads, 701 x 500 15.8, 16.5 by 256, 3001 x 2500 243,
+// 248.
 //   600 x 400 (475: more than three to an SM)  12.0, 11.2, 13.1
-//   700 x 500 (704)  17.4, 14.7, 16.1;  900 x 500 (928)  21.2, 19.4
+//   700 x 500 (704)  17.4, 14.7, by 512 16.1;  900 x 500 (928)  21.2, 19.4
 //   1000 x 700 (1408)  26.8, 25.6, 28.4;  1200 x 900  40.3, 36.4
 //   1500 x 1100  55.5, 47.7;  3000 x 2500  245, 205
 // Rows that are no multiples of 4 cells go cell by cell or in pairs into the
@@ -183,10 +188,11 @@ int hydro_step_tile(int tile, int n0, int n1, bool open, int device, int grid_li
   auto tiles = [&](int tx, int ty) { return (long long)((n0 + tx - 1) / tx) * ((n1 + ty - 1) / ty); };
   if (!open && tiles(16, 8) <= sms) return kThin16x8;
   if (tiles(32, 16) <= sms) return kThin32x16;
-  if (tiles(32, 16) <= (open ? 2 : 3) * sms) return kThin32x16h;
+  if (tiles(32, 16) <= 2 * sms) return kThin32x16h;
+  if (tiles(32, 16) <= 3 * sms) return kThin32x16t;
   if (open || hydro_persist_any(n0, n1)) return tile;
   if (tiles(32, 32) <= 2 * sms) return kTile32x32;
-  return tiles(32, 16) <= 6 * sms ? kThin32x16h : kTile32x32;
+  return tiles(32, 16) <= 6 * sms ? kThin32x16t : kTile32x32;
 }
 
 cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaStream_t s,
@@ -195,13 +201,15 @@ cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaSt
   // an open grid (margins, jet boundary condition) runs 32x16 tiles
   if (a.lm > 0) switch (tile) {
     case kThin32x16: return launch_fast<32, 16, 1024, true>(a, s, grid_out);
-    case kThin32x16h: return launch_fast<32, 16, 512, true>(a, s, grid_out);
-    default: return launch_fast<32, 16, 256, true>(a, s, grid_out);
+    case kThin32x16h: return launch_fast<32, 16, 544, true>(a, s, grid_out);
+    case kThin32x16t: return launch_fast<32, 16, 512, true>(a, s, grid_out);
+    default: return launch_fast<32, 16, 288, true>(a, s, grid_out);
   }
   switch (tile) {
     case kThin16x8: return launch_fast<16, 8, 256>(a, s, grid_out);
     case kThin32x16: return launch_fast<32, 16, 1024>(a, s, grid_out);
-    case kThin32x16h: return launch_fast<32, 16, 512>(a, s, grid_out);
+    case kThin32x16h: return launch_fast<32, 16, 544>(a, s, grid_out);
+    case kThin32x16t: return launch_fast<32, 16, 512>(a, s, grid_out);
     case kPersist32x32:
     case kPair32x32:
     case kPairGroups32x32:

@@ -45,7 +45,10 @@ enum HydroTile {
   // shapes with more threads per cell that the default choice takes on grids
   // too small to fill the GPU (hydro_step_tile): 16 x 8 cells by 256 threads,
   // 32 x 16 by 1024, by 544 and by 512 (three blocks an SM)
-  kThin16x8 = 11, kThin32x16 = 12, kThin32x16h = 13, kThin32x16t = 14
+  kThin16x8 = 11, kThin32x16 = 12, kThin32x16h = 13, kThin32x16t = 14,
+  // and one for large grids that the persistent kernel does not take: 32 x 24 by
+  // 416
+  kLarge32x24 = 15
 };
 // The tile a step of the production build runs: `tile`, but on small grids of
 // the default configuration (kPairGroups32x32, no grid_limit) or with the open

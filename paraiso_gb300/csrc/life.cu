@@ -48,8 +48,9 @@ static const int kHistory = 4096;
 
 struct LifeState {
   bool binary = true;           // every cell is known to be 0 or 1
-  // populations of a run, per generation; all 0 between runs of at most
-  // kHistory generations, whose results go to the host block (pop_clear)
+  // populations of a run, per generation.  pop_clear: the first kHistory of them
+  // are 0, as runs of at most that many generations leave them, whose results
+  // go to the host block; those after may hold an earlier, longer run's
   uint32_t *d_pop = nullptr;
   bool pop_clear = false;
   uint32_t *d_flag = nullptr;   // raised by the cell-value check; [1]: a wait ran out
@@ -2038,7 +2039,7 @@ static om_status life_proceed(Handle *h, int n) {
     st->last_n = n;
     return OM_OK;
   }
-  if (!st->pop_clear)
+  if (!hist || !st->pop_clear)
     OM_CUDA_CHECK(cudaMemsetAsync(st->d_pop, 0, sizeof(uint32_t) * (size_t)std::max(n, kHistory),
                                   h->stream));
   st->pop_clear = false;

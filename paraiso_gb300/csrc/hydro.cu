@@ -64,7 +64,10 @@ static om_status hydro_reserve(Handle *h, int kernel_id, int n) {
     return OM_ERR_NOMEM;
   }
   OM_CUDA_CHECK(cudaStreamSynchronize(h->stream));
-  if (st->d_dt) cudaFree(st->d_dt);
+  if (st->d_dt) {
+    cudaFree(st->d_dt);
+    h->replaced++;
+  }
   st->d_dt = p;
   st->dt_cap = cap;
   return OM_OK;

@@ -1498,7 +1498,10 @@ static om_status life_reserve(Handle *h, int kernel_id, int n) {
     return OM_ERR_NOMEM;
   }
   OM_CUDA_CHECK(cudaStreamSynchronize(h->stream));
-  if (st->d_pop) cudaFree(st->d_pop);
+  if (st->d_pop) {
+    cudaFree(st->d_pop);
+    h->replaced++;
+  }
   st->d_pop = p;
   st->pop_cap = cap;
   st->pop_clear = false;

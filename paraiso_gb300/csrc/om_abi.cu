@@ -192,7 +192,15 @@ struct om_handle_s {
   std::map<std::tuple<int, int, uint64_t>, GraphEntry> graphs;
   // keys run once, by plain launches: a run is captured when it comes again
   std::set<std::tuple<int, int, uint64_t>> once;
+  unsigned replaced = 0;  // h.replaced when the graphs were captured
   int last_launches = 0;
+
+  void drop_graphs() {
+    for (auto &kv : graphs)
+      if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+    graphs.clear();
+    once.clear();
+  }
 };
 
 namespace om {
@@ -312,8 +320,7 @@ om_status om_destroy(om_handle H) {
   Handle *h = &H->h;
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  for (auto &kv : H->graphs)
-    if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+  H->drop_graphs();
   if (h->impl_free) h->impl_free(h);
   for (auto &a : h->arrays) {
     cudaFree(a.dev[0]);
@@ -405,6 +412,10 @@ om_status om_run_n(om_handle H, int kernel_id, int n) {
   if (n < 0) { set_error("om_run_n: n < 0"); return OM_ERR_ARG; }
   if (n == 0) return OM_OK;
   if (h->ops.reserve) OM_TRY(h->ops.reserve(h, kernel_id, n));
+  if (H->replaced != h->replaced) {  // here or in a run that took no graph
+    H->drop_graphs();
+    H->replaced = h->replaced;
+  }
   OM_TRY(prepare(h));
   const bool graph_ok = h->cfg.use_graph && n > 1 && !h->profiling &&
                         (!h->ops.graph_ok || h->ops.graph_ok(h, kernel_id));

@@ -138,6 +138,9 @@ struct Handle {
   KindOps ops;
   int launches = 0;           // kernel launches issued by the current run
   int current_kernel = -1;    // index of the kernel whose function is running
+  // raised when device memory that a run's launches name is replaced: graphs
+  // captured before hold its old address
+  unsigned replaced = 0;
   bool profiling = false;
   bool capturing = false;
   std::vector<ProfPending> prof_pending;

@@ -127,9 +127,11 @@ om_status om_upper_margin(om_handle h, int axis, int *out);
 om_status om_kernel_id(om_handle h, const char *name, int *id);
 /* Runs one kernel: `void init()` / `void proceed()` of the generated class. */
 om_status om_run(om_handle h, int kernel_id);
-/* Runs a kernel n times back to back (a driver's step loop), captured in a
- * CUDA graph the second time when cfg.use_graph is set.  Scalars are synced once
- * at the end. */
+/* Runs a kernel n times back to back (a driver's step loop), with cfg.use_graph
+ * captured in a CUDA graph from the second run of the same kernel and n on (one
+ * graph per buffer and state that such a run starts from: a run that swaps the
+ * buffers an odd number of times replays from the fourth).  Scalars are synced
+ * once at the end. */
 om_status om_run_n(om_handle h, int kernel_id, int n);
 
 /* ---- static variable accessors (PlanTrans.hs:117-157) ------------------ */
@@ -220,6 +222,9 @@ om_status om_hydro_time_tape(om_handle h, int reps, float *ms);
 om_status om_time_run(om_handle h, int kernel_id, int n, float *ms);
 /* Number of kernel launches issued by the last om_run / om_run_n / om_time_run. */
 om_status om_last_launch_count(om_handle h, int *launches);
+/* Number of om_run_n calls of this handle so far that replayed a graph captured
+ * by an earlier one. */
+om_status om_replay_count(om_handle h, long *replays);
 /* Per-launch device timing: while enabled, every kernel launch is bracketed
  * by CUDA events on the handle's stream (runs then skip graph capture).
  * Disabling clears the totals. */

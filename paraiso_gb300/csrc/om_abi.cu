@@ -15,6 +15,7 @@
 #include <set>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "om_internal.cuh"
@@ -190,8 +191,13 @@ struct om_handle_s {
     int launches = 0;
   };
   std::map<std::tuple<int, int, uint64_t>, GraphEntry> graphs;
-  // keys run once, by plain launches: a run is captured when it comes again
-  std::set<std::tuple<int, int, uint64_t>> once;
+  // (kernel, n) of runs that went by plain launches once: such a run is captured
+  // when it comes again, whichever buffers and state it starts from then (a run
+  // that swaps the buffers an odd number of times would otherwise go four times
+  // before its first replay).  Bounded, for callers whose n is always another.
+  static constexpr size_t kMostOnce = 1024;
+  std::set<std::pair<int, int>> once;
+  long replays = 0;
   unsigned replaced = 0;  // h.replaced when the graphs were captured
   int last_launches = 0;
 
@@ -430,11 +436,16 @@ om_status om_run_n(om_handle H, int kernel_id, int n) {
   const uint64_t key2 = mask ^ (skey << 32);
   auto key = std::make_tuple(kernel_id, n, key2);
   auto it = H->graphs.find(key);
-  if (it == H->graphs.end() && H->once.insert(key).second) {
+  const std::pair<int, int> run(kernel_id, n);
+  if (it == H->graphs.end() && !H->once.count(run)) {
+    if (H->once.size() >= om_handle_s::kMostOnce) H->once.clear();
+    H->once.insert(run);
     OM_TRY(run_plain(H, kernel_id, n));
     return finish(h);
   }
-  if (it == H->graphs.end()) {
+  if (it != H->graphs.end()) {
+    H->replays++;
+  } else {
     om_handle_s::GraphEntry e;
     cudaGraph_t g = nullptr;
     OM_CUDA_CHECK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -617,6 +628,12 @@ om_status om_profile_query(om_handle H, const char *kernel, long *launches,
   if (launches) *launches = it->second.launches;
   if (total_ms) *total_ms = it->second.ms;
   if (total_units) *total_units = it->second.units;
+  return OM_OK;
+}
+
+om_status om_replay_count(om_handle H, long *replays) {
+  if (!H || !replays) { set_error("null argument"); return OM_ERR_ARG; }
+  *replays = H->replays;
   return OM_OK;
 }
 

@@ -36,6 +36,7 @@ EXPORTS = [
     "om_array_host_const", "om_array_device", "om_array_read", "om_array_write",
     "om_life_fill_random", "om_life_population_history", "om_hydro_init_kh",
     "om_hydro_totals", "om_hydro_dt_history", "om_time_run", "om_last_launch_count",
+    "om_replay_count",
     "om_profile_enable", "om_profile_query",
     "om_ensemble_create", "om_ensemble_destroy", "om_ensemble_info", "om_ensemble_init_kh",
     "om_ensemble_step", "om_ensemble_time_step", "om_ensemble_read", "om_ensemble_write",
@@ -101,6 +102,7 @@ def load_library(path: str | None = None) -> C.CDLL:
         "om_hydro_dt_history": (i, [vp, vp, i, ip]),
         "om_time_run": (i, [vp, i, i, C.POINTER(C.c_float)]),
         "om_last_launch_count": (i, [vp, ip]),
+        "om_replay_count": (i, [vp, C.POINTER(C.c_long)]),
         "om_profile_enable": (i, [vp, i]),
         "om_ensemble_create": (i, [i, ip, C.POINTER(Config), C.POINTER(vp)]),
         "om_ensemble_destroy": (i, [vp]),
@@ -238,6 +240,12 @@ class OrthotopeMachine:
     def last_launch_count(self) -> int:
         out = C.c_int()
         _check(self._L.om_last_launch_count(self._h, C.byref(out)))
+        return out.value
+
+    def replay_count(self) -> int:
+        """Runs of this machine so far that replayed a captured graph."""
+        out = C.c_long()
+        _check(self._L.om_replay_count(self._h, C.byref(out)))
         return out.value
 
     def profile(self, enable: bool = True) -> None:

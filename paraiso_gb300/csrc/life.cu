@@ -58,6 +58,7 @@ struct LifeState {
   int last_n = 0;
   int depth = 0, tile_w = 0, tile_h = 0;  // tuned or configured
   uint32_t *packed[2] = {nullptr, nullptr};  // the packed grid between launches
+  bool packed_refused = false;  // no memory for it: runs do without
   // tensor maps of the two cell buffers (cells x words x rows) for the TMA
   // kernels, keyed by buffer address, and their one-word maps (32 cells x 1
   // word x 1 row, no swizzle) for the halo word that wraps around;
@@ -1477,17 +1478,17 @@ static bool life_run_packed(const Handle *h, int n) {
 
 static om_status life_reserve(Handle *h, int kernel_id, int n) {
   LifeState *st = life_state(h);
-  if (h->kernels[kernel_id].name == "proceed" && !st->packed[0] && life_run_packed(h, n)) {
+  if (h->kernels[kernel_id].name == "proceed" && !st->packed[0] && !st->packed_refused &&
+      life_run_packed(h, n)) {
     const size_t words = (size_t)((h->size[0] + 31) / 32) * h->size[1];
-    for (int i = 0; i < 2; ++i)
-      if (injected_alloc_failure() ||
-          cudaMalloc(&st->packed[i], words * sizeof(uint32_t)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(st->packed[0]);
-        st->packed[0] = st->packed[1] = nullptr;
-        set_error("Life: cannot allocate the packed grid");
-        return OM_ERR_NOMEM;
-      }
+    for (int i = 0; i < 2 && !st->packed_refused; ++i)
+      st->packed_refused = injected_alloc_failure() ||
+                           cudaMalloc(&st->packed[i], words * sizeof(uint32_t)) != cudaSuccess;
+    if (st->packed_refused) {  // 1/16 more than the cells take: the run goes without
+      cudaGetLastError();
+      cudaFree(st->packed[0]);
+      st->packed[0] = st->packed[1] = nullptr;
+    }
   }
   if (n <= st->pop_cap) return OM_OK;
   int cap = std::max(n, kHistory);
@@ -1920,10 +1921,6 @@ static const int kWsEdgeDepth = 22;
 // faster (1144 to 1208 us over its row counts, warps and depths).
 static om_status proceed_packed(Handle *h, int n, int g) {
   LifeState *st = life_state(h);
-  if (!st->packed[0]) {
-    set_error("Life: packed grid not reserved");
-    return OM_ERR_STATE;
-  }
   Array &a = h->arrays[0];
   TbParams p{};
   p.n0 = h->size[0];
@@ -2035,8 +2032,11 @@ static om_status life_proceed(Handle *h, int n) {
   const bool ragged = n0 % 32 != 0;
   const bool small = life_small(h);
   // on rows that are no whole number of words, a single generation is cheaper
-  // one cell per thread than packed, advanced and unpacked
-  const bool packed_ok = life_packed_ok(h) && (!ragged || small || n >= 2);
+  // one cell per thread than packed, advanced and unpacked; without memory for
+  // the packed grid all of them go so, and runs of whole words go in launches of
+  // at most 32 generations
+  const bool packed_ok =
+      life_packed_ok(h) && (!ragged || small || (n >= 2 && st->packed[0]));
   if (life_one_launch(h, n)) {
     OM_TRY(launch_small(h, n, nullptr, hist, 0));
     st->last_n = n;
@@ -2063,7 +2063,7 @@ static om_status life_proceed(Handle *h, int n) {
       gens = std::min(n - g, kSmallMaxGens);
       OM_TRY(launch_small(h, gens, st->d_pop + g, nullptr, 0));
     }
-  } else if (g < n && (ragged || life_run_packed(h, n - g))) {
+  } else if (g < n && (ragged || (st->packed[0] && life_run_packed(h, n - g)))) {
     OM_TRY(proceed_packed(h, n, g));
   } else if (g < n) {
     const int wd = n0 / 32;

@@ -9,6 +9,7 @@
 //   precision 32, variant 0  fused tiled step, FP32, multiply-add contraction
 //   precision 32, variant 2  fused tiled step, FP32, exact operation order
 //   precision 64, variant 0  two-kernel tiled step, FP64, exact operation order
+//                            (fused where its scratch finds no memory)
 //   precision 32/64, variant 1  plain path: the generated structure (timescale
 //                            pass, min-reduce with a host round trip,
 //                            all-Delayed recompute step, manifest copies)
@@ -36,7 +37,8 @@ struct HydroState {
   double ts_ext1 = 0;             // extent1 it was computed with (open grids)
   int lm = 0;                     // margin width: 3 on an open grid, else 0
   unsigned long long *d_margin = nullptr;  // open grid: margin cells' CFL minimum
-  HydroStage1 q{};             // FP64: the stage-1 state (one allocation, q[0] its base)
+  HydroStage1 q{};             // FP64: the stage-1 state (one allocation, q[0] its base;
+                               // null: no memory for it)
   double *d_dt = nullptr;      // dt history of the last run
   int dt_cap = 0;
   int last_n = 0;
@@ -158,7 +160,9 @@ static om_status proceed_fused(Handle *h, int n) {
                                                         ((h->size[1] + 31) / 32),
                                                     h->device, h->cfg.grid_limit)
                            : -1;
-  const char *kname = st->fp64 ? "hydro_stage_kernels_f64"
+  const bool two = st->fp64 && st->q.q[0];  // two kernels a step
+  const char *kname = two ? "hydro_stage_kernels_f64"
+                      : st->fp64 ? "hydro_fused_kernel_f64"
                       : st->variant == 2 ? "hydro_fused_kernel_f32_exact"
                       : persist          ? (form == 2   ? "hydro_pair2_kernel"
                                             : form == 1 ? "hydro_pair_kernel"
@@ -195,7 +199,7 @@ static om_status proceed_fused(Handle *h, int n) {
       return OM_ERR_CUDA;
     }
     prof_end(h, ev, kname, cells);
-    h->launches += st->fp64 ? 2 : 1;
+    h->launches += two ? 2 : 1;
     for (int i = 0; i < 4; ++i) h->arrays[i].swap();
     rd = wr;
     wr = third;
@@ -480,17 +484,6 @@ om_status hydro_setup(Handle *h) {
   h->kernels.push_back({"init", hydro_init});
   h->kernels.push_back({"proceed", hydro_proceed});
   const size_t cells = h->memory_size_total();
-  if (st->fp64 && st->variant == 0) {
-    const size_t pitch = (cells * es + 255) / 256 * 256;
-    if (cudaMalloc(&st->q.q[0], 4 * pitch) != cudaSuccess) {
-      cudaGetLastError();
-      st->q.q[0] = nullptr;
-      set_error("Hydro: cannot allocate the stage-1 state");
-      return OM_ERR_NOMEM;
-    }
-    for (int i = 1; i < 4; ++i) st->q.q[i] = (char *)st->q.q[0] + pitch * i;
-    hydro_f64_tile(st->q, h->size[0], h->size[1], h->device);
-  }
   if (cudaMalloc(&st->d_ts, cells * es) != cudaSuccess ||
       cudaMalloc(&st->d_min, sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&st->d_margin, sizeof(unsigned long long)) != cudaSuccess ||
@@ -501,6 +494,17 @@ om_status hydro_setup(Handle *h) {
     cudaGetLastError();
     set_error("Hydro: scratch allocation failed");
     return OM_ERR_NOMEM;
+  }
+  if (st->fp64 && st->variant == 0) {
+    // last, and not needed: without it a step is one kernel
+    const size_t pitch = (cells * es + 255) / 256 * 256;
+    if (injected_alloc_failure() || cudaMalloc(&st->q.q[0], 4 * pitch) != cudaSuccess) {
+      cudaGetLastError();
+      st->q.q[0] = nullptr;
+    } else {
+      for (int i = 1; i < 4; ++i) st->q.q[i] = (char *)st->q.q[0] + pitch * i;
+      hydro_f64_tile(st->q, h->size[0], h->size[1], h->device);
+    }
   }
   return OM_OK;
 }

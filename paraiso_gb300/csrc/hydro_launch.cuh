@@ -88,7 +88,7 @@ inline int hydro_tile_of(int tile_x, int tile_y, bool production) {
 // fused two-stage step; `exact` selects the no-contraction build
 cudaError_t hydro_fused_f32(const HydroStepArgs &a, int tile, bool exact, cudaStream_t s,
                             int *grid_out);
-// the FP64 step, its stage-1 state in q
+// the FP64 step, its stage-1 state in q (q.q[0] null: one kernel without)
 void hydro_f64_tile(HydroStage1 &q, int n0, int n1, int device);
 cudaError_t hydro_step_f64(const HydroStepArgs &a, const HydroStage1 &q, cudaStream_t s);
 // one fused step of a periodic grid that also writes the tape of the

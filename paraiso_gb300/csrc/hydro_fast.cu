@@ -141,8 +141,10 @@ static cudaError_t launch_tape_fast(const HydroStepArgs &a0, const HydroTapeOut 
 cudaError_t hydro_fused_tape(int fp64, bool exact, const HydroStepArgs &a0, const HydroTapeOut &t,
                              cudaStream_t s, int tile) {
   if (fp64 || exact) return hydro_fused_tape_exact(fp64, a0, t, s);
-  // the taped step runs the code of the handle's production step, so a
-  // recomputed state equals the forward pass's bit for bit
+  // The forward pass may run another shape of the same algebra (hydro_step_tile,
+  // partial persistent tiles): every production kernel rounds each operation of
+  // the scheme explicitly, so the states of all shapes are the same bit for bit,
+  // and a recomputed state equals the forward pass's.
   switch (tile) {
     case kPersist32x32:
     case kPair32x32:

@@ -30,7 +30,8 @@ cudaError_t launch_step(void (*kernel)(P...), int grid, int threads, size_t smem
 }
 
 // Tile shapes of the fused kernel available to the tuner (FP32 production
-// build; FP64 and the exact FP32 variant run 32x16).
+// build; the exact FP32 variant and the FP64 ensembles, taped step and step
+// without scratch run 32x16, other FP64 steps the two kernels of hydro_step_f64).
 // The sweep shapes (kSweep*) walk strips of TX columns down the grid in
 // chunks of TY rows (hydro_sweep.cuh).  kPersist32x32, kPair32x32 and
 // kPairGroups32x32 are the persistent 32 x 32 kernel with prefetched boxes

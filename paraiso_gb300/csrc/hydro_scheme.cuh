@@ -293,7 +293,8 @@ __device__ __forceinline__ R timescale(R g, R dR0, R dR1, R rho, R v0, R v1, R p
 // The timescale and the MUSCL reconstruction stay those of hs:: (the reverse
 // sweep recomputes both and must find the forward's values; the
 // reconstruction's values are exact selections and halvings, the same in
-// any spelling).
+// either spelling of the minmod for finite states but where the product of two
+// differences underflows, see hf::minmod).
 // ---------------------------------------------------------------------------
 namespace hf {
 
@@ -459,10 +460,13 @@ template <class T> struct NF {
   T fd, fn, ft, fe;
 };
 
-// minmod of two differences (hs::absmaller's value: the one of smaller
-// magnitude when both have the same sign, else zero) in three operations: the
-// smaller magnitude under the product of the signs, not below zero, under a's
-// sign
+// minmod of two differences (the one of smaller magnitude when both have the
+// same sign, else zero) in three operations: the smaller magnitude under the
+// product of the signs, not below zero, under a's sign.  That is hs::absmaller's
+// value but in two cases.  hs::absmaller tests the sign by the product, so where
+// that underflows (both below about 1e-19) it gives zero and this the smaller
+// difference; the reverse sweep decides by the product, as hs:: does.  Beside a
+// NaN hs::absmaller gives NaN or zero, this the other difference or zero.
 __device__ __forceinline__ float minmod(float a, float b) {
   float m;
   asm("min.ftz.xorsign.abs.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));

@@ -923,8 +923,10 @@ __device__ __forceinline__ hs::Flux<R> plain_wall2(const hs::Prim<R> &a0, const 
   return hs::hllc<AX>(k, L, hs::sound(g, L.rho, L.p), Rt, hs::sound(g, Rt.rho, Rt.p));
 }
 
+// (single precision: four blocks an SM; of 136 registers a thread only three fit,
+// 640 us for 1024^2 against 440)
 template <class R>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
 hydro_plain_step_kernel(PlainView<R> V, R *__restrict__ orho, R *__restrict__ ov0,
                         R *__restrict__ ov1, R *__restrict__ op, double gamma, R dtG, R dR0,
                         R dR1) {

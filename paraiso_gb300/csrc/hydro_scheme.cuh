@@ -124,10 +124,18 @@ template <class R> __device__ __forceinline__ R sound(R g, R rho, R p) {
   return root(div(g * p, rho));
 }
 
+// Whether a value that only one side of a selection needs is formed behind a
+// branch: in double, where a quotient or a root is dozens of integer instructions.
+// In single precision both sides are formed and one is selected: with branches a
+// plain step of 1024^2 took 530 us instead of 440, an exact ensemble step 3 % more.
+template <class R> constexpr bool kBranch = sizeof(R) == 8;
+
 // hllcQ sp p, condition as written in HydroMain.hs
 template <class R> __device__ __forceinline__ R hllc_q(const Gas<R> &k, R sp, R p) {
-  if (lesseq(p, sp)) return R(1);
-  return root(R(1) + k.qc * (div(sp, p) - R(1)));
+  const bool one = lesseq(p, sp);
+  if (kBranch<R> && one) return R(1);
+  const R t = root(R(1) + k.qc * (div(sp, p) - R(1)));
+  return one ? R(1) : t;
 }
 
 template <int AX, class R>
@@ -182,8 +190,11 @@ __device__ __forceinline__ Flux<R> hllc(const Gas<R> &k, const Prim<R> &L, R cl,
           xp = useL ? L.p : Rt.p;
   const R shock = useL ? shockLeft : shockRight;
   const Cons<R> c = cons.side(useL, xr, x0, x1, xp);
-  if (star) return star_flux<AX>(k, shockStar, shock, xr, x0, x1, xp, c.e);
-  return flux_prim<AX>(c, x0, x1, xp);
+  if (kBranch<R> && !star) return flux_prim<AX>(c, x0, x1, xp);
+  const Flux<R> fs = star_flux<AX>(k, shockStar, shock, xr, x0, x1, xp, c.e);
+  if (kBranch<R>) return fs;
+  const Flux<R> fp = flux_prim<AX>(c, x0, x1, xp);
+  return star ? fs : fp;
 }
 template <int AX, class R>
 __device__ __forceinline__ Flux<R> hllc(const Gas<R> &k, const Prim<R> &L, R cl,

@@ -241,31 +241,15 @@ def life_workload(args, dist: Dist) -> dict:
     life.profile(True)
     life.time_run("proceed", gens * min(args.steps, 4))
     best = None
-    for kn in ("life_packed_kernel", "life_reg_kernel", "life_ws_kernel", "life_ws_tma_kernel", "life_tb32_kernel",
-               "life_tb_kernel",
-               "life_smallreg_kernel", "life_smallgrid_kernel", "life_general_kernel"):
+    for kn in ("life_packed_kernel", "life_reg_kernel", "life_ws_kernel", "life_ws_tma_kernel",
+               "life_tb32_kernel", "life_tb_kernel", "life_smallreg_kernel",
+               "life_general_kernel"):
         q = life.profile_query(kn)
         if q[0] and (best is None or q[1] > best[1][1]):
             best = (kn, q)
     kname, (nl, kms, kunits) = best
     life.profile(False)
-    peak, peak_kind = peaks()
-    bytes_per_update = 8.0           # int32 read + int32 write per cell-update
-    per_launch_units = kunits / max(nl, 1)
-    per_launch_ms = kms / max(nl, 1)
-    achieved = bytes_per_update * per_launch_units / (per_launch_ms * 1e-3) / 1e9
-    traffic = profile_traffic(kname, n)
-    roofline = {"bound": "hbm", "kernel": kname, "achieved": round(achieved, 1),
-                "peak": peak, "peak_source": peak_source(peak_kind),
-                "unit": "GB/s", "frac": round(achieved / peak, 3),
-                "traffic": traffic["bytes_per_launch"] if traffic else None,
-                "algorithmic_bytes_per_launch": bytes_per_update * per_launch_units,
-                "launch_ms": round(per_launch_ms, 4), "launches_profiled": nl,
-                "note": "algorithmic 8 B per cell-update; temporal blocking re-uses each "
-                        "loaded cell for several generations, so frac may exceed 1"}
-    if traffic:
-        roofline["dram_gbs"] = round(traffic["bytes_per_launch"] / (per_launch_ms * 1e-3) / 1e9, 1)
-        roofline["dram_frac"] = round(roofline["dram_gbs"] / peak, 3)
+    roofline = life_roofline(kname, nl, kms, kunits, n, clk)
 
     # end to end through the public API with host buffers: per step, upload
     # the cells from pinned host memory, run `gens` generations, read the
@@ -314,6 +298,47 @@ def life_workload(args, dist: Dist) -> dict:
     if not args.no_self_check:
         out["self_check"] = life_self_check(pg, n, gens, dist, args, oracle_sample)
     return out
+
+
+def life_roofline(kname: str, nl: int, kms: float, kunits: float, n: int, clk: dict) -> dict:
+    """The roofline entry of the Life kernel `kname`: nl launches of kms ms in
+    all that advanced kunits cells by a generation."""
+    peak, peak_kind = peaks()
+    per_launch_units = kunits / max(nl, 1)
+    per_launch_ms = kms / max(nl, 1)
+    traffic = profile_traffic(kname, n)
+    # a launch of the packed kernel reads and writes one bit a cell, whatever its
+    # generations; the others int32 cells, counted per cell-update
+    packed = kname == "life_packed_kernel"
+    launch_bytes = n * n / 4.0 if packed else 8.0 * per_launch_units
+    achieved = launch_bytes / (per_launch_ms * 1e-3) / 1e9
+    roofline = {"bound": "hbm", "kernel": kname, "achieved": round(achieved, 1),
+                "peak": peak, "peak_source": peak_source(peak_kind),
+                "unit": "GB/s", "frac": round(achieved / peak, 3),
+                "traffic": traffic["bytes_per_launch"] if traffic else None,
+                "algorithmic_bytes_per_launch": launch_bytes,
+                "launch_ms": round(per_launch_ms, 4), "launches_profiled": nl,
+                "note": "algorithmic 8 B per cell-update; temporal blocking re-uses each "
+                        "loaded cell for several generations, so frac may exceed 1"}
+    if packed:
+        # bound by the integer ALU (64 lanes a cycle per SM): eight three-input
+        # operations and two funnel shifts per word of 32 cells and generation
+        import torch
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        mhz = clk.get("sm_mhz") or clk.get("sm_max_mhz") or 2070.0
+        alu_peak = 64.0 * sms * mhz * 1e6 / 1e12
+        alu = per_launch_units / 32 * 10 / (per_launch_ms * 1e-3) / 1e12
+        roofline.update(
+            bound="alu", achieved=round(alu, 2), peak=round(alu_peak, 2), unit="Tops/s",
+            peak_source=f"64 integer operations a cycle per SM, {sms} SMs at {mhz:.0f} MHz",
+            frac=round(alu / alu_peak, 3), hbm_gbs=round(achieved, 1),
+            hbm_frac=round(achieved / peak, 3),
+            note="10 integer operations per word of 32 cells and generation; a launch reads and "
+                 "writes one bit a cell (hbm_gbs)")
+    if traffic:
+        roofline["dram_gbs"] = round(traffic["bytes_per_launch"] / (per_launch_ms * 1e-3) / 1e9, 1)
+        roofline["dram_frac"] = round(roofline["dram_gbs"] / peak, 3)
+    return roofline
 
 
 def profile_traffic(kernel: str, n: int):

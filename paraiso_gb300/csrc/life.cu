@@ -1917,7 +1917,7 @@ static const int kWsEdgeDepth = 22;
 // takes 1133 us, bound by the ALU's bit operations (78 % of its cycles) between
 // the ends.  2048^2 x 100: 205 -> 102 us.  Rows of 1000 cells (1000 x 700 x
 // 100) no longer take a launch of the one-cell kernel per generation: 496 ->
-// 72 us.  A kernel of the warp-specialised form between the ends too was no
+// 79 us.  A kernel of the warp-specialised form between the ends too was no
 // faster (1144 to 1208 us over its row counts, warps and depths).
 static om_status proceed_packed(Handle *h, int n, int g) {
   LifeState *st = life_state(h);
